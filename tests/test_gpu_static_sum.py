@@ -1,0 +1,28 @@
+"""The allocation-free sum at its edges: remainders of the 4-element vectors, buffers that are only
+4-byte aligned, the smallest and largest size, every number of buffers."""
+
+import pytest
+import torch
+
+from test_zz_no_alloc import _call, _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("offset", [0, 1])  # elements from a 16-byte boundary
+@pytest.mark.parametrize("n", [1, 3, 4, 511, 512, 513, 4095])
+@pytest.mark.parametrize("world", [2, 3, 5, 8])
+def test_sum_in_buffer_order(world, n, offset):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    gen = torch.Generator().manual_seed(17 * n + world)
+    pads = [torch.randn(n + 8, generator=gen).cuda() for _ in range(world)]
+    before = [p.clone() for p in pads]
+    expect = before[0][offset:offset + n].clone()
+    for p in before[1:]:
+        expect += p[offset:offset + n]  # the same fp32 additions in the same order: bit for bit
+    rc, msg = _call(_lib(), [p[offset:offset + n] for p in pads])
+    assert rc == 0, msg
+    for p, b in zip(pads, before):
+        assert torch.equal(p[offset:offset + n], expect)
+        assert torch.equal(p[:offset], b[:offset]) and torch.equal(p[offset + n:], b[offset + n:])
