@@ -45,6 +45,7 @@ SOURCES = [
     "kernels/local_ops.cu",
     "kernels/layernorm.cu",
     "kernels/cross_entropy.cu",
+    "kernels/batchnorm.cu",
     "kernels/noalloc_allreduce.cu",
     "kernels/pipe_allreduce.cu",
 ]

@@ -70,6 +70,28 @@ cudaError_t launchCrossEntropyBackward(void* logits, bool bf16, const int64_t* t
                                        const float* upstream, float scale, int64_t rows, int vocab,
                                        int sm_count, cudaStream_t stream);
 
+// Training-mode BatchNorm of a channels-last tensor, [rows = N*H*W, channels], fp32
+// or bf16, `channels` a power of two from 8 to 2048, more than one row; the
+// affine parameters and statistics are fp32.  All tensors 16-byte aligned.
+struct BatchNormShape {
+  int64_t rows;
+  int channels;
+};
+int batchNormParts(const BatchNormShape& s, int sm_count);
+int64_t batchNormScratchFloats(const BatchNormShape& s, int sm_count);
+// y = BatchNorm(x) [+ residual] [, ReLU]; writes the batch's mean and 1/std, moves
+// the running statistics (variance with n - 1) and counts the batch in *tracked.
+cudaError_t launchBatchNormForward(const BatchNormShape& s, bool bf16, const void* x, const void* residual, void* y,
+                                   bool relu, const float* gamma, const float* beta, float* mean, float* rstd,
+                                   float* running_mean, float* running_var, int64_t* tracked, float momentum,
+                                   float eps, float* scratch, int sm_count, cudaStream_t stream);
+// `y`, `dz`: given when there was a residual and a ReLU: the output, and where the
+// residual's gradient goes.  Without a ReLU the residual's gradient is dy.
+cudaError_t launchBatchNormBackward(const BatchNormShape& s, bool bf16, const void* dy, const void* x, const void* y,
+                                    void* dz, void* dx, bool relu, const float* gamma, const float* beta,
+                                    const float* mean, const float* rstd, float* dgamma, float* dbeta,
+                                    float* scratch, int sm_count, cudaStream_t stream);
+
 uint64_t localLaunchCountImpl();
 void noteLocalLaunch();
 

@@ -234,6 +234,98 @@ void crossEntropyBackward(at::Tensor logits, at::Tensor targets, at::Tensor lse,
       sms, c10::cuda::getCurrentCUDAStream());
   TORCH_CHECK(e == cudaSuccess, "cross_entropy backward launch failed: ", cudaGetErrorString(e));
 }
+
+BatchNormShape batchNormShape(const at::Tensor& x) {
+  TORCH_CHECK(x.is_cuda() && x.dim() == 4 && x.is_contiguous(at::MemoryFormat::ChannelsLast) &&
+                  (x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16),
+              "x must be a channels-last fp32 or bf16 CUDA tensor");
+  const int64_t c = x.size(1);
+  TORCH_CHECK(c >= 8 && c <= 2048 && (c & (c - 1)) == 0, "channels must be a power of two from 8 to 2048");
+  TORCH_CHECK(x.numel() / c > 1, "more than one value per channel is needed");
+  return {x.numel() / c, (int)c};
+}
+
+void checkLikeX(const at::Tensor& t, const at::Tensor& x, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.device() == x.device() && t.scalar_type() == x.scalar_type() &&
+                  t.sizes() == x.sizes() && t.is_contiguous(at::MemoryFormat::ChannelsLast),
+              name, " must be like x: device, type, shape, channels-last");
+}
+
+at::Tensor aligned16(const at::Tensor& t) {
+  return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone();
+}
+
+void checkPerChannel(const at::Tensor& t, const at::Tensor& x, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.device() == x.device() && t.scalar_type() == at::kFloat && t.is_contiguous() &&
+                  t.numel() == x.size(1) && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0,
+              name, " must be a contiguous, 16-byte aligned fp32 CUDA vector with one entry per channel");
+}
+
+// y, mean, rstd of training-mode BatchNorm [+ residual] [, ReLU]; moves the running statistics.
+std::tuple<at::Tensor, at::Tensor, at::Tensor> batchNormForward(
+    at::Tensor x, std::optional<at::Tensor> residual, at::Tensor gamma, at::Tensor beta, at::Tensor running_mean,
+    at::Tensor running_var, at::Tensor tracked, double momentum, double eps, bool relu) {
+  const BatchNormShape s = batchNormShape(x);
+  checkPerChannel(gamma, x, "weight");
+  checkPerChannel(beta, x, "bias");
+  checkPerChannel(running_mean, x, "running_mean");
+  checkPerChannel(running_var, x, "running_var");
+  TORCH_CHECK(tracked.is_cuda() && tracked.device() == x.device() && tracked.scalar_type() == at::kLong &&
+                  tracked.numel() == 1,
+              "num_batches_tracked must be one int64 on the GPU");
+  c10::cuda::CUDAGuard guard(x.device());
+  x = aligned16(x);
+  at::Tensor res;
+  if (residual.has_value() && residual->defined()) {
+    checkLikeX(*residual, x, "residual");
+    res = aligned16(*residual);
+  }
+  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  auto fopt = x.options().dtype(at::kFloat).memory_format(at::MemoryFormat::Contiguous);
+  at::Tensor y = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
+  at::Tensor mean = at::empty({s.channels}, fopt), rstd = at::empty({s.channels}, fopt);
+  at::Tensor scratch = at::empty({batchNormScratchFloats(s, sms)}, fopt);
+  cudaError_t e = launchBatchNormForward(
+      s, x.scalar_type() == at::kBFloat16, x.data_ptr(), res.defined() ? res.data_ptr() : nullptr, y.data_ptr(), relu,
+      gamma.data_ptr<float>(), beta.data_ptr<float>(), mean.data_ptr<float>(), rstd.data_ptr<float>(),
+      running_mean.data_ptr<float>(), running_var.data_ptr<float>(), tracked.data_ptr<int64_t>(), (float)momentum,
+      (float)eps, scratch.data_ptr<float>(), sms, c10::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(e == cudaSuccess, "batch_norm forward launch failed: ", cudaGetErrorString(e));
+  return std::make_tuple(y, mean, rstd);
+}
+
+// dx, gradient of the residual, dgamma, dbeta.  `y`: the output, given when there
+// was a residual and a ReLU; otherwise the second result is undefined.
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> batchNormBackward(
+    at::Tensor dy, at::Tensor x, std::optional<at::Tensor> y, at::Tensor gamma, at::Tensor beta, at::Tensor mean,
+    at::Tensor rstd, bool relu) {
+  const BatchNormShape s = batchNormShape(x);
+  checkLikeX(dy, x, "dy");
+  checkPerChannel(gamma, x, "weight");
+  checkPerChannel(beta, x, "bias");
+  checkPerChannel(mean, x, "mean");
+  checkPerChannel(rstd, x, "rstd");
+  c10::cuda::CUDAGuard guard(x.device());
+  x = aligned16(x);
+  dy = aligned16(dy);
+  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  at::Tensor dz, yt;
+  if (y.has_value() && y->defined()) {
+    checkLikeX(*y, x, "y");
+    yt = aligned16(*y);
+    dz = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
+  }
+  at::Tensor dx = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
+  at::Tensor dgamma = at::empty_like(gamma), dbeta = at::empty_like(gamma);
+  at::Tensor scratch = at::empty({batchNormScratchFloats(s, sms)}, gamma.options());
+  cudaError_t e = launchBatchNormBackward(
+      s, x.scalar_type() == at::kBFloat16, dy.data_ptr(), x.data_ptr(), yt.defined() ? yt.data_ptr() : nullptr,
+      dz.defined() ? dz.data_ptr() : nullptr, dx.data_ptr(), relu, gamma.data_ptr<float>(), beta.data_ptr<float>(),
+      mean.data_ptr<float>(), rstd.data_ptr<float>(), dgamma.data_ptr<float>(), dbeta.data_ptr<float>(),
+      scratch.data_ptr<float>(), sms, c10::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(e == cudaSuccess, "batch_norm backward launch failed: ", cudaGetErrorString(e));
+  return std::make_tuple(dx, dz, dgamma, dbeta);
+}
 }  // namespace
 
 uint64_t localLaunchCount() { return localLaunchCountImpl(); }
@@ -254,6 +346,11 @@ void bindLocalOps(pybind11::module_& m) {
         py::arg("bias"), py::arg("eps"), py::arg("out_dtype"));
   m.def("add_layer_norm_bwd", &addLayerNormBackward, py::arg("dy"), py::arg("xnew"), py::arg("weight"),
         py::arg("mean"), py::arg("rstd"), py::arg("gres"), py::arg("want_bf16"));
+  m.def("batch_norm_fwd", &batchNormForward, py::arg("x"), py::arg("residual"), py::arg("weight"), py::arg("bias"),
+        py::arg("running_mean"), py::arg("running_var"), py::arg("tracked"), py::arg("momentum"), py::arg("eps"),
+        py::arg("relu"));
+  m.def("batch_norm_bwd", &batchNormBackward, py::arg("dy"), py::arg("x"), py::arg("y"), py::arg("weight"),
+        py::arg("bias"), py::arg("mean"), py::arg("rstd"), py::arg("relu"));
   m.def("layer_norm_fwd", &layerNormForward, py::arg("x"), py::arg("weight"), py::arg("bias"),
         py::arg("eps"), py::arg("out_dtype"));
   m.def("layer_norm_bwd", &layerNormBackward, py::arg("dy"), py::arg("x"), py::arg("weight"),

@@ -1,7 +1,8 @@
 """ResNet-50 (bottleneck blocks [3, 4, 6, 3], 25.6M parameters) for the
 image-classification data-parallel workload: many small gradient buckets, which
 stresses the small-message (one-shot) path of the backend.  Plain PyTorch
-layers; channels-last friendly.
+layers; on channels-last activations BatchNorm, residual add and ReLU run as
+one fused op (:func:`fairring_b200.ops.batch_norm_act`).
 """
 
 from __future__ import annotations
@@ -25,11 +26,24 @@ class Bottleneck(nn.Module):
         self.downsample = downsample
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        from ..ops import batch_norm_act
+
         identity = x if self.downsample is None else self.downsample(x)
-        out = self.relu(self.bn1(self.conv1(x)))
-        out = self.relu(self.bn2(self.conv2(out)))
-        out = self.bn3(self.conv3(out))
-        return self.relu(out + identity)
+        out = batch_norm_act(self.bn1, self.conv1(x), relu=self.relu)
+        out = batch_norm_act(self.bn2, self.conv2(out), relu=self.relu)
+        return batch_norm_act(self.bn3, self.conv3(out), residual=identity, relu=self.relu)
+
+
+class Downsample(nn.Sequential):
+    """Strided 1x1 convolution and BatchNorm of a block's shortcut."""
+
+    def forward(self, x: torch.Tensor) -> torch.Tensor:
+        from ..ops import batch_norm_act
+
+        if len(self) != 2:
+            return super().forward(x)
+        conv, bn = self
+        return batch_norm_act(bn, conv(x))
 
 
 class ResNet50(nn.Module):
@@ -56,7 +70,7 @@ class ResNet50(nn.Module):
     def _make_layer(self, planes: int, blocks: int, stride: int = 1) -> nn.Sequential:
         downsample = None
         if stride != 1 or self.inplanes != planes * Bottleneck.expansion:
-            downsample = nn.Sequential(
+            downsample = Downsample(
                 nn.Conv2d(self.inplanes, planes * Bottleneck.expansion, 1, stride=stride, bias=False),
                 nn.BatchNorm2d(planes * Bottleneck.expansion),
             )
@@ -69,7 +83,9 @@ class ResNet50(nn.Module):
         return sum(p.numel() for p in self.parameters())
 
     def forward(self, images: torch.Tensor, labels: torch.Tensor | None = None):
-        x = self.maxpool(self.relu(self.bn1(self.conv1(images))))
+        from ..ops import batch_norm_act
+
+        x = self.maxpool(batch_norm_act(self.bn1, self.conv1(images), relu=self.relu))
         x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
         logits = self.fc(torch.flatten(self.avgpool(x), 1))
         if labels is None:

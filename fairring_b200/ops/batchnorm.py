@@ -1,0 +1,85 @@
+"""Training-mode BatchNorm with the residual add and ReLU behind it
+(``csrc/kernels/batchnorm.cu``), for channels-last activations.
+
+torch runs BatchNorm, the add and the ReLU as separate passes over the
+activations in both directions.  Here the forward is two passes (statistics,
+then everything else) and the backward two (the channel sums, then ``dx``); the
+ReLU's mask is recomputed from the input instead of being read back.
+"""
+
+from __future__ import annotations
+
+import torch
+import torch.nn as nn
+import torch.nn.functional as F
+
+from .. import _C
+from ._plain import plain_autograd, plain_module
+
+
+class _BatchNormActFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, residual, weight, bias, running_mean, running_var, tracked, momentum, eps, relu):
+        y, mean, rstd = _C.batch_norm_fwd(x, residual, weight, bias, running_mean, running_var, tracked, momentum,
+                                          eps, relu)
+        torch.autograd.graph.increment_version(tracked)  # as torch's own layer does, which adds 1 in place
+        ctx.relu, ctx.eps, ctx.has_residual = relu, eps, residual is not None
+        ctx.save_for_backward(x, weight, bias, mean, rstd, residual, y if relu and residual is not None else None)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, weight, bias, mean, rstd, residual, y = ctx.saved_tensors
+        if torch.is_grad_enabled():  # the graph of this backward is wanted: torch's own ops have one
+            inputs = (x, weight, bias) if residual is None else (x, weight, bias, residual)
+            wanted = [t for t in inputs if t.requires_grad]
+            with torch.enable_grad():
+                out = F.batch_norm(x, None, None, weight, bias, True, 0.0, ctx.eps)
+                out = out if residual is None else out + residual
+                out = F.relu(out) if ctx.relu else out
+                grads = iter(torch.autograd.grad(out, wanted, dy, create_graph=True))
+            got = [next(grads) if t.requires_grad else None for t in inputs] + [None]
+            return got[0], got[3], got[1], got[2], None, None, None, None, None, None
+        dy = dy.contiguous(memory_format=torch.channels_last)
+        dx, dres, dgamma, dbeta = _C.batch_norm_bwd(dy, x, y, weight, bias, mean, rstd, ctx.relu)
+        if ctx.has_residual and not ctx.relu:
+            dres = dy
+        return dx, dres if ctx.has_residual else None, dgamma, dbeta, None, None, None, None, None, None
+
+
+def _channels_last(t: torch.Tensor) -> bool:
+    return t.is_contiguous(memory_format=torch.channels_last) and t.data_ptr() % 16 == 0
+
+
+def _fusable(bn: nn.BatchNorm2d, x: torch.Tensor, residual: torch.Tensor | None) -> bool:
+    if not (bn.training and plain_module(bn, nn.BatchNorm2d) and x.is_cuda and x.dim() == 4):
+        return False
+    c = x.shape[1]
+    params = (bn.weight, bn.bias, bn.running_mean, bn.running_var)
+    if bn.momentum is None or bn.num_batches_tracked is None or any(
+            p is None or p.dtype != torch.float32 or p.device != x.device or p.numel() != c or not p.is_contiguous()
+            or p.data_ptr() % 16 for p in params):
+        return False
+    if bn.num_batches_tracked.device != x.device or bn.num_batches_tracked.dtype != torch.long:
+        return False
+    if x.dtype not in (torch.float32, torch.bfloat16) or not 8 <= c <= 2048 or c & (c - 1) or x.numel() <= c:
+        return False
+    if residual is not None and (residual.dtype != x.dtype or residual.shape != x.shape or residual.device != x.device
+                                 or not _channels_last(residual)):
+        return False
+    return _channels_last(x) and plain_autograd()
+
+
+def batch_norm_act(bn: nn.Module, x: torch.Tensor, residual: torch.Tensor | None = None,
+                   relu: nn.Module | None = None) -> torch.Tensor:
+    """``relu(bn(x) + residual)``; ``residual`` and ``relu`` may be left out.  Fused for an
+    ``nn.BatchNorm2d`` in training mode and a channels-last fp32 or bf16 ``x`` on the GPU with a
+    power of two from 8 to 2048 channels; otherwise, and when one of the modules carries hooks or
+    has been replaced, the modules are called."""
+    if (relu is None or plain_module(relu, nn.ReLU)) and _fusable(bn, x, residual):
+        return _BatchNormActFn.apply(x, residual, bn.weight, bn.bias, bn.running_mean, bn.running_var,
+                                     bn.num_batches_tracked, bn.momentum, bn.eps, relu is not None)
+    y = bn(x)
+    if residual is not None:
+        y = y + residual
+    return y if relu is None else relu(y)

@@ -1,0 +1,127 @@
+"""BatchNorm + residual + ReLU in one op against the same in fp64."""
+
+import pytest
+import torch
+import torch.nn as nn
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _need_gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+
+
+def _reference(x, res, bn, relu, dy):
+    leaves = [t.detach().double().requires_grad_(True) for t in (x, bn.weight, bn.bias)]
+    r = None if res is None else res.detach().double().requires_grad_(True)
+    z = F.batch_norm(leaves[0], None, None, leaves[1], leaves[2], True, 0.0, bn.eps)
+    z = z if r is None else z + r
+    y = F.relu(z) if relu else z
+    grads = torch.autograd.grad(y, leaves + ([] if r is None else [r]), dy.double())
+    return y.detach(), z.detach(), grads
+
+
+def _close(got, want, eps, scale=0.0):
+    """Within `eps` of the value (the type's rounding) plus 1e-4 of `scale` (fp32 sums and their inputs)."""
+    bad = (got.double() - want).abs() > eps * want.abs() + 1e-4 * scale + 1e-12
+    assert not bad.any(), (int(bad.sum()), float((got.double() - want).abs().max()))
+
+
+# rows: 2 (the fewest), fewer than a block holds, remainders of the unrolled loops, more than one pass of the grid
+@pytest.mark.parametrize("shape", [(2, 8, 1, 1), (3, 8, 5, 7), (2, 16, 9, 9), (4, 64, 33, 31), (8, 256, 14, 13),
+                                   (16, 2048, 7, 7), (1, 2048, 1, 3), (16, 64, 112, 112)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("residual,relu", [(False, False), (False, True), (True, False), (True, True)])
+def test_matches_fp64(shape, dtype, residual, relu):
+    _need_gpu()
+    from fairring_b200.ops import batch_norm_act
+    from fairring_b200.ops.batchnorm import _fusable
+
+    gen = torch.Generator(device="cuda").manual_seed(sum(shape))
+    rand = lambda: torch.randn(shape, device="cuda", generator=gen).to(  # noqa: E731
+        dtype=dtype, memory_format=torch.channels_last)
+    offset = 3.0 * torch.arange(shape[1], device="cuda").view(1, -1, 1, 1).remainder(7)  # means far from zero
+    x = (rand().float() + offset).to(dtype=dtype, memory_format=torch.channels_last).requires_grad_(True)
+    res = rand().requires_grad_(True) if residual else None
+    dy = rand()
+    bn = nn.BatchNorm2d(shape[1], device="cuda")
+    with torch.no_grad():
+        bn.weight.normal_(1.0, 0.2, generator=gen)
+        bn.bias.normal_(0.0, 0.5, generator=gen)
+    want_stats = nn.BatchNorm2d(shape[1], device="cuda").double()
+    want_stats(x.detach().double())
+
+    assert _fusable(bn, x, res)
+    y = batch_norm_act(bn, x, res, nn.ReLU(inplace=True) if relu else None)
+    y_ref, z, grads_ref = _reference(x, res, bn, relu, dy)
+    grads = torch.autograd.grad(y, [x, bn.weight, bn.bias] + ([res] if residual else []), dy)
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
+    _close(y, y_ref, eps, 1.0)
+    # elements whose sign the rounding of z decides are left out, and where one is left out its channel's sums are off
+    sure = (z.abs() > 1e-4) if relu else torch.ones_like(z, dtype=torch.bool)
+    unsure = (~sure).sum((0, 2, 3)).double()
+    n = x.numel() / shape[1]
+    slack = 4.0 * float((unsure / n).max()) * float(dy.abs().max())
+    wide = max(1.0, float(grads_ref[0].abs().max()))
+    bad = ((grads[0].double() - grads_ref[0]).abs() > eps * grads_ref[0].abs() + 1e-4 * wide + slack * wide) & sure
+    assert not bad.any(), int(bad.sum())
+    for got, want in zip(grads[1:3], grads_ref[1:3]):
+        assert ((got.double() - want).abs() <= 1e-4 * n ** 0.5 * 10 + 8.0 * unsure * float(dy.abs().max())).all()
+    if residual:
+        assert ((grads[3].double() - grads_ref[3]).abs()[sure] <= 1e-12).all()  # dy or zero: exact
+    _close(bn.running_mean, want_stats.running_mean, 2.0 ** -22, 1e-2)
+    _close(bn.running_var, want_stats.running_var, 2.0 ** -20, 1e-2)
+    assert int(bn.num_batches_tracked) == 1
+
+
+def test_a_channel_far_from_zero_keeps_its_variance():
+    """Standard deviation 1 around a mean of 1000, with an outlier in front."""
+    _need_gpu()
+    from fairring_b200.ops import batch_norm_act
+
+    x = torch.randn(32, 64, 28, 28, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)) + 1000
+    x[0, :, 0, 0] += 300
+    x = x.contiguous(memory_format=torch.channels_last)
+    bn = nn.BatchNorm2d(64, device="cuda", momentum=1.0)
+    batch_norm_act(bn, x)
+    want = x.double().var((0, 2, 3))
+    assert ((bn.running_var.double() - want).abs() <= 1e-5 * want).all()
+
+
+def test_calls_the_modules_where_they_cannot_be_skipped():
+    _need_gpu()
+    from fairring_b200.ops import batch_norm_act
+    from fairring_b200.ops.batchnorm import _fusable
+
+    x = torch.randn(4, 16, 6, 6, device="cuda").contiguous(memory_format=torch.channels_last)
+    bn, relu = nn.BatchNorm2d(16, device="cuda"), nn.ReLU()
+    assert _fusable(bn, x, None)
+    assert not _fusable(bn, x.contiguous(), None)  # NCHW
+    assert not _fusable(bn, x.half(), None)
+    assert not _fusable(bn, x, x.bfloat16())
+    assert not _fusable(nn.BatchNorm2d(24, device="cuda"), x.new_zeros(4, 24, 6, 6), None)
+    seen = []
+    handle = relu.register_forward_hook(lambda *a: seen.append(1))
+    batch_norm_act(bn, x, relu=relu)
+    assert seen == [1]
+    handle.remove()
+    bn.eval()
+    torch.testing.assert_close(batch_norm_act(bn, x, relu=relu), relu(bn(x)))
+
+
+def test_second_derivative():
+    _need_gpu()
+    from fairring_b200.ops import batch_norm_act
+
+    torch.manual_seed(0)
+    x0 = torch.randn(3, 8, 4, 4, device="cuda").contiguous(memory_format=torch.channels_last)
+    got = []
+    for fused in (True, False):
+        x = x0.clone(memory_format=torch.channels_last).requires_grad_(True)
+        bn = nn.BatchNorm2d(8, device="cuda")
+        y = batch_norm_act(bn, x) if fused else bn(x)
+        (g,) = torch.autograd.grad((y ** 3).sum(), x, create_graph=True)
+        got.append(torch.autograd.grad((g ** 2).sum(), x)[0])
+    torch.testing.assert_close(got[0], got[1], rtol=1e-3, atol=1e-4 * float(got[1].abs().max()))
