@@ -60,15 +60,20 @@ cudaError_t launchAddLayerNormBackward(const void* dy, bool y_bf16, const float*
                                        float* dbeta, int64_t rows, int cols, int sm_count,
                                        cudaStream_t stream);
 
-// Softmax cross-entropy over [rows, vocab] logits (fp32 or bf16, vocab a
-// multiple of 8): per-row loss and log-sum-exp; the backward overwrites the
-// logits with their gradient, scaled by *upstream (a device scalar) * scale.
+// Softmax cross-entropy over [rows, vocab] logits (fp32 or bf16): per-row loss
+// and log-sum-exp; a negative target's row has loss 0, one past the vocabulary
+// has loss `bad_target`.
 cudaError_t launchCrossEntropyForward(const void* logits, bool bf16, const int64_t* targets, float* loss,
-                                      float* lse, int64_t rows, int vocab, int sm_count,
-                                      cudaStream_t stream);
-cudaError_t launchCrossEntropyBackward(void* logits, bool bf16, const int64_t* targets, const float* lse,
-                                       const float* upstream, float scale, int64_t rows, int vocab,
-                                       int sm_count, cudaStream_t stream);
+                                      float* lse, int64_t rows, int vocab, float bad_target, cudaStream_t stream);
+// *mean = sum of `loss` / *count, *count = max(number of targets >= 0, least).
+cudaError_t launchCrossEntropyMean(const float* loss, const int64_t* targets, int64_t rows, float least,
+                                   float* mean, float* count, cudaStream_t stream);
+// The gradient, scaled by *upstream / *count * scale (device scalars, count may be
+// null); `grad` may be the logits themselves and lies as they do relative to a
+// 16-byte boundary.
+cudaError_t launchCrossEntropyBackward(const void* logits, void* grad, bool bf16, const int64_t* targets,
+                                       const float* lse, const float* upstream, const float* count, float scale,
+                                       int64_t rows, int vocab, cudaStream_t stream);
 
 // Training-mode BatchNorm of a channels-last tensor, [rows = N*H*W, channels], fp32
 // or bf16, `channels` a power of two from 8 to 2048, more than one row; the

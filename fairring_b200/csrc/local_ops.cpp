@@ -199,40 +199,75 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerNormBackward(
   return std::make_tuple(dx, dbr, dgamma, dbeta);
 }
 
-// (per-row loss, per-row log-sum-exp) of logits [rows, vocab] against targets [rows].
-std::tuple<at::Tensor, at::Tensor> crossEntropyForward(at::Tensor logits, at::Tensor targets) {
+void checkLogits(const at::Tensor& logits, const at::Tensor& targets) {
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.is_contiguous(),
               "logits must be a contiguous 2-D CUDA tensor");
   TORCH_CHECK(logits.scalar_type() == at::kFloat || logits.scalar_type() == at::kBFloat16,
               "logits must be fp32 or bf16");
-  TORCH_CHECK(targets.is_cuda() && targets.scalar_type() == at::kLong && targets.is_contiguous() &&
-                  targets.numel() == logits.size(0),
+  TORCH_CHECK(targets.is_cuda() && targets.device() == logits.device() && targets.scalar_type() == at::kLong &&
+                  targets.is_contiguous() && targets.numel() == logits.size(0),
               "targets must be a contiguous int64 CUDA vector with one entry per row");
-  TORCH_CHECK(logits.size(1) % 8 == 0, "the vocabulary size must be a multiple of 8");
+  TORCH_CHECK(logits.size(1) > 0 && logits.size(1) <= INT32_MAX, "the vocabulary must not be empty");
+}
+
+// (per-row loss, per-row log-sum-exp) of logits [rows, vocab] against targets [rows];
+// a target past the vocabulary gives `bad_target`.
+std::tuple<at::Tensor, at::Tensor> crossEntropyForward(at::Tensor logits, at::Tensor targets, double bad_target) {
+  checkLogits(logits, targets);
   c10::cuda::CUDAGuard guard(logits.device());
   auto fopt = logits.options().dtype(at::kFloat);
   at::Tensor loss = at::empty({logits.size(0)}, fopt), lse = at::empty({logits.size(0)}, fopt);
-  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   cudaError_t e = launchCrossEntropyForward(logits.data_ptr(), logits.scalar_type() == at::kBFloat16,
                                             targets.data_ptr<int64_t>(), loss.data_ptr<float>(),
-                                            lse.data_ptr<float>(), logits.size(0), (int)logits.size(1), sms,
-                                            c10::cuda::getCurrentCUDAStream());
+                                            lse.data_ptr<float>(), logits.size(0), (int)logits.size(1),
+                                            (float)bad_target, c10::cuda::getCurrentCUDAStream());
   TORCH_CHECK(e == cudaSuccess, "cross_entropy forward launch failed: ", cudaGetErrorString(e));
   return std::make_tuple(loss, lse);
 }
 
-// Overwrites logits with d(loss)/d(logits) * upstream * scale.
-void crossEntropyBackward(at::Tensor logits, at::Tensor targets, at::Tensor lse, at::Tensor upstream,
-                          double scale) {
+// (mean loss over the rows whose target is not negative, how many those are, at least `least`)
+std::tuple<at::Tensor, at::Tensor> crossEntropyMean(at::Tensor losses, at::Tensor targets, double least) {
+  checkFlat(losses, "losses");
+  TORCH_CHECK(targets.is_cuda() && targets.device() == losses.device() && targets.scalar_type() == at::kLong &&
+                  targets.is_contiguous() && targets.numel() == losses.numel(),
+              "targets must be a contiguous int64 CUDA vector with one entry per row");
+  c10::cuda::CUDAGuard guard(losses.device());
+  at::Tensor mean = at::empty({}, losses.options()), count = at::empty({1}, losses.options());
+  cudaError_t e = launchCrossEntropyMean(losses.data_ptr<float>(), targets.data_ptr<int64_t>(), losses.numel(),
+                                         (float)least, mean.data_ptr<float>(), count.data_ptr<float>(),
+                                         c10::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(e == cudaSuccess, "cross_entropy mean launch failed: ", cudaGetErrorString(e));
+  return std::make_tuple(mean, count);
+}
+
+// Writes d(loss)/d(logits) * upstream / count * scale to `grad`, which may be the logits.
+void crossEntropyBackward(at::Tensor grad, at::Tensor logits, at::Tensor targets, at::Tensor lse, at::Tensor upstream,
+                          double scale, std::optional<at::Tensor> count) {
+  checkLogits(logits, targets);
+  TORCH_CHECK(grad.is_cuda() && grad.device() == logits.device() && grad.is_contiguous() &&
+                  grad.sizes() == logits.sizes() && grad.scalar_type() == logits.scalar_type(),
+              "grad must be like the logits");
+  TORCH_CHECK(lse.is_cuda() && lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.numel() == logits.size(0),
+              "lse must be a contiguous fp32 CUDA vector with one entry per row");
   TORCH_CHECK(upstream.is_cuda() && upstream.scalar_type() == at::kFloat && upstream.numel() == 1,
               "upstream must be a one-element fp32 CUDA tensor");
+  const float* count_ptr = nullptr;
+  if (count.has_value() && count->defined()) {
+    TORCH_CHECK(count->is_cuda() && count->scalar_type() == at::kFloat && count->numel() == 1,
+                "count must be a one-element fp32 CUDA tensor");
+    count_ptr = count->data_ptr<float>();
+  }
   c10::cuda::CUDAGuard guard(logits.device());
-  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   cudaError_t e = launchCrossEntropyBackward(
-      logits.data_ptr(), logits.scalar_type() == at::kBFloat16, targets.data_ptr<int64_t>(),
-      lse.data_ptr<float>(), upstream.data_ptr<float>(), (float)scale, logits.size(0), (int)logits.size(1),
-      sms, c10::cuda::getCurrentCUDAStream());
+      logits.data_ptr(), grad.data_ptr(), logits.scalar_type() == at::kBFloat16, targets.data_ptr<int64_t>(),
+      lse.data_ptr<float>(), upstream.data_ptr<float>(), count_ptr, (float)scale, logits.size(0),
+      (int)logits.size(1), c10::cuda::getCurrentCUDAStream());
   TORCH_CHECK(e == cudaSuccess, "cross_entropy backward launch failed: ", cudaGetErrorString(e));
+}
+
+void crossEntropyBackwardInPlace(at::Tensor logits, at::Tensor targets, at::Tensor lse, at::Tensor upstream,
+                                 double scale, std::optional<at::Tensor> count) {
+  crossEntropyBackward(logits, logits, targets, lse, upstream, scale, count);
 }
 
 BatchNormShape batchNormShape(const at::Tensor& x) {
@@ -339,9 +374,13 @@ void bindLocalOps(pybind11::module_& m) {
   m.def("bf16_grad_to_f32_", &bf16GradToF32, py::arg("dst"), py::arg("src"),
         py::arg("accumulate") = false);
   m.def("sumsq", &sumSq, py::arg("x"));
-  m.def("cross_entropy_fwd", &crossEntropyForward, py::arg("logits"), py::arg("targets"));
-  m.def("cross_entropy_bwd_", &crossEntropyBackward, py::arg("logits"), py::arg("targets"),
-        py::arg("lse"), py::arg("upstream"), py::arg("scale"));
+  m.def("cross_entropy_fwd", &crossEntropyForward, py::arg("logits"), py::arg("targets"),
+        py::arg("bad_target") = 0.0);
+  m.def("cross_entropy_mean", &crossEntropyMean, py::arg("losses"), py::arg("targets"), py::arg("least"));
+  m.def("cross_entropy_bwd", &crossEntropyBackward, py::arg("grad"), py::arg("logits"), py::arg("targets"),
+        py::arg("lse"), py::arg("upstream"), py::arg("scale"), py::arg("count") = py::none());
+  m.def("cross_entropy_bwd_", &crossEntropyBackwardInPlace, py::arg("logits"), py::arg("targets"),
+        py::arg("lse"), py::arg("upstream"), py::arg("scale"), py::arg("count") = py::none());
   m.def("add_layer_norm_fwd", &addLayerNormForward, py::arg("x"), py::arg("branch"), py::arg("weight"),
         py::arg("bias"), py::arg("eps"), py::arg("out_dtype"));
   m.def("add_layer_norm_bwd", &addLayerNormBackward, py::arg("dy"), py::arg("xnew"), py::arg("weight"),

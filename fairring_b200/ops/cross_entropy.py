@@ -1,8 +1,11 @@
-"""Softmax cross-entropy for language-model heads in two kernels
-(``csrc/kernels/cross_entropy.cu``): the forward keeps one float per row, the
-backward writes the gradient over the logits in their own dtype.  The logits
-must not be used after the loss (their memory becomes their gradient) -- true
-for a language-model head, where the loss is their only consumer.
+"""Softmax cross-entropy for language-model heads
+(``csrc/kernels/cross_entropy.cu``): the forward reads the logits once and keeps
+one float per row, the backward writes the gradient in the logits' own dtype.
+
+With a vocabulary that is a multiple of 8 the gradient is written over the
+logits: they must not be used after the loss (their memory becomes their
+gradient) -- true for a language-model head, where the loss is their only
+consumer.  With any other vocabulary the logits are left alone.
 """
 
 from __future__ import annotations
@@ -11,34 +14,59 @@ import torch
 import torch.nn.functional as F
 
 from .. import _C
+from ._plain import plain_autograd
 
 
 class _FusedCrossEntropyFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, targets):
         losses, lse = _C.cross_entropy_fwd(logits, targets)
-        valid = (targets >= 0).sum().clamp_(min=1)
-        ctx.save_for_backward(logits, targets, lse, valid)
-        return losses.sum() / valid
+        mean, count = _C.cross_entropy_mean(losses, targets, 1.0)
+        ctx.save_for_backward(logits, targets, lse, count)
+        return mean
 
     @staticmethod
     def backward(ctx, g):
-        logits, targets, lse, valid = ctx.saved_tensors
-        upstream = (g.float() / valid).reshape(1)
+        logits, targets, lse, count = ctx.saved_tensors
         grad = logits.detach()
-        _C.cross_entropy_bwd_(grad, targets, lse, upstream, 1.0)
+        _C.cross_entropy_bwd_(grad, targets, lse, g.float().reshape(1), 1.0, count)
+        return grad, None
+
+
+class _KeepingCrossEntropyFn(torch.autograd.Function):
+    """As ``F.cross_entropy(logits.float(), targets)``: the logits stay as they are, no counted row
+    gives NaN, and so does a target past the vocabulary."""
+
+    @staticmethod
+    def forward(ctx, logits, targets):
+        losses, lse = _C.cross_entropy_fwd(logits, targets, float("nan"))
+        mean, count = _C.cross_entropy_mean(losses, targets, 0.0)
+        ctx.save_for_backward(logits, targets, lse, count)
+        return mean
+
+    @staticmethod
+    def backward(ctx, g):
+        logits, targets, lse, count = ctx.saved_tensors
+        if torch.is_grad_enabled():  # the graph of this backward is wanted: torch's own ops have one
+            with torch.enable_grad():
+                loss = F.cross_entropy(logits.float(), targets.where(targets >= 0, -100))
+                return torch.autograd.grad(loss, logits, g, create_graph=True)[0], None
+        grad = torch.empty_like(logits)
+        _C.cross_entropy_bwd(grad, logits, targets, lse, g.float().reshape(1), 1.0, count)
         return grad, None
 
 
 def fused_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
     """Mean cross-entropy of ``logits`` [rows, vocab] (fp32 or bf16) against
-    ``targets`` [rows] (negative entries are ignored).  Consumes the logits: after
-    backward their storage holds the gradient.  Falls back to
-    ``F.cross_entropy(logits.float(), targets)`` off the GPU and for shapes the
-    kernels do not take."""
+    ``targets`` [rows] (negative entries are ignored).  Consumes the logits when the
+    vocabulary is a multiple of 8: after backward their storage holds the gradient.
+    Falls back to ``F.cross_entropy(logits.float(), targets)`` off the GPU and for
+    what the kernels do not take."""
     ok = (logits.is_cuda and logits.dim() == 2 and logits.is_contiguous()
-          and logits.dtype in (torch.float32, torch.bfloat16) and logits.shape[1] % 8 == 0
-          and targets.dtype == torch.long)
-    if not ok:
-        return F.cross_entropy(logits.float(), targets, ignore_index=-100)
-    return _FusedCrossEntropyFn.apply(logits, targets.contiguous())
+          and logits.dtype in (torch.float32, torch.bfloat16) and targets.dtype == torch.long)
+    if ok and logits.shape[1] % 8 == 0:
+        return _FusedCrossEntropyFn.apply(logits, targets.contiguous())
+    if (ok and logits.shape[1] > 0 and logits.data_ptr() % 16 == 0 and targets.shape == logits.shape[:1]
+            and targets.device == logits.device and plain_autograd()):
+        return _KeepingCrossEntropyFn.apply(logits, targets.contiguous())
+    return F.cross_entropy(logits.float(), targets, ignore_index=-100)
