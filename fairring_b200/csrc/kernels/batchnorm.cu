@@ -31,6 +31,7 @@
 #include <cstdint>
 
 #include "local_kernels.h"
+#include "vec8.cuh"
 
 namespace fairring {
 namespace {
@@ -39,46 +40,6 @@ constexpr int kBnThreads = 256;
 constexpr int kBnFinishWarps = 32;
 constexpr int kBnFinishLoads = 20;
 constexpr int kBnMaxBlocks = kBnFinishWarps * kBnFinishLoads;
-
-// 8 elements as they lie in memory.
-template <typename T> struct Raw8;
-template <> struct Raw8<__nv_bfloat16> {
-  uint4 r;
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) { r = *reinterpret_cast<const uint4*>(p); }
-  __device__ __forceinline__ void store(__nv_bfloat16* p) const { *reinterpret_cast<uint4*>(p) = r; }
-  __device__ __forceinline__ void get(float (&v)[8]) const {
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = __bfloat1622float2(h[i]);
-      v[2 * i] = f.x;
-      v[2 * i + 1] = f.y;
-    }
-  }
-  __device__ __forceinline__ void set(const float (&v)[8]) {
-    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&r);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-  }
-};
-template <> struct Raw8<float> {
-  float4 a, b;
-  __device__ __forceinline__ void load(const float* p) {
-    a = reinterpret_cast<const float4*>(p)[0];
-    b = reinterpret_cast<const float4*>(p)[1];
-  }
-  __device__ __forceinline__ void store(float* p) const {
-    reinterpret_cast<float4*>(p)[0] = a;
-    reinterpret_cast<float4*>(p)[1] = b;
-  }
-  __device__ __forceinline__ void get(float (&v)[8]) const {
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  }
-  __device__ __forceinline__ void set(const float (&v)[8]) {
-    a = make_float4(v[0], v[1], v[2], v[3]);
-    b = make_float4(v[4], v[5], v[6], v[7]);
-  }
-};
 
 __device__ __forceinline__ void loadChannels(const float* p, int group, float (&v)[8]) {
   Raw8<float> r;

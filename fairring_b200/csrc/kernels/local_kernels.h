@@ -97,6 +97,15 @@ cudaError_t launchBatchNormBackward(const BatchNormShape& s, bool bf16, const vo
                                     const float* mean, const float* rstd, float* dgamma, float* dbeta,
                                     float* scratch, int sm_count, cudaStream_t stream);
 
+// y = GELU(x) of n bf16 elements (a multiple of 8), tanh or erf form; 16-byte aligned.
+cudaError_t launchGeluForward(const void* x, void* y, int64_t n, bool tanh_form, cudaStream_t stream);
+// out[c] (fp32 or bf16) = sum over the rows of a [rows, cols] bf16 matrix, cols a multiple of
+// 8: of dy or, with `gelu_x`, of dx = dy * GELU'(gelu_x), which is written.  `partial`:
+// scratch of columnSumStrips(rows, cols, sm_count) x cols floats.
+int columnSumStrips(int64_t rows, int cols, int sm_count);
+cudaError_t launchColumnSum(const void* dy, const void* gelu_x, bool tanh_form, void* dx, float* partial, void* out,
+                            bool out_bf16, int64_t rows, int cols, int sm_count, cudaStream_t stream);
+
 uint64_t localLaunchCountImpl();
 void noteLocalLaunch();
 

@@ -20,6 +20,11 @@ void checkFlat(const at::Tensor& t, const char* name) {
               " must be a contiguous fp32 CUDA tensor");
 }
 
+// The tensor itself where its memory starts on a 16-byte boundary, else a copy that does.
+at::Tensor aligned16(const at::Tensor& t) {
+  return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone();
+}
+
 // One AdamW step over flat buffers, in place.  `step` counts from 1.
 void adamwFlat(at::Tensor p, at::Tensor g, at::Tensor m, at::Tensor v, double lr, double beta1,
                double beta2, double eps, double weight_decay, int64_t step, double grad_scale,
@@ -199,6 +204,56 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerNormBackward(
   return std::make_tuple(dx, dbr, dgamma, dbeta);
 }
 
+void checkBf16Matrix(const at::Tensor& t, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.is_contiguous() && t.scalar_type() == at::kBFloat16 && t.dim() >= 1 &&
+                  t.size(-1) % 8 == 0 && t.size(-1) > 0 && t.size(-1) <= INT32_MAX,
+              name, " must be a contiguous bf16 CUDA tensor whose last dimension is a multiple of 8");
+}
+
+at::Tensor geluForward(at::Tensor x, bool tanh_form) {
+  checkBf16Matrix(x, "x");
+  c10::cuda::CUDAGuard guard(x.device());
+  x = aligned16(x);
+  at::Tensor y = at::empty_like(x);
+  cudaError_t e = launchGeluForward(x.data_ptr(), y.data_ptr(), x.numel(), tanh_form,
+                                    c10::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(e == cudaSuccess, "gelu forward launch failed: ", cudaGetErrorString(e));
+  return y;
+}
+
+// Column sums of dy or, with `gelu_x`, of dx = dy * gelu'(gelu_x), in `out_dtype`; and dx.
+std::tuple<at::Tensor, at::Tensor> columnSumOf(at::Tensor dy, std::optional<at::Tensor> gelu_x, bool tanh_form,
+                                               at::ScalarType out_dtype) {
+  checkBf16Matrix(dy, "dy");
+  TORCH_CHECK(out_dtype == at::kFloat || out_dtype == at::kBFloat16, "the sums are fp32 or bf16");
+  c10::cuda::CUDAGuard guard(dy.device());
+  dy = aligned16(dy);
+  at::Tensor x, dx;
+  if (gelu_x.has_value()) {
+    checkBf16Matrix(*gelu_x, "x");
+    TORCH_CHECK(gelu_x->sizes() == dy.sizes() && gelu_x->device() == dy.device(), "x and dy must be equally shaped");
+    x = aligned16(*gelu_x);
+    dx = at::empty_like(dy);
+  }
+  const int64_t cols = dy.size(-1), rows = dy.numel() / cols;
+  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  at::Tensor out = at::empty({cols}, dy.options().dtype(out_dtype));
+  at::Tensor partial = at::empty({(int64_t)columnSumStrips(rows, (int)cols, sms), cols}, dy.options().dtype(at::kFloat));
+  cudaError_t e = launchColumnSum(dy.data_ptr(), x.defined() ? x.data_ptr() : nullptr, tanh_form,
+                                  dx.defined() ? dx.data_ptr() : nullptr, partial.data_ptr<float>(), out.data_ptr(),
+                                  out_dtype == at::kBFloat16, rows, (int)cols, sms, c10::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(e == cudaSuccess, "column sum launch failed: ", cudaGetErrorString(e));
+  return std::make_tuple(dx, out);
+}
+
+at::Tensor columnSum(at::Tensor dy, at::ScalarType out_dtype) {
+  return std::get<1>(columnSumOf(dy, std::nullopt, false, out_dtype));
+}
+
+std::tuple<at::Tensor, at::Tensor> geluBackward(at::Tensor dy, at::Tensor x, bool tanh_form, at::ScalarType sum_dtype) {
+  return columnSumOf(dy, x, tanh_form, sum_dtype);
+}
+
 void checkLogits(const at::Tensor& logits, const at::Tensor& targets) {
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.is_contiguous(),
               "logits must be a contiguous 2-D CUDA tensor");
@@ -284,10 +339,6 @@ void checkLikeX(const at::Tensor& t, const at::Tensor& x, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.device() == x.device() && t.scalar_type() == x.scalar_type() &&
                   t.sizes() == x.sizes() && t.is_contiguous(at::MemoryFormat::ChannelsLast),
               name, " must be like x: device, type, shape, channels-last");
-}
-
-at::Tensor aligned16(const at::Tensor& t) {
-  return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone();
 }
 
 void checkPerChannel(const at::Tensor& t, const at::Tensor& x, const char* name) {
@@ -385,6 +436,9 @@ void bindLocalOps(pybind11::module_& m) {
         py::arg("bias"), py::arg("eps"), py::arg("out_dtype"));
   m.def("add_layer_norm_bwd", &addLayerNormBackward, py::arg("dy"), py::arg("xnew"), py::arg("weight"),
         py::arg("mean"), py::arg("rstd"), py::arg("gres"), py::arg("want_bf16"));
+  m.def("gelu_fwd", &geluForward, py::arg("x"), py::arg("tanh_form"));
+  m.def("gelu_bwd", &geluBackward, py::arg("dy"), py::arg("x"), py::arg("tanh_form"), py::arg("sum_dtype"));
+  m.def("column_sum", &columnSum, py::arg("x"), py::arg("dtype"));
   m.def("batch_norm_fwd", &batchNormForward, py::arg("x"), py::arg("residual"), py::arg("weight"), py::arg("bias"),
         py::arg("running_mean"), py::arg("running_var"), py::arg("tracked"), py::arg("momentum"), py::arg("eps"),
         py::arg("relu"));

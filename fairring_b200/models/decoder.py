@@ -71,16 +71,16 @@ class Block(nn.Module):
         follows it: takes the stream and the output of the block before that is
         still to be added to it, returns the stream and this block's own
         pending output."""
-        from ..ops import add_layer_norm
+        from ..ops import add_layer_norm, linear, linear_gelu
 
         b, s, d = x.shape
         x, h = add_layer_norm(self.ln1, x, pending)
-        q, k, v = self.qkv(h).view(b, s, 3, self.n_head, d // self.n_head).unbind(2)
+        q, k, v = linear(self.qkv, h).view(b, s, 3, self.n_head, d // self.n_head).unbind(2)
         a = F.scaled_dot_product_attention(
             q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), is_causal=True
         )
-        x, h = add_layer_norm(self.ln2, x, self.proj(a.transpose(1, 2).reshape(b, s, d)))
-        return x, self.fc2(F.gelu(self.fc1(h), approximate="tanh"))
+        x, h = add_layer_norm(self.ln2, x, linear(self.proj, a.transpose(1, 2).reshape(b, s, d)))
+        return x, linear(self.fc2, linear_gelu(self.fc1, h, approximate="tanh"))
 
 
 class DecoderLM(nn.Module):
