@@ -12,8 +12,10 @@
 // before the first is used.
 //
 // 1229 x 50265 bf16, an odd vocabulary: torch's kernels and casts take 620 us in both
-// directions, these 85 us.  8192 x 51200 bf16: forward 212 us (3.9 TB/s), backward 277
-// us (6.1 TB/s; 289 us with a block per row instead of per batch), the mean 4 us.
+// directions, these 82 us.  8192 x 51200 bf16: forward 189 us (4.4 TB/s; exp() and the
+// conversions around it keep the issue slots about half busy; 212 us with 512 threads
+// that use a batch before they load the next), backward 276 us (6.1 TB/s; 289 us with
+// a block per row instead of per batch), the mean 4 us.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -38,6 +40,11 @@ template <> struct Vec16<float> {
   static __device__ __forceinline__ void get(const uint4& r, float (&v)[4]) {
     v[0] = __uint_as_float(r.x); v[1] = __uint_as_float(r.y); v[2] = __uint_as_float(r.z); v[3] = __uint_as_float(r.w);
   }
+  static __device__ __forceinline__ float max(const uint4& r) {
+    float v[4];
+    get(r, v);
+    return fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
+  }
   static __device__ __forceinline__ uint4 set(const float (&v)[4]) {
     return make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
   }
@@ -53,6 +60,11 @@ template <> struct Vec16<__nv_bfloat16> {
       v[2 * i] = f.x;
       v[2 * i + 1] = f.y;
     }
+  }
+  static __device__ __forceinline__ float max(const uint4& r) {  // packed: half the comparisons
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+    const float2 m = __bfloat1622float2(__hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+    return fmaxf(m.x, m.y);
   }
   static __device__ __forceinline__ uint4 set(const float (&v)[8]) {
     uint4 r;
@@ -105,9 +117,10 @@ __device__ __forceinline__ float blockReduce(float v, bool is_max, float* scratc
 // loss[r] = logsumexp(row r) - row r[target]; lse[r] kept for the backward.
 // A negative target marks a row that does not count: loss 0.  A target past the
 // vocabulary gives `bad_target`.  One block per row, one sweep over it: a thread
-// rescales its sum once per batch of vectors when its maximum grew.
+// rescales its sum once per batch of vectors when its maximum grew, and the next
+// batch is on its way while this one is used.
 template <typename T, int kThreads>
-__global__ void __launch_bounds__(kThreads, 1024 / kThreads)
+__global__ void __launch_bounds__(kThreads, 1280 / kThreads)
 cross_entropy_fwd_kernel(const T* __restrict__ logits, const int64_t* __restrict__ targets,
                          float* __restrict__ loss, float* __restrict__ lse, int vocab, float bad_target) {
   constexpr int E = Vec16<T>::kElems, U = kCeBatch;
@@ -117,31 +130,35 @@ cross_entropy_fwd_kernel(const T* __restrict__ logits, const int64_t* __restrict
   const RowParts<T> parts(row, vocab);
   const uint4* vecs = reinterpret_cast<const uint4*>(row + parts.head);
   SoftSum a;
-  for (int i = threadIdx.x; i < parts.nvec; i += U * kThreads) {
-    uint4 raw[U];
+  uint4 raw[U];
+  auto fetch = [&](int i) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       constexpr uint32_t w = Vec16<T>::kMinusInf;
       raw[u] = i + u * kThreads < parts.nvec ? vecs[i + u * kThreads] : make_uint4(w, w, w, w);
     }
+  };
+  int i = threadIdx.x;
+  fetch(i);
+  while (i < parts.nvec) {
+    uint4 now[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) now[u] = raw[u];
+    i += U * kThreads;
+    fetch(i);
     float top = a.m;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      float v[E];
-      Vec16<T>::get(raw[u], v);
-#pragma unroll
-      for (int k = 0; k < E; ++k) top = fmaxf(top, v[k]);
-    }
+    for (int u = 0; u < U; ++u) top = fmaxf(top, Vec16<T>::max(now[u]));
     const float ref = SoftSum::reference(top);
-    float s = 0.f;
+    float s[2] = {};
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       float v[E];
-      Vec16<T>::get(raw[u], v);
+      Vec16<T>::get(now[u], v);
 #pragma unroll
-      for (int k = 0; k < E; ++k) s += __expf(v[k] - ref);
+      for (int k = 0; k < E; ++k) s[k & 1] += __expf(v[k] - ref);
     }
-    a.s = a.s * __expf(a.m - ref) + s;
+    a.s = a.s * __expf(a.m - ref) + (s[0] + s[1]);
     a.m = top;
   }
   if ((int)threadIdx.x < parts.head) a.add(toFloat(row[threadIdx.x]));
@@ -225,12 +242,12 @@ cross_entropy_bwd_kernel(const T* logits, T* grad, const int64_t* __restrict__ t
   }
 }
 
-constexpr int kCeFwdWide = 512, kCeFwdNarrow = 128, kCeBwdThreads = 256;
+constexpr int kCeFwdWide = 256, kCeFwdNarrow = 128, kCeBwdThreads = 256;
 
 template <typename T>
 void forwardOf(const void* logits, const int64_t* targets, float* loss, float* lse, int64_t rows, int vocab,
                float bad_target, cudaStream_t stream) {
-  // A row that one batch of 512 threads would not fill takes 128.
+  // A row that one batch of 256 threads would not fill takes 128.
   for (int64_t done = 0; done < rows; done += 1 << 30) {
     const unsigned n = (unsigned)(rows - done < (1 << 30) ? rows - done : (1 << 30));
     const T* at = static_cast<const T*>(logits) + done * vocab;

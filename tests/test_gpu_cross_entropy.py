@@ -27,7 +27,7 @@ def _check(logits, leaf, loss, targets):
 
 
 # one thread's worth, remainders on both sides of the 16-byte vectors, the batch of the narrow block
-# (128 x 4 vectors) and of the wide one (512 x 4), where the wide block takes over, two pieces of the backward
+# (128 x 4 vectors) and of the wide one (256 x 4), where the wide block takes over, two pieces of the backward
 @pytest.mark.parametrize("vocab", [1, 7, 8, 9, 1000, 1001, 4095, 4097, 8191, 8192, 8193, 16383, 16384, 16385, 50265])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_every_row_length(vocab, dtype):
