@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "local_kernels.h"
+#include "vec8.cuh"
 
 namespace fairring {
 namespace {
@@ -24,37 +25,22 @@ namespace {
 constexpr int kLnThreads = 256;
 
 template <typename T>
-__device__ __forceinline__ void load8(const T* p, float (&v)[8]);
-template <>
-__device__ __forceinline__ void load8<float>(const float* p, float (&v)[8]) {
-  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-template <>
-__device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[8]) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(p);
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __bfloat1622float2(h[i]);
-    v[2 * i] = f.x;
-    v[2 * i + 1] = f.y;
-  }
+__device__ __forceinline__ void load8(const T* p, float (&v)[8]) {
+  Raw8<T> r;
+  r.load(p);
+  r.get(v);
 }
 template <typename T>
-__device__ __forceinline__ void store8(T* p, const float (&v)[8]);
-template <>
-__device__ __forceinline__ void store8<float>(float* p, const float (&v)[8]) {
-  reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-  reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+__device__ __forceinline__ void store8(T* p, const float (&v)[8]) {
+  Raw8<T> r;
+  r.set(v);
+  r.store(p);
 }
-template <>
-__device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* p, const float (&v)[8]) {
-  uint4 raw;
-  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
+
+__device__ __forceinline__ float warpSum(float v) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-  *reinterpret_cast<uint4*>(p) = raw;
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
 // Sum of two values over the block; every thread gets the result.
@@ -182,54 +168,105 @@ layer_norm_bwd_kernel(const TY* __restrict__ dy, const TX* __restrict__ x,
   }
 }
 
-// dgamma[c] = sum over blocks of partial[b][0][c]; dbeta likewise.  A block of
-// 8 warps owns 32 of the 2 x cols columns: warp w sums partial rows w, w+8, ...
-// (one 128-byte line per load, four loads in flight), then the warps' sums
-// are added through shared memory.
-__global__ void __launch_bounds__(256)
+// dgamma[c] = sum over blocks of partial[b][0][c]; dbeta likewise.  A block owns 32
+// of the 2 x cols columns; warp w sums partial rows w, w+32, ... (one 128-byte line
+// per load, eight loads in flight), then the warps' sums are added through shared
+// memory.  Bound by the launch and two trips to L2: 592 rows of 2 x 2048 take 3.9 us;
+// eight warps with four loads in flight took 9.8 us.
+__global__ void __launch_bounds__(1024, 1)
 layer_norm_param_grad_kernel(const float* __restrict__ partial, int nblocks, int cols,
                              float* __restrict__ dgamma, float* __restrict__ dbeta) {
-  __shared__ float acc[8][33];
+  constexpr int W = 32, U = 8;
+  __shared__ float acc[W][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
   const size_t stride = (size_t)2 * cols;
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+  float s = 0.f;
   if (c < 2 * cols) {
-    int b = w;
-    for (; b + 24 < nblocks; b += 32) {
-      s0 += partial[(size_t)b * stride + c];
-      s1 += partial[(size_t)(b + 8) * stride + c];
-      s2 += partial[(size_t)(b + 16) * stride + c];
-      s3 += partial[(size_t)(b + 24) * stride + c];
-    }
-    for (; b < nblocks; b += 8) s0 += partial[(size_t)b * stride + c];
-  }
-  acc[w][lane] = (s0 + s1) + (s2 + s3);
-  __syncthreads();
-  if (w == 0 && c < 2 * cols) {
-    float s = acc[0][lane];
+    for (int b = w; b < nblocks; b += W * U) {
+      float v[U];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) s += acc[i][lane];
-    if (c < cols)
-      dgamma[c] = s;
+      for (int u = 0; u < U; ++u) v[u] = b + u * W < nblocks ? partial[(size_t)(b + u * W) * stride + c] : 0.f;
+#pragma unroll
+      for (int u = 0; u < U; ++u) s += v[u];
+    }
+  }
+  acc[w][lane] = s;
+  __syncthreads();
+  s = warpSum(acc[lane][w]);  // warp w: column w of the block
+  const int mine = blockIdx.x * 32 + w;
+  if (lane == 0 && mine < 2 * cols) {
+    if (mine < cols)
+      dgamma[mine] = s;
     else
-      dbeta[c - cols] = s;
+      dbeta[mine - cols] = s;
   }
 }
 
 // ---- residual add + LayerNorm ---------------------------------------------------
+// Mean of a row and the sum of squared differences from it.  Each warp takes its
+// own mean first and the warps' results are merged, so a row whose mean is large
+// against its deviation keeps its variance.  `scratch` is in two halves that rows
+// alternate between: one barrier per row.
+template <int ITER>
+__device__ __forceinline__ float2 blockMoments(const float (&v)[ITER][8], int cols,
+                                               float2 (&scratch)[2][kLnThreads / 32], int half) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto columnsOf = [&](int w) {
+    int n = 0;
+#pragma unroll
+    for (int it = 0; it < ITER; ++it) n += max(0, min(256, cols - (it * kLnThreads + w * 32) * 8));
+    return (float)n;
+  };
+  float s = 0.f;
+#pragma unroll
+  for (int it = 0; it < ITER; ++it) {
+    if ((it * kLnThreads + (int)threadIdx.x) * 8 < cols) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += v[it][i];
+    }
+  }
+  const float n = columnsOf(warp), mean = warpSum(s) / fmaxf(n, 1.f);
+  float q = 0.f;
+#pragma unroll
+  for (int it = 0; it < ITER; ++it) {
+    if ((it * kLnThreads + (int)threadIdx.x) * 8 < cols) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) q = fmaf(v[it][i] - mean, v[it][i] - mean, q);
+    }
+  }
+  q = warpSum(q);
+  if (lane == 0) scratch[half][warp] = make_float2(mean, q);
+  __syncthreads();
+  // every eight lanes merge the eight warps
+  const float2 t = scratch[half][lane & 7];
+  const float k = columnsOf(lane & 7);
+  auto sum8 = [](float a) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+  };
+  const float all = sum8(k * t.x) / cols, d = t.x - all;
+  return make_float2(all, sum8(t.y + k * d * d));
+}
+static_assert(kLnThreads == 256, "eight warps are merged by eight lanes");
+
 // xnew = x + branch (the fp32 residual stream plus a block's output, bf16 under
 // autocast), y = LayerNorm(xnew).  A separate add reads and writes the stream
 // once more per LayerNorm; here the sum is formed in the registers that the
-// statistics are computed from.
-template <typename TB, typename TY, int ITER>
+// statistics are computed from.  With kPair `y32` receives y in fp32 as well: the
+// stream of a post-LayerNorm block next to its copy for the next GEMM.  With kPair
+// the statistics are blockMoments().
+template <typename TB, typename TY, int ITER, bool kPair>
 __global__ void __launch_bounds__(kLnThreads, ITER == 1 ? 6 : 1)
 add_layer_norm_fwd_kernel(const float* __restrict__ x, const TB* __restrict__ branch,
                           const float* __restrict__ gamma, const float* __restrict__ beta,
-                          float* __restrict__ xnew, TY* __restrict__ y, float* __restrict__ mean_out,
-                          float* __restrict__ rstd_out, int64_t rows, int cols, float eps) {
-  __shared__ float2 scratch[kLnThreads / 32];
-  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+                          float* __restrict__ xnew, TY* __restrict__ y, float* __restrict__ y32,
+                          float* __restrict__ mean_out, float* __restrict__ rstd_out, int64_t rows, int cols,
+                          float eps) {
+  __shared__ float2 scratch[2][kLnThreads / 32];
+  int half = 0;
+  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, half ^= 1) {
     float v[ITER][8];
     float s = 0.f, ss = 0.f;
 #pragma unroll
@@ -248,9 +285,16 @@ add_layer_norm_fwd_kernel(const float* __restrict__ x, const TB* __restrict__ br
         store8<float>(xnew + r * cols + c, v[it]);
       }
     }
-    const float2 t = blockSum2(s, ss, scratch);
-    const float mean = t.x / cols;
-    const float var = fmaxf(t.y / cols - mean * mean, 0.f);
+    float mean, var;
+    if constexpr (kPair) {
+      const float2 t = blockMoments<ITER>(v, cols, scratch, half);
+      mean = t.x;
+      var = t.y / cols;
+    } else {
+      const float2 t = blockSum2(s, ss, scratch[0]);
+      mean = t.x / cols;
+      var = fmaxf(t.y / cols - mean * mean, 0.f);
+    }
     const float rstd = rsqrtf(var + eps);
     if (threadIdx.x == 0) {
       mean_out[r] = mean;
@@ -266,17 +310,19 @@ add_layer_norm_fwd_kernel(const float* __restrict__ x, const TB* __restrict__ br
 #pragma unroll
         for (int i = 0; i < 8; ++i) o[i] = (v[it][i] - mean) * rstd * g[i] + b[i];
         store8<TY>(y + r * cols + c, o);
+        if constexpr (kPair) store8<float>(y32 + r * cols + c, o);
       }
     }
   }
 }
 
-// dx = LayerNorm backward of dy at xnew, plus `gres`, the gradient that reaches
+// dx = LayerNorm backward at xnew of dy (with kPair + `dy32`, what reached y's fp32
+// copy; one of the two may be null), plus `gres`, the gradient that reaches
 // xnew along the residual path (null: none).  dx is the gradient of both
 // addends; `dbranch` (null: not wanted) receives it in bf16 for a bf16 branch.
-template <typename TY, int ITER>
+template <typename TY, int ITER, bool kPair>
 __global__ void __launch_bounds__(kLnThreads, ITER == 1 ? 4 : 1)
-add_layer_norm_bwd_kernel(const TY* __restrict__ dy, const float* __restrict__ xnew,
+add_layer_norm_bwd_kernel(const TY* __restrict__ dy, const float* __restrict__ dy32, const float* __restrict__ xnew,
                           const float* __restrict__ gres, const float* __restrict__ gamma,
                           const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                           float* __restrict__ dx, __nv_bfloat16* __restrict__ dbranch,
@@ -296,9 +342,17 @@ add_layer_norm_bwd_kernel(const TY* __restrict__ dy, const float* __restrict__ x
     for (int it = 0; it < ITER; ++it) {
       const int c = (it * kLnThreads + threadIdx.x) * 8;
       if (c < cols) {
-        float xv[8], dv[8], gv[8];
+        float xv[8], dv[8] = {}, gv[8];
         load8<float>(xnew + r * cols + c, xv);
-        load8<TY>(dy + r * cols + c, dv);
+        if (!kPair || dy != nullptr) load8<TY>(dy + r * cols + c, dv);
+        if constexpr (kPair) {
+          if (dy32 != nullptr) {
+            float e[8];
+            load8<float>(dy32 + r * cols + c, e);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) dv[i] += e[i];
+          }
+        }
         load8<float>(gamma + c, gv);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -342,14 +396,15 @@ add_layer_norm_bwd_kernel(const TY* __restrict__ dy, const float* __restrict__ x
   }
 }
 
-template <typename TB, typename TY>
+template <typename TB, typename TY, bool kPair>
 cudaError_t addFwdDispatch(const float* x, const void* branch, const float* gamma, const float* beta,
-                           float* xnew, void* y, float* mean, float* rstd, int64_t rows, int cols,
-                           float eps, int blocks, cudaStream_t s) {
+                           float* xnew, void* y, float* y32, float* mean, float* rstd, int64_t rows,
+                           int cols, float eps, int blocks, cudaStream_t s) {
   const int iter = (cols / 8 + kLnThreads - 1) / kLnThreads;
 #define FR_ALN_FWD(I)                                                                         \
-  add_layer_norm_fwd_kernel<TB, TY, I><<<blocks, kLnThreads, 0, s>>>(                          \
-      x, static_cast<const TB*>(branch), gamma, beta, xnew, static_cast<TY*>(y), mean, rstd, rows, cols, eps)
+  add_layer_norm_fwd_kernel<TB, TY, I, kPair><<<blocks, kLnThreads, 0, s>>>(                          \
+      x, static_cast<const TB*>(branch), gamma, beta, xnew, static_cast<TY*>(y), y32, mean, rstd, rows, \
+      cols, eps)
   switch (iter) {
     case 1: FR_ALN_FWD(1); break;
     case 2: FR_ALN_FWD(2); break;
@@ -361,14 +416,14 @@ cudaError_t addFwdDispatch(const float* x, const void* branch, const float* gamm
   return cudaGetLastError();
 }
 
-template <typename TY>
-cudaError_t addBwdDispatch(const void* dy, const float* xnew, const float* gres, const float* gamma,
+template <typename TY, bool kPair>
+cudaError_t addBwdDispatch(const void* dy, const float* dy32, const float* xnew, const float* gres, const float* gamma,
                            const float* mean, const float* rstd, float* dx, void* dbranch,
                            float* partial, int64_t rows, int cols, int blocks, cudaStream_t s) {
   const int iter = (cols / 8 + kLnThreads - 1) / kLnThreads;
 #define FR_ALN_BWD(I)                                                                         \
-  add_layer_norm_bwd_kernel<TY, I><<<blocks, kLnThreads, 0, s>>>(                              \
-      static_cast<const TY*>(dy), xnew, gres, gamma, mean, rstd, dx,                           \
+  add_layer_norm_bwd_kernel<TY, I, kPair><<<blocks, kLnThreads, 0, s>>>(                              \
+      static_cast<const TY*>(dy), dy32, xnew, gres, gamma, mean, rstd, dx,                     \
       static_cast<__nv_bfloat16*>(dbranch), partial, rows, cols)
   switch (iter) {
     case 1: FR_ALN_BWD(1); break;
@@ -460,7 +515,7 @@ cudaError_t launchLayerNormBackward(const void* dy, bool y_bf16, const void* x, 
     e = y_bf16 ? bwdDispatch<float, __nv_bfloat16>(dy, x, gamma, mean, rstd, dx, partial, rows, cols, blocks, stream)
                : bwdDispatch<float, float>(dy, x, gamma, mean, rstd, dx, partial, rows, cols, blocks, stream);
   if (e != cudaSuccess) return e;
-  layer_norm_param_grad_kernel<<<(2 * cols + 31) / 32, 256, 0, stream>>>(partial, blocks, cols, dgamma, dbeta);
+  layer_norm_param_grad_kernel<<<(2 * cols + 31) / 32, 1024, 0, stream>>>(partial, blocks, cols, dgamma, dbeta);
   noteLocalLaunch();
   noteLocalLaunch();
   return cudaGetLastError();
@@ -468,35 +523,38 @@ cudaError_t launchLayerNormBackward(const void* dy, bool y_bf16, const void* x, 
 
 cudaError_t launchAddLayerNormForward(const float* x, const void* branch, bool branch_bf16,
                                       const float* gamma, const float* beta, float* xnew, void* y,
-                                      bool y_bf16, float* mean, float* rstd, int64_t rows, int cols,
+                                      bool y_bf16, float* y32, float* mean, float* rstd, int64_t rows, int cols,
                                       float eps, int sm_count, cudaStream_t stream) {
   if (rows <= 0) return cudaSuccess;
   if (cols % 8 != 0 || cols > 8192) return cudaErrorInvalidValue;
   int64_t blocks = (int64_t)sm_count * 6;
   if (blocks > rows) blocks = rows;
-  cudaError_t e;
-  if (branch_bf16)
-    e = y_bf16 ? addFwdDispatch<__nv_bfloat16, __nv_bfloat16>(x, branch, gamma, beta, xnew, y, mean, rstd, rows, cols, eps, (int)blocks, stream)
-               : addFwdDispatch<__nv_bfloat16, float>(x, branch, gamma, beta, xnew, y, mean, rstd, rows, cols, eps, (int)blocks, stream);
-  else
-    e = y_bf16 ? addFwdDispatch<float, __nv_bfloat16>(x, branch, gamma, beta, xnew, y, mean, rstd, rows, cols, eps, (int)blocks, stream)
-               : addFwdDispatch<float, float>(x, branch, gamma, beta, xnew, y, mean, rstd, rows, cols, eps, (int)blocks, stream);
+  using bf16 = __nv_bfloat16;
+  auto f = branch_bf16 ? (y_bf16 ? addFwdDispatch<bf16, bf16, false> : addFwdDispatch<bf16, float, false>)
+                       : (y_bf16 ? addFwdDispatch<float, bf16, false> : addFwdDispatch<float, float, false>);
+  if (y32 != nullptr) {
+    if (!y_bf16) return cudaErrorInvalidValue;
+    f = branch_bf16 ? addFwdDispatch<bf16, bf16, true> : addFwdDispatch<float, bf16, true>;
+  }
+  const cudaError_t e =
+      f(x, branch, gamma, beta, xnew, y, y32, mean, rstd, rows, cols, eps, (int)blocks, stream);
   noteLocalLaunch();
   return e;
 }
 
-cudaError_t launchAddLayerNormBackward(const void* dy, bool y_bf16, const float* xnew, const float* gres,
-                                       const float* gamma, const float* mean, const float* rstd,
+cudaError_t launchAddLayerNormBackward(const void* dy, bool y_bf16, const float* dy32, const float* xnew,
+                                       const float* gres, const float* gamma, const float* mean, const float* rstd,
                                        float* dx, void* dbranch_bf16, float* partial, float* dgamma,
                                        float* dbeta, int64_t rows, int cols, int sm_count,
                                        cudaStream_t stream) {
   if (rows <= 0) return cudaSuccess;
-  if (cols % 8 != 0 || cols > 8192) return cudaErrorInvalidValue;
+  if (cols % 8 != 0 || cols > 8192 || (dy == nullptr && dy32 == nullptr)) return cudaErrorInvalidValue;
   const int blocks = layerNormBackwardBlocks(rows, sm_count);
-  cudaError_t e = y_bf16 ? addBwdDispatch<__nv_bfloat16>(dy, xnew, gres, gamma, mean, rstd, dx, dbranch_bf16, partial, rows, cols, blocks, stream)
-                         : addBwdDispatch<float>(dy, xnew, gres, gamma, mean, rstd, dx, dbranch_bf16, partial, rows, cols, blocks, stream);
+  auto f = y_bf16 ? addBwdDispatch<__nv_bfloat16, false> : addBwdDispatch<float, false>;
+  if (dy32 != nullptr) f = y_bf16 || dy == nullptr ? addBwdDispatch<__nv_bfloat16, true> : addBwdDispatch<float, true>;
+  cudaError_t e = f(dy, dy32, xnew, gres, gamma, mean, rstd, dx, dbranch_bf16, partial, rows, cols, blocks, stream);
   if (e != cudaSuccess) return e;
-  layer_norm_param_grad_kernel<<<(2 * cols + 31) / 32, 256, 0, stream>>>(partial, blocks, cols, dgamma, dbeta);
+  layer_norm_param_grad_kernel<<<(2 * cols + 31) / 32, 1024, 0, stream>>>(partial, blocks, cols, dgamma, dbeta);
   noteLocalLaunch();
   noteLocalLaunch();
   return cudaGetLastError();

@@ -101,6 +101,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> layerNormForward(at::Tensor x, at
               "weight and bias must be contiguous fp32 CUDA vectors of the row length");
   TORCH_CHECK(cols % 8 == 0 && cols <= 8192, "row length must be a multiple of 8, at most 8192");
   c10::cuda::CUDAGuard guard(x.device());
+  x = aligned16(x);
+  gamma = aligned16(gamma);
+  beta = aligned16(beta);
   at::Tensor y = at::empty(x.sizes(), x.options().dtype(out_dtype));
   at::Tensor mean = at::empty({rows}, x.options().dtype(at::kFloat));
   at::Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
@@ -124,6 +127,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> layerNormBackward(at::Tensor dy, 
   const int64_t rows = x.numel() / std::max<int64_t>(cols, 1);
   c10::cuda::CUDAGuard guard(x.device());
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  dy = aligned16(dy);
+  x = aligned16(x);
+  gamma = aligned16(gamma);
   at::Tensor dx = at::empty_like(x);
   at::Tensor dgamma = at::empty({cols}, gamma.options());
   at::Tensor dbeta = at::empty({cols}, gamma.options());
@@ -137,10 +143,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> layerNormBackward(at::Tensor dy, 
   return std::make_tuple(dx, dgamma, dbeta);
 }
 
-// xnew, y, mean, rstd = x + branch, layer_norm(x + branch); x fp32, branch fp32 or bf16.
-std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerNormForward(
+// xnew, y, mean, rstd [, y in fp32] = x + branch, layer_norm(x + branch); x fp32, branch fp32 or
+// bf16.  The last result is undefined unless `want_y32`.
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerNormForward(
     at::Tensor x, at::Tensor branch, at::Tensor gamma, at::Tensor beta, double eps,
-    at::ScalarType out_dtype) {
+    at::ScalarType out_dtype, bool want_y32) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.scalar_type() == at::kFloat && x.dim() >= 1,
               "x must be a contiguous fp32 CUDA tensor");
   TORCH_CHECK(branch.is_cuda() && branch.is_contiguous() && branch.sizes() == x.sizes() &&
@@ -155,39 +162,47 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerNormForward(
               "weight and bias must be contiguous fp32 CUDA vectors of the row length");
   TORCH_CHECK(cols % 8 == 0 && cols <= 8192, "row length must be a multiple of 8, at most 8192");
   c10::cuda::CUDAGuard guard(x.device());
+  x = aligned16(x);
+  branch = aligned16(branch);
+  gamma = aligned16(gamma);
+  beta = aligned16(beta);
   at::Tensor xnew = at::empty_like(x);
-  at::Tensor y = at::empty(x.sizes(), x.options().dtype(out_dtype));
+  at::Tensor y = at::empty(x.sizes(), x.options().dtype(out_dtype)), y32;
+  if (want_y32) y32 = at::empty_like(x);
   at::Tensor mean = at::empty({rows}, x.options());
   at::Tensor rstd = at::empty({rows}, x.options());
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   cudaError_t e = launchAddLayerNormForward(
       x.data_ptr<float>(), branch.data_ptr(), branch.scalar_type() == at::kBFloat16, gamma.data_ptr<float>(),
       beta.data_ptr<float>(), xnew.data_ptr<float>(), y.data_ptr(), out_dtype == at::kBFloat16,
-      mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, (int)cols, (float)eps, sms,
-      c10::cuda::getCurrentCUDAStream());
+      want_y32 ? y32.data_ptr<float>() : nullptr, mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, (int)cols,
+      (float)eps, sms, c10::cuda::getCurrentCUDAStream());
   TORCH_CHECK(e == cudaSuccess, "add_layer_norm forward launch failed: ", cudaGetErrorString(e));
-  return std::make_tuple(xnew, y, mean, rstd);
+  return std::make_tuple(xnew, y, mean, rstd, y32);
 }
 
-// dx (fp32), dx in bf16 (or an undefined tensor), dgamma, dbeta.  `gres`: the
-// gradient that reaches xnew along the residual path, or nothing.
+// dx (fp32), dx in bf16 (or an undefined tensor), dgamma, dbeta.  `dy`: the gradient
+// of y, `dy32`: of its fp32 copy (one may be missing); `gres`: the gradient that
+// reaches xnew along the residual path, or nothing.
 std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerNormBackward(
-    at::Tensor dy, at::Tensor xnew, at::Tensor gamma, at::Tensor mean, at::Tensor rstd,
-    std::optional<at::Tensor> gres, bool want_bf16) {
-  TORCH_CHECK(dy.is_cuda() && dy.is_contiguous() && xnew.is_contiguous() && dy.sizes() == xnew.sizes() &&
-                  xnew.scalar_type() == at::kFloat,
-              "dy and xnew must be contiguous and equally shaped, xnew fp32");
-  TORCH_CHECK(dy.scalar_type() == at::kFloat || dy.scalar_type() == at::kBFloat16, "dy must be fp32 or bf16");
-  const float* gres_ptr = nullptr;
-  if (gres.has_value() && gres->defined()) {
-    TORCH_CHECK(gres->is_cuda() && gres->is_contiguous() && gres->scalar_type() == at::kFloat &&
-                    gres->sizes() == xnew.sizes(),
-                "the residual gradient must be contiguous fp32, shaped like xnew");
-    gres_ptr = gres->data_ptr<float>();
-  }
+    std::optional<at::Tensor> dy, at::Tensor xnew, at::Tensor gamma, at::Tensor mean, at::Tensor rstd,
+    std::optional<at::Tensor> gres, bool want_bf16, std::optional<at::Tensor> dy32) {
+  TORCH_CHECK(xnew.is_cuda() && xnew.is_contiguous() && xnew.scalar_type() == at::kFloat,
+              "xnew must be a contiguous fp32 CUDA tensor");
+  c10::cuda::CUDAGuard guard(xnew.device());
+  auto given = [&](const std::optional<at::Tensor>& t, const char* name, bool fp32) -> at::Tensor {
+    if (!t.has_value() || !t->defined()) return {};
+    TORCH_CHECK(t->is_cuda() && t->is_contiguous() && t->sizes() == xnew.sizes() &&
+                    (t->scalar_type() == at::kFloat || (!fp32 && t->scalar_type() == at::kBFloat16)),
+                name, " must be contiguous, shaped like xnew, fp32", fp32 ? "" : " or bf16");
+    return aligned16(*t);
+  };
+  const at::Tensor d = given(dy, "dy", false), d32 = given(dy32, "dy32", true), res = given(gres, "gres", true);
+  TORCH_CHECK(d.defined() || d32.defined(), "one of dy and dy32 is needed");
+  xnew = aligned16(xnew);
+  gamma = aligned16(gamma);
   const int64_t cols = xnew.size(-1);
   const int64_t rows = xnew.numel() / std::max<int64_t>(cols, 1);
-  c10::cuda::CUDAGuard guard(xnew.device());
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   at::Tensor dx = at::empty_like(xnew);
   at::Tensor dbr;
@@ -196,10 +211,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerNormBackward(
   at::Tensor dbeta = at::empty({cols}, gamma.options());
   at::Tensor partial = at::empty({(int64_t)layerNormBackwardBlocks(rows, sms), 2, cols}, gamma.options());
   cudaError_t e = launchAddLayerNormBackward(
-      dy.data_ptr(), dy.scalar_type() == at::kBFloat16, xnew.data_ptr<float>(), gres_ptr,
-      gamma.data_ptr<float>(), mean.data_ptr<float>(), rstd.data_ptr<float>(), dx.data_ptr<float>(),
-      want_bf16 ? dbr.data_ptr() : nullptr, partial.data_ptr<float>(), dgamma.data_ptr<float>(),
-      dbeta.data_ptr<float>(), rows, (int)cols, sms, c10::cuda::getCurrentCUDAStream());
+      d.defined() ? d.data_ptr() : nullptr, d.defined() && d.scalar_type() == at::kBFloat16,
+      d32.defined() ? d32.data_ptr<float>() : nullptr, xnew.data_ptr<float>(),
+      res.defined() ? res.data_ptr<float>() : nullptr, gamma.data_ptr<float>(), mean.data_ptr<float>(),
+      rstd.data_ptr<float>(), dx.data_ptr<float>(), want_bf16 ? dbr.data_ptr() : nullptr, partial.data_ptr<float>(),
+      dgamma.data_ptr<float>(), dbeta.data_ptr<float>(), rows, (int)cols, sms, c10::cuda::getCurrentCUDAStream());
   TORCH_CHECK(e == cudaSuccess, "add_layer_norm backward launch failed: ", cudaGetErrorString(e));
   return std::make_tuple(dx, dbr, dgamma, dbeta);
 }
@@ -433,9 +449,9 @@ void bindLocalOps(pybind11::module_& m) {
   m.def("cross_entropy_bwd_", &crossEntropyBackwardInPlace, py::arg("logits"), py::arg("targets"),
         py::arg("lse"), py::arg("upstream"), py::arg("scale"), py::arg("count") = py::none());
   m.def("add_layer_norm_fwd", &addLayerNormForward, py::arg("x"), py::arg("branch"), py::arg("weight"),
-        py::arg("bias"), py::arg("eps"), py::arg("out_dtype"));
+        py::arg("bias"), py::arg("eps"), py::arg("out_dtype"), py::arg("want_y32") = false);
   m.def("add_layer_norm_bwd", &addLayerNormBackward, py::arg("dy"), py::arg("xnew"), py::arg("weight"),
-        py::arg("mean"), py::arg("rstd"), py::arg("gres"), py::arg("want_bf16"));
+        py::arg("mean"), py::arg("rstd"), py::arg("gres"), py::arg("want_bf16"), py::arg("dy32") = py::none());
   m.def("gelu_fwd", &geluForward, py::arg("x"), py::arg("tanh_form"));
   m.def("gelu_bwd", &geluBackward, py::arg("dy"), py::arg("x"), py::arg("tanh_form"), py::arg("sum_dtype"));
   m.def("column_sum", &columnSum, py::arg("x"), py::arg("dtype"));

@@ -68,8 +68,8 @@ class _AddLayerNormFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, branch, weight, bias, eps, out_dtype):
-        xnew, y, mean, rstd = _C.add_layer_norm_fwd(x.contiguous(), branch.contiguous(), weight, bias, eps,
-                                                    out_dtype)
+        xnew, y, mean, rstd, _ = _C.add_layer_norm_fwd(x.contiguous(), branch.contiguous(), weight, bias, eps,
+                                                       out_dtype)
         ctx.save_for_backward(xnew, weight, mean, rstd)
         ctx.set_materialize_grads(False)  # an unused output arrives as None, not as zeros
         ctx.out_dtype = out_dtype

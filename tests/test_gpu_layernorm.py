@@ -1,0 +1,47 @@
+"""The LayerNorm kernels where their groups of warps begin and end, against fp64."""
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _need_gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+
+
+# one thread, one warp full and one column group past it, 2 and 3 warps, one group per block, 8 and 9 warps
+# (two ways to merge them), all 32; one row, fewer rows than groups, more rows than blocks
+@pytest.mark.parametrize("cols", [8, 248, 256, 264, 768, 1032, 2048, 2056, 8184, 8192])
+@pytest.mark.parametrize("rows", [1, 5, 3001])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_layer_norm_against_fp64(cols, rows, dtype):
+    _need_gpu()
+    from fairring_b200.ops import fused_layer_norm
+
+    gen = torch.Generator(device="cuda").manual_seed(cols + rows)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    x = (rand(rows, cols) * 2 + 0.5).to(dtype).requires_grad_(True)
+    w, b = rand(cols).requires_grad_(True), rand(cols).requires_grad_(True)
+    dy = rand(rows, cols).to(dtype)
+    y = fused_layer_norm(x, w, b)
+    grads = torch.autograd.grad(y, [x, w, b], dy)
+    leaves = [t.detach().double().requires_grad_(True) for t in (x, w, b)]
+    want = F.layer_norm(leaves[0], (cols,), leaves[1], leaves[2], 1e-5)
+    wants = torch.autograd.grad(want, leaves, dy.double())
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22
+    for got, ref in zip([y, grads[0]], [want, wants[0]]):  # a rounding of the type, and of the fp32 terms of the sum
+        assert ((got.double() - ref).abs() <= eps * ref.abs() + 4e-6 * max(1.0, float(ref.abs().max()))).all()
+    for got, ref in zip(grads[1:], wants[1:]):  # fp32 sums over the rows
+        assert ((got.double() - ref).abs() <= 1e-5 * (rows ** 0.5 + 1) * 4).all()
+
+
+def test_rows_off_a_16_byte_boundary():
+    _need_gpu()
+    from fairring_b200.ops import fused_layer_norm
+
+    x = torch.randn(5 * 64 + 1, device="cuda")[1:].view(5, 64)
+    w, b = torch.ones(65, device="cuda")[1:], torch.zeros(65, device="cuda")[1:]
+    torch.testing.assert_close(fused_layer_norm(x, w, b), F.layer_norm(x, (64,)), rtol=1e-5, atol=1e-5)
