@@ -46,6 +46,7 @@ SOURCES = [
     "kernels/layernorm.cu",
     "kernels/cross_entropy.cu",
     "kernels/batchnorm.cu",
+    "kernels/maxpool.cu",
     "kernels/gelu.cu",
     "kernels/noalloc_allreduce.cu",
     "kernels/pipe_allreduce.cu",

@@ -50,12 +50,11 @@ __device__ __forceinline__ void loadChannels(const float* p, int group, float (&
 // Vectors in flight per thread and stream: 64 bytes.
 template <typename T> constexpr int kBnUnroll = sizeof(T) == 2 ? 4 : 2;
 
-// part[block][0][c] = mean and part[block][1][c] = M2 of this block's rows;
-// counts[block] = how many rows those are.
+// part[block][0][c] = mean and part[block][1][c] = M2 of this block's rows, of which
+// there are as many as rowsOfBlock() says.
 template <typename T>
 __global__ void __launch_bounds__(kBnThreads, 4)
-bn_stats_kernel(const T* __restrict__ x, int64_t nvec, int groups, float* __restrict__ part,
-                float* __restrict__ counts) {
+bn_stats_kernel(const T* __restrict__ x, int64_t nvec, int groups, float* __restrict__ part) {
   constexpr int U = kBnUnroll<T>;
   const int64_t stride = (int64_t)gridDim.x * kBnThreads;
   int64_t i = (int64_t)blockIdx.x * kBnThreads + threadIdx.x;
@@ -118,68 +117,68 @@ bn_stats_kernel(const T* __restrict__ x, int64_t nvec, int groups, float* __rest
     }
     part[(size_t)blockIdx.x * 2 * channels + c] = mean;
     part[((size_t)blockIdx.x * 2 + 1) * channels + c] = m2;
-    if (c == 0) counts[blockIdx.x] = count;
   }
 }
 
-// Sum over the 32 warps of a block, one column per lane; warp 0 has the result.
-__device__ __forceinline__ double sumOverWarps(double v, double (&sm)[kBnFinishWarps][33]) {
+// Sum over the 32 warps of a block of what each lane holds for its column: warp w
+// gets column w's.
+__device__ __forceinline__ double sumOfColumn(double v, double (&sm)[kBnFinishWarps][33]) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   __syncthreads();
   sm[w][lane] = v;
   __syncthreads();
-  double t = 0.0;
-  if (w == 0) {
-#pragma unroll 8
-    for (int i = 0; i < kBnFinishWarps; ++i) t += sm[i][lane];
-  }
+  double t = sm[lane][w];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   return t;
 }
 
 // Merges the blocks' statistics, 32 channels per block, and updates the running ones.
+// `members`: rows that a block of the first pass visits at a time.
 __global__ void __launch_bounds__(kBnFinishWarps * 32, 1)
-bn_finish_stats_kernel(const float* __restrict__ part, const float* __restrict__ counts, int nparts,
-                       int channels, int64_t rows, float eps, float momentum, float* __restrict__ mean_out,
-                       float* __restrict__ rstd_out, float* __restrict__ running_mean,
-                       float* __restrict__ running_var, int64_t* __restrict__ tracked) {
+bn_finish_stats_kernel(const float* __restrict__ part, int nparts, int members, int channels, int64_t rows,
+                       float eps, float momentum, float* __restrict__ mean_out, float* __restrict__ rstd_out,
+                       float* __restrict__ running_mean, float* __restrict__ running_var,
+                       int64_t* __restrict__ tracked) {
   __shared__ double sm[kBnFinishWarps][33];
-  __shared__ double sm_mean[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
-  float mean[kBnFinishLoads], m2[kBnFinishLoads];
+  const float first = c < channels ? part[c] : 0.f;  // block 0's mean: what the others are merged around
+  // Rows of block b: whole rounds of the grid, and its share of the last one.
+  const int64_t round = (int64_t)nparts * members;
+  const int whole = (int)(rows / round) * members, rest = (int)(rows % round);
+  double d = 0.0, q = 0.0;
+  for (int b0 = w; b0 < nparts; b0 += kBnFinishLoads / 2 * kBnFinishWarps) {
+    float mean[kBnFinishLoads / 2], m2[kBnFinishLoads / 2];
 #pragma unroll
-  for (int j = 0; j < kBnFinishLoads; ++j) {
-    const int b = w + j * kBnFinishWarps;
-    const bool in = b < nparts && c < channels;
-    mean[j] = in ? part[(size_t)b * 2 * channels + c] : 0.f;
-    m2[j] = in ? part[((size_t)b * 2 + 1) * channels + c] : 0.f;
-  }
-  double t = 0.0;
+    for (int j = 0; j < kBnFinishLoads / 2; ++j) {
+      const int b = b0 + j * kBnFinishWarps;
+      const bool in = b < nparts && c < channels;
+      mean[j] = in ? part[(size_t)b * 2 * channels + c] : 0.f;
+      m2[j] = in ? part[((size_t)b * 2 + 1) * channels + c] : 0.f;
+    }
 #pragma unroll
-  for (int j = 0; j < kBnFinishLoads; ++j) {
-    const int b = w + j * kBnFinishWarps;
-    if (b < nparts) t += (double)counts[b] * mean[j];
-  }
-  t = sumOverWarps(t, sm);
-  if (w == 0) sm_mean[lane] = t / (double)rows;
-  __syncthreads();
-  const double mu = sm_mean[lane];
-  t = 0.0;
-#pragma unroll
-  for (int j = 0; j < kBnFinishLoads; ++j) {
-    const int b = w + j * kBnFinishWarps;
-    if (b < nparts) {
-      const double e = (double)mean[j] - mu;
-      t += (double)m2[j] + (double)counts[b] * e * e;
+    for (int j = 0; j < kBnFinishLoads / 2; ++j) {
+      const int b = b0 + j * kBnFinishWarps;
+      if (b < nparts) {
+        const double n = whole + min(members, max(0, rest - b * members)), e = (double)mean[j] - (double)first;
+        d += n * e;
+        q += (double)m2[j] + n * e * e;
+      }
     }
   }
-  t = sumOverWarps(t, sm);
-  if (w == 0 && c < channels) {
-    const float var = (float)(t / (double)rows);
-    mean_out[c] = (float)mu;
-    rstd_out[c] = rsqrtf(var + eps);
-    running_mean[c] = (1.f - momentum) * running_mean[c] + momentum * (float)mu;
-    running_var[c] = (1.f - momentum) * running_var[c] + momentum * (float)(t / (double)(rows - 1));
+  d = sumOfColumn(d, sm) / (double)rows;
+  q = sumOfColumn(q, sm) / (double)rows;
+  const int mine = blockIdx.x * 32 + w;
+  if (lane == 0 && mine < channels) {
+    const float mu = (float)((double)part[mine] + d);
+    double var = q - d * d;
+    if (var < 0.0) var = 0.0;  // NaN stays
+    mean_out[mine] = mu;
+    rstd_out[mine] = rsqrtf((float)var + eps);
+    running_mean[mine] = (1.f - momentum) * running_mean[mine] + momentum * mu;
+    running_var[mine] =
+        (1.f - momentum) * running_var[mine] + momentum * (float)(var * ((double)rows / (double)(rows - 1)));
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *tracked += 1;
 }
@@ -343,14 +342,15 @@ bn_finish_sums_kernel(const float* __restrict__ part, int nparts, int channels, 
     t1 += v1[j];
     t2 += v2[j];
   }
-  t1 = sumOverWarps(t1, sm);
-  t2 = sumOverWarps(t2, sm);
-  if (w == 0 && c < channels) {
-    const double r = rstd[c];
-    dbeta[c] = (float)t1;
-    dgamma[c] = (float)(t2 * r);
-    coef[c] = (float)(t1 / (double)rows);
-    coef[channels + c] = (float)(t2 * r * r / (double)rows);
+  t1 = sumOfColumn(t1, sm);
+  t2 = sumOfColumn(t2, sm);
+  const int mine = blockIdx.x * 32 + w;
+  if (lane == 0 && mine < channels) {
+    const double r = rstd[mine];
+    dbeta[mine] = (float)t1;
+    dgamma[mine] = (float)(t2 * r);
+    coef[mine] = (float)(t1 / (double)rows);
+    coef[channels + mine] = (float)(t2 * r * r / (double)rows);
   }
 }
 
@@ -426,10 +426,9 @@ cudaError_t forwardOf(const BatchNormShape& s, const void* x, const void* residu
   const T* xt = static_cast<const T*>(x);
   const T* rt = static_cast<const T*>(residual);
   T* yt = static_cast<T*>(y);
-  float* counts = part + (size_t)nparts * 2 * s.channels;
-  bn_stats_kernel<T><<<nparts, kBnThreads, 0, stream>>>(xt, nvec, groups, part, counts);
+  bn_stats_kernel<T><<<nparts, kBnThreads, 0, stream>>>(xt, nvec, groups, part);
   bn_finish_stats_kernel<<<(s.channels + 31) / 32, kBnFinishWarps * 32, 0, stream>>>(
-      part, counts, nparts, s.channels, s.rows, eps, momentum, mean, rstd, running_mean, running_var, tracked);
+      part, nparts, kBnThreads / groups, s.channels, s.rows, eps, momentum, mean, rstd, running_mean, running_var, tracked);
   const unsigned blocks = streamBlocks(nvec, 4, sm_count);
 #define FR_BN_APPLY(R, A) \
   bn_apply_kernel<T, R, A><<<blocks, kBnThreads, 0, stream>>>(xt, rt, yt, mean, rstd, gamma, beta, nvec, groups)
@@ -494,7 +493,7 @@ int batchNormParts(const BatchNormShape& s, int sm_count) {
 
 int64_t batchNormScratchFloats(const BatchNormShape& s, int sm_count) {
   const int64_t nparts = batchNormParts(s, sm_count);
-  return nparts * 2 * s.channels + (nparts > 2 * s.channels ? nparts : 2 * s.channels);
+  return nparts * 2 * s.channels + 2 * s.channels;
 }
 
 cudaError_t launchBatchNormForward(const BatchNormShape& s, bool bf16, const void* x, const void* residual, void* y,

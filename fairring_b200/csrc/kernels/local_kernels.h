@@ -107,6 +107,17 @@ int columnSumStrips(int64_t rows, int cols, int sm_count);
 cudaError_t launchColumnSum(const void* dy, const void* gelu_x, bool tanh_form, void* dx, float* partial, void* out,
                             bool out_bf16, int64_t rows, int cols, int sm_count, cudaStream_t stream);
 
+// Max pooling of a channels-last tensor, fp32 or bf16, channels a multiple of 8, square windows of at
+// most 16 x 16; all tensors 16-byte aligned.  `chosen`: one byte per output element, the position of
+// the largest element in its window.
+struct PoolShape {
+  int images, channels, in_h, in_w, out_h, out_w, window, stride, pad;
+};
+cudaError_t launchMaxPoolForward(const PoolShape& s, bool bf16, const void* x, void* y, void* chosen,
+                                 cudaStream_t stream);
+cudaError_t launchMaxPoolBackward(const PoolShape& s, bool bf16, const void* dy, const void* chosen, void* dx,
+                                  cudaStream_t stream);
+
 uint64_t localLaunchCountImpl();
 void noteLocalLaunch();
 

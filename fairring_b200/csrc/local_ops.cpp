@@ -428,6 +428,50 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> batchNormBackward(
   TORCH_CHECK(e == cudaSuccess, "batch_norm backward launch failed: ", cudaGetErrorString(e));
   return std::make_tuple(dx, dz, dgamma, dbeta);
 }
+
+PoolShape poolShape(const at::Tensor& x, int64_t window, int64_t stride, int64_t pad) {
+  TORCH_CHECK(x.is_cuda() && x.dim() == 4 && x.is_contiguous(at::MemoryFormat::ChannelsLast) &&
+                  (x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16) && x.size(1) % 8 == 0 &&
+                  x.numel() > 0,
+              "x must be a channels-last fp32 or bf16 CUDA tensor whose channels are a multiple of 8");
+  TORCH_CHECK(window >= 1 && window <= 16 && stride >= 1 && pad >= 0 && 2 * pad <= window &&
+                  x.size(2) + 2 * pad >= window && x.size(3) + 2 * pad >= window && x.numel() / 8 < INT32_MAX,
+              "the window does not fit");
+  const int64_t oh = (x.size(2) + 2 * pad - window) / stride + 1, ow = (x.size(3) + 2 * pad - window) / stride + 1;
+  return {(int)x.size(0), (int)x.size(1), (int)x.size(2), (int)x.size(3), (int)oh, (int)ow, (int)window, (int)stride,
+          (int)pad};
+}
+
+// y and, one byte per element of it, which element of the window it is.
+std::tuple<at::Tensor, at::Tensor> maxPoolForward(at::Tensor x, int64_t window, int64_t stride, int64_t pad) {
+  const PoolShape s = poolShape(x, window, stride, pad);
+  c10::cuda::CUDAGuard guard(x.device());
+  x = aligned16(x);
+  const at::Tensor y = at::empty({s.images, s.channels, s.out_h, s.out_w}, x.options(), at::MemoryFormat::ChannelsLast);
+  const at::Tensor chosen = at::empty({y.numel()}, x.options().dtype(at::kByte));
+  cudaError_t e = launchMaxPoolForward(s, x.scalar_type() == at::kBFloat16, x.data_ptr(), y.data_ptr(),
+                                       chosen.data_ptr(), c10::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(e == cudaSuccess, "max_pool forward launch failed: ", cudaGetErrorString(e));
+  return std::make_tuple(y, chosen);
+}
+
+at::Tensor maxPoolBackward(at::Tensor dy, at::Tensor x, at::Tensor chosen, int64_t window, int64_t stride, int64_t pad) {
+  const PoolShape s = poolShape(x, window, stride, pad);
+  TORCH_CHECK(dy.is_cuda() && dy.device() == x.device() && dy.scalar_type() == x.scalar_type() && dy.dim() == 4 &&
+                  dy.size(0) == s.images && dy.size(1) == s.channels && dy.size(2) == s.out_h &&
+                  dy.size(3) == s.out_w && dy.is_contiguous(at::MemoryFormat::ChannelsLast),
+              "dy must be channels-last and shaped like the output");
+  TORCH_CHECK(chosen.is_cuda() && chosen.scalar_type() == at::kByte && chosen.is_contiguous() &&
+                  chosen.numel() == dy.numel(),
+              "chosen must hold one byte per output element");
+  c10::cuda::CUDAGuard guard(x.device());
+  dy = aligned16(dy);
+  const at::Tensor dx = at::empty_like(x, x.options(), at::MemoryFormat::ChannelsLast);
+  cudaError_t e = launchMaxPoolBackward(s, x.scalar_type() == at::kBFloat16, dy.data_ptr(), chosen.data_ptr(),
+                                        dx.data_ptr(), c10::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(e == cudaSuccess, "max_pool backward launch failed: ", cudaGetErrorString(e));
+  return dx;
+}
 }  // namespace
 
 uint64_t localLaunchCount() { return localLaunchCountImpl(); }
@@ -460,6 +504,9 @@ void bindLocalOps(pybind11::module_& m) {
         py::arg("relu"));
   m.def("batch_norm_bwd", &batchNormBackward, py::arg("dy"), py::arg("x"), py::arg("y"), py::arg("weight"),
         py::arg("bias"), py::arg("mean"), py::arg("rstd"), py::arg("relu"));
+  m.def("max_pool_fwd", &maxPoolForward, py::arg("x"), py::arg("window"), py::arg("stride"), py::arg("pad"));
+  m.def("max_pool_bwd", &maxPoolBackward, py::arg("dy"), py::arg("x"), py::arg("chosen"), py::arg("window"),
+        py::arg("stride"), py::arg("pad"));
   m.def("layer_norm_fwd", &layerNormForward, py::arg("x"), py::arg("weight"), py::arg("bias"),
         py::arg("eps"), py::arg("out_dtype"));
   m.def("layer_norm_bwd", &layerNormBackward, py::arg("dy"), py::arg("x"), py::arg("weight"),

@@ -2,7 +2,8 @@
 image-classification data-parallel workload: many small gradient buckets, which
 stresses the small-message (one-shot) path of the backend.  Plain PyTorch
 layers; on channels-last activations BatchNorm, residual add and ReLU run as
-one fused op (:func:`fairring_b200.ops.batch_norm_act`).
+one fused op (:func:`fairring_b200.ops.batch_norm_act`), and the pooling has
+kernels of its own.
 """
 
 from __future__ import annotations
@@ -83,9 +84,9 @@ class ResNet50(nn.Module):
         return sum(p.numel() for p in self.parameters())
 
     def forward(self, images: torch.Tensor, labels: torch.Tensor | None = None):
-        from ..ops import batch_norm_act
+        from ..ops import batch_norm_act, max_pool
 
-        x = self.maxpool(batch_norm_act(self.bn1, self.conv1(images), relu=self.relu))
+        x = max_pool(self.maxpool, batch_norm_act(self.bn1, self.conv1(images), relu=self.relu))
         x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
         logits = self.fc(torch.flatten(self.avgpool(x), 1))
         if labels is None:
