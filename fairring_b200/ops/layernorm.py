@@ -16,8 +16,12 @@ import torch
 import torch.nn as nn
 
 from .. import _C
+from ._plain import plain_autograd
 
 
+# The nodes below are used where torch looks into an autograd function (tracing, compilation) or
+# refuses it (its transforms); otherwise the same nodes are native, ``_C.layer_norm`` and
+# ``_C.add_layer_norm``, which cost a fraction of the host time.
 class _FusedLayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, eps, out_dtype):
@@ -42,7 +46,7 @@ def fused_layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, 
     dtype inside an autocast region and to ``x.dtype`` otherwise."""
     if out_dtype is None:
         out_dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
-    return _FusedLayerNormFn.apply(x, weight, bias, eps, out_dtype)
+    return (_C.layer_norm if plain_autograd() else _FusedLayerNormFn.apply)(x, weight, bias, eps, out_dtype)
 
 
 class FusedLayerNorm(nn.LayerNorm):
@@ -58,7 +62,7 @@ class FusedLayerNorm(nn.LayerNorm):
         out_dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
         if out_dtype not in (torch.float32, torch.bfloat16):
             return super().forward(x)
-        return _FusedLayerNormFn.apply(x, self.weight, self.bias, self.eps, out_dtype)
+        return fused_layer_norm(x, self.weight, self.bias, self.eps, out_dtype)
 
 
 class _AddLayerNormFn(torch.autograd.Function):
@@ -69,7 +73,7 @@ class _AddLayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, branch, weight, bias, eps, out_dtype):
         xnew, y, mean, rstd, _ = _C.add_layer_norm_fwd(x.contiguous(), branch.contiguous(), weight, bias, eps,
-                                                       out_dtype)
+                                                    out_dtype)
         ctx.save_for_backward(xnew, weight, mean, rstd)
         ctx.set_materialize_grads(False)  # an unused output arrives as None, not as zeros
         ctx.out_dtype = out_dtype
@@ -102,6 +106,7 @@ def add_layer_norm(norm: nn.LayerNorm, x: torch.Tensor, branch: torch.Tensor | N
     if fusable:
         out_dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
         if out_dtype in (torch.float32, torch.bfloat16):
-            return _AddLayerNormFn.apply(x, branch, norm.weight, norm.bias, norm.eps, out_dtype)
+            apply = _C.add_layer_norm if plain_autograd() else _AddLayerNormFn.apply
+            return apply(x, branch, norm.weight, norm.bias, norm.eps, out_dtype)
     xnew = x + branch
     return xnew, norm(xnew)

@@ -64,9 +64,11 @@ class FlatAdamW:
     def _run(self, a: int, b: int, grad_scale: float) -> None:
         if b <= a:
             return
-        _C.adamw_flat_(self.param[a:b], self.grad[a:b], self.exp_avg[a:b], self.exp_avg_sq[a:b], self.lr,
-                       self.betas[0], self.betas[1], self.eps, self.weight_decay,
-                       self.step_count, grad_scale, None if self.shadow is None else self.shadow[a:b])
+        flat = (self.param, self.grad, self.exp_avg, self.exp_avg_sq, self.shadow)
+        if (a, b) != (0, self.param.numel()):
+            flat = tuple(None if t is None else t[a:b] for t in flat)
+        _C.adamw_flat_(*flat[:4], self.lr, self.betas[0], self.betas[1], self.eps, self.weight_decay,
+                       self.step_count, grad_scale, flat[4])
 
     def zero_grad(self, set_to_none: bool = True) -> None:  # noqa: ARG002
         """Gradients are overwritten by the next backward; nothing to do."""
