@@ -48,6 +48,7 @@ SOURCES = [
     "kernels/batchnorm.cu",
     "kernels/maxpool.cu",
     "kernels/gelu.cu",
+    "kernels/embedding.cu",
     "kernels/noalloc_allreduce.cu",
     "kernels/pipe_allreduce.cu",
 ]

@@ -118,6 +118,13 @@ cudaError_t launchMaxPoolForward(const PoolShape& s, bool bf16, const void* x, v
 cudaError_t launchMaxPoolBackward(const PoolShape& s, bool bf16, const void* dy, const void* chosen, void* dx,
                                   cudaStream_t stream);
 
+// x[b][s] = table[tokens[b][s]] + pos[s], rows of d floats (a multiple of 4), 16-byte aligned.
+cudaError_t launchEmbedForward(const int64_t* tokens, const float* table, const float* pos, float* x, int batch, int seq,
+                               int64_t vocab, int d, cudaStream_t stream);
+// dtable[tokens[b][s]] += dx[b][s]; dpos[s] = sum over b of dx[b][s].
+cudaError_t launchEmbedBackward(const float* dx, const int64_t* tokens, float* dtable, float* dpos, int batch, int seq,
+                                int64_t vocab, int d, cudaStream_t stream);
+
 uint64_t localLaunchCountImpl();
 void noteLocalLaunch();
 

@@ -473,6 +473,63 @@ at::Tensor maxPoolBackward(at::Tensor dy, at::Tensor x, at::Tensor chosen, int64
   return dx;
 }
 
+void checkTokens(const at::Tensor& tokens, int64_t positions) {
+  TORCH_CHECK(tokens.is_cuda() && tokens.dim() == 2 && tokens.scalar_type() == at::kLong && tokens.is_contiguous() &&
+                  tokens.numel() < INT32_MAX && tokens.size(1) <= positions,
+              "tokens must be a contiguous [batch, sequence] int64 CUDA tensor, no longer than the positions");
+}
+
+// table[tokens] + pos[0..sequence), fp32.
+at::Tensor embedForward(at::Tensor tokens, at::Tensor table, at::Tensor pos) {
+  for (const at::Tensor& t : {table, pos})
+    TORCH_CHECK(t.is_cuda() && t.device() == tokens.device() && t.dim() == 2 && t.scalar_type() == at::kFloat &&
+                    t.is_contiguous() && t.size(1) == table.size(1) && t.size(1) % 8 == 0 &&
+                    reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0,
+                "the tables must be contiguous, 16-byte aligned fp32 CUDA matrices of equal width, a multiple of 8");
+  checkTokens(tokens, pos.size(0));
+  c10::cuda::CUDAGuard guard(tokens.device());
+  at::Tensor x = at::empty({tokens.size(0), tokens.size(1), table.size(1)}, table.options());
+  cudaError_t e = launchEmbedForward(tokens.data_ptr<int64_t>(), table.data_ptr<float>(), pos.data_ptr<float>(),
+                                     x.data_ptr<float>(), (int)tokens.size(0), (int)tokens.size(1), table.size(0),
+                                     (int)table.size(1), c10::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(e == cudaSuccess, "embedding forward launch failed: ", cudaGetErrorString(e));
+  return x;
+}
+
+// Gradients of the table and of the positions: `dx` reached the lookup, `dlow` (bf16) the
+// table's bf16 copy; either may be missing.
+std::tuple<at::Tensor, at::Tensor> embedBackward(std::optional<at::Tensor> dx, std::optional<at::Tensor> dlow,
+                                                 at::Tensor tokens, int64_t vocab, int64_t positions, int64_t d) {
+  checkTokens(tokens, positions);
+  c10::cuda::CUDAGuard guard(tokens.device());
+  auto fopt = tokens.options().dtype(at::kFloat);
+  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  const auto stream = c10::cuda::getCurrentCUDAStream();
+  at::Tensor dtable;
+  if (dlow.has_value() && dlow->defined()) {
+    TORCH_CHECK(dlow->is_cuda() && dlow->device() == tokens.device() && dlow->scalar_type() == at::kBFloat16 &&
+                    dlow->is_contiguous() && dlow->dim() == 2 && dlow->size(0) == vocab && dlow->size(1) == d,
+                "dlow must be a contiguous bf16 matrix shaped like the table");
+    const at::Tensor low = aligned16(*dlow);
+    dtable = at::empty({vocab, d}, fopt);
+    cudaError_t e = launchBf16GradToF32(dtable.data_ptr<float>(), low.data_ptr(), dtable.numel(), false, sms, stream);
+    TORCH_CHECK(e == cudaSuccess, "embedding backward launch failed: ", cudaGetErrorString(e));
+  } else {
+    dtable = at::zeros({vocab, d}, fopt);
+  }
+  if (!dx.has_value() || !dx->defined()) return std::make_tuple(dtable, at::zeros({positions, d}, fopt));
+  TORCH_CHECK(dx->is_cuda() && dx->device() == tokens.device() && dx->scalar_type() == at::kFloat &&
+                  dx->is_contiguous() && dx->numel() == tokens.numel() * d && d % 8 == 0,
+              "dx must be contiguous fp32 with one row per token");
+  const at::Tensor g = aligned16(*dx);
+  at::Tensor dpos = tokens.size(1) < positions ? at::zeros({positions, d}, fopt) : at::empty({positions, d}, fopt);
+  cudaError_t e = launchEmbedBackward(g.data_ptr<float>(), tokens.data_ptr<int64_t>(), dtable.data_ptr<float>(),
+                                      dpos.data_ptr<float>(), (int)tokens.size(0), (int)tokens.size(1), vocab, (int)d,
+                                      stream);
+  TORCH_CHECK(e == cudaSuccess, "embedding backward launch failed: ", cudaGetErrorString(e));
+  return std::make_tuple(dtable, dpos);
+}
+
 // ---- autograd nodes ------------------------------------------------------------
 // LayerNorm and the loss as native nodes: one call from Python forward and none backward.  For
 // 777 x 4104 rows the kernels take 27 us of a pass that took 110 us with Python nodes.
@@ -604,6 +661,9 @@ void bindLocalOps(pybind11::module_& m) {
   m.def("max_pool_fwd", &maxPoolForward, py::arg("x"), py::arg("window"), py::arg("stride"), py::arg("pad"));
   m.def("max_pool_bwd", &maxPoolBackward, py::arg("dy"), py::arg("x"), py::arg("chosen"), py::arg("window"),
         py::arg("stride"), py::arg("pad"));
+  m.def("embed_fwd", &embedForward, py::arg("tokens"), py::arg("table"), py::arg("pos"));
+  m.def("embed_bwd", &embedBackward, py::arg("dx"), py::arg("dlow"), py::arg("tokens"), py::arg("vocab"),
+        py::arg("positions"), py::arg("d"));
   m.def("layer_norm_fwd", &layerNormForward, py::arg("x"), py::arg("weight"), py::arg("bias"),
         py::arg("eps"), py::arg("out_dtype"));
   m.def("layer_norm_bwd", &layerNormBackward, py::arg("dy"), py::arg("x"), py::arg("weight"),

@@ -108,9 +108,10 @@ class DecoderLM(nn.Module):
         return sum(p.numel() for p in self.parameters())
 
     def forward(self, tokens: torch.Tensor, targets: torch.Tensor | None = None):
+        from ..ops import tied_embedding
+
         b, s = tokens.shape
-        pos = torch.arange(s, device=tokens.device)
-        x = self.tok(tokens) + self.pos(pos)
+        x, table = tied_embedding(self.tok, self.pos, tokens)
         if self.cfg.fused_residual and self.cfg.fused_norm and x.is_cuda and x.dtype == torch.float32:
             from ..ops import add_layer_norm
 
@@ -122,7 +123,7 @@ class DecoderLM(nn.Module):
             for blk in self.blocks:
                 x = blk(x)
             x = self.ln_f(x)
-        logits = F.linear(x, self.tok.weight)  # tied output embedding
+        logits = F.linear(x, table)  # tied output embedding
         if targets is None:
             return logits
         if self.cfg.fused_loss and logits.is_cuda:

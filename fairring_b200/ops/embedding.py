@@ -1,0 +1,62 @@
+"""Token plus position embedding of a model whose token table is also its output
+projection (``csrc/kernels/embedding.cu``).
+"""
+
+from __future__ import annotations
+
+import torch
+import torch.nn as nn
+
+from .. import _C
+from ._plain import plain_autograd, plain_module
+
+
+class _TiedEmbeddingFn(torch.autograd.Function):
+    """The embedded tokens and the table's bf16 copy for the projection: one node for both uses of
+    the table, so that its gradient is built once."""
+
+    @staticmethod
+    def forward(ctx, tokens, table, pos):
+        ctx.save_for_backward(tokens)
+        ctx.set_materialize_grads(False)  # an unused output arrives as None, not as zeros
+        ctx.vocab, ctx.positions, ctx.d = table.shape[0], pos.shape[0], table.shape[1]
+        return _C.embed_fwd(tokens, table, pos), table.to(torch.bfloat16)
+
+    @staticmethod
+    def backward(ctx, dx, dlow):
+        (tokens,) = ctx.saved_tensors
+        if dx is None and dlow is None:
+            return None, None, None
+        if torch.is_grad_enabled():  # the graph of this backward is wanted: torch's own ops have one
+            scatter = torch.ops.aten.embedding_dense_backward
+            dtable = dlow.float() if dlow is not None else None
+            if dx is None:
+                return None, dtable, None
+            rows = scatter(dx, tokens, ctx.vocab, -1, False)
+            places = torch.arange(tokens.shape[1], device=tokens.device).expand_as(tokens)
+            return None, rows if dtable is None else dtable + rows, scatter(dx, places, ctx.positions, -1, False)
+        dx = None if dx is None else dx.contiguous()
+        dlow = None if dlow is None else dlow.contiguous()
+        dtable, dpos = _C.embed_bwd(dx, dlow, tokens, ctx.vocab, ctx.positions, ctx.d)
+        return None, dtable, dpos
+
+
+def _plain_table(m: nn.Module) -> bool:
+    return (plain_module(m, nn.Embedding) and m.padding_idx is None and m.max_norm is None and not m.sparse
+            and not m.scale_grad_by_freq and m.weight.requires_grad and m.weight.dtype == torch.float32
+            and m.weight.is_contiguous() and m.weight.data_ptr() % 16 == 0)
+
+
+def tied_embedding(tok: nn.Embedding, pos: nn.Embedding, tokens: torch.Tensor):
+    """``(tok(tokens) + pos(0, 1, ...), table)``: ``table`` is what the output projection multiplies
+    with, ``tok.weight`` or, where the fused form applies, its bf16 copy.  Fused in training under bf16
+    autocast on the GPU.  The rows of equal tokens are added in no fixed order, so under
+    ``torch.use_deterministic_algorithms`` the modules are called."""
+    if (tokens.is_cuda and tokens.dim() == 2 and tokens.dtype == torch.long and tokens.numel() > 0
+            and torch.is_grad_enabled() and torch.is_autocast_enabled("cuda")
+            and torch.get_autocast_dtype("cuda") == torch.bfloat16 and _plain_table(tok) and _plain_table(pos)
+            and tok.weight.device == pos.weight.device == tokens.device and tok.embedding_dim == pos.embedding_dim
+            and tok.embedding_dim % 8 == 0 and tokens.shape[1] <= pos.num_embeddings
+            and not torch.are_deterministic_algorithms_enabled() and plain_autograd()):
+        return _TiedEmbeddingFn.apply(tokens.contiguous(), tok.weight, pos.weight)
+    return tok(tokens) + pos(torch.arange(tokens.shape[1], device=tokens.device)), tok.weight

@@ -1,0 +1,65 @@
+"""The tied embedding against torch's modules."""
+
+import pytest
+import torch
+import torch.nn as nn
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _need_gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+
+
+# one column group, a ragged block, a second block of columns; one sequence, fewer tokens than positions,
+# a token that fills most of the batch
+@pytest.mark.parametrize("d", [8, 264, 1032, 2048])
+@pytest.mark.parametrize("batch,seq,positions", [(1, 1, 1), (5, 33, 40), (9, 64, 64)])
+@pytest.mark.parametrize("use", ["both", "lookup", "projection"])
+def test_matches_torch(d, batch, seq, positions, use):
+    _need_gpu()
+    from fairring_b200.ops import tied_embedding
+
+    gen = torch.Generator(device="cuda").manual_seed(d + seq)
+    tok, pos = nn.Embedding(101, d, device="cuda"), nn.Embedding(positions, d, device="cuda")
+    tokens = torch.randint(0, 101, (batch, seq), device="cuda", generator=gen)
+    tokens[:, ::2] = 7
+    h = torch.randn(50, d, device="cuda", generator=gen).bfloat16()
+    dx = torch.randn(batch, seq, d, device="cuda", generator=gen)
+    dl = torch.randn(50, 101, device="cuda", generator=gen).bfloat16()
+    got = []
+    for fused in (True, False):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            if fused:
+                x, table = tied_embedding(tok, pos, tokens)
+                assert table.dtype == torch.bfloat16
+            else:
+                x, table = tok(tokens) + pos(torch.arange(seq, device="cuda")), tok.weight
+            logits = F.linear(h, table)
+        outs = {"both": ([x, logits], [dx, dl]), "lookup": ([x], [dx]), "projection": ([logits], [dl])}[use]
+        params = [tok.weight, pos.weight] if use != "projection" else [tok.weight]
+        got.append([x, logits, *torch.autograd.grad(outs[0], params, outs[1])])
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    for a, b in zip(got[0][2:], got[1][2:]):  # sums of up to batch * seq / 2 rows in another order
+        assert a.dtype == b.dtype == torch.float32
+        assert float((a - b).abs().max()) <= 2e-6 * (batch * seq) ** 0.5 * max(1.0, float(b.abs().max()))
+
+
+def test_calls_the_modules_where_they_cannot_be_skipped():
+    _need_gpu()
+    from fairring_b200.ops import tied_embedding
+
+    pos, tokens = nn.Embedding(4, 8, device="cuda"), torch.tensor([[0, 1, 2]], device="cuda")
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        for tok in (nn.Embedding(5, 8, device="cuda", padding_idx=0), nn.Embedding(5, 8, device="cuda", max_norm=1.0)):
+            assert tied_embedding(tok, pos, tokens)[1] is tok.weight
+        tok = nn.Embedding(5, 8, device="cuda")
+        seen = []
+        handle = tok.register_forward_hook(lambda *a: seen.append(1))
+        tied_embedding(tok, pos, tokens)
+        handle.remove()
+        assert seen == [1]
+        assert tied_embedding(tok, pos, tokens)[1].dtype == torch.bfloat16
+    assert tied_embedding(tok, pos, tokens)[1] is tok.weight  # no autocast
