@@ -19,7 +19,7 @@
 //
 // ResNet-50, 256 images of 224 x 224 in bf16 (53 BatchNorms): torch's statistics,
 // transform, reduction and gradient kernels took 31.4 ms of a step, its ReLU and add
-// passes around them another 4.9 ms; the kernels here take 9.9 ms for all of it, at
+// passes around them another 4.9 ms; the kernels here take 9.4 ms for all of it, at
 // 4.5 to 6 TB/s in the large layers (a copy moves 6.5), and the step went from 54.3
 // to 27.5 ms.
 //
@@ -242,7 +242,7 @@ enum BnMask { kBnNone, kBnFromX, kBnFromY };
 // part[block][0][c] = sum dz, part[block][1][c] = sum dz * (x - mean), where dz is
 // dy behind the mask; with kBnFromY dz is written out as well.
 template <typename T, BnMask kMask>
-__global__ void __launch_bounds__(kBnThreads, 3)
+__global__ void __launch_bounds__(kBnThreads, 4)
 bn_bwd_sums_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ y,
                    T* __restrict__ dz, const float* __restrict__ mean, const float* __restrict__ rstd,
                    const float* __restrict__ gamma, const float* __restrict__ beta, int64_t nvec, int groups,

@@ -10,7 +10,7 @@
 // accesses, several rows in flight per thread.
 //
 // 8192 x 8192 bf16 (134 MB), tanh form: GELU 77 -> 49 us (5.5 TB/s); its backward and
-// the bias gradient 97 + about 45 -> 85 + 4 us (4.7 TB/s; the erf form takes 109 us,
+// the bias gradient 97 + about 45 -> 79 + 4 us (5.1 TB/s; the erf form takes 109 us,
 // bound by erff).  A plain column sum of the other layers of that block (6144 and
 // 2048 wide): 28 us on average -> 12 + 4 us.
 #include <cuda_bf16.h>
@@ -75,15 +75,18 @@ gelu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, int64_t nvec) 
 }
 
 enum ColumnSumOf { kOfInput, kOfTanhGelu, kOfErfGelu };
+// Measured for 8192 x 8192 (tanh, erf) and the mean of 8192 x 6144 and 2048 (input), four blocks with
+// half the loads in flight against three with all: 79 against 85 us, 112 against 109, 12.8 against 12.4.
+template <ColumnSumOf kOf> constexpr int kColumnBlocksPerSm = kOf == kOfTanhGelu ? 4 : 3;
 
 // partial[strip][c] = sum of column c over the strip's rows: of dy itself, or of
 // dx = dy * gelu'(x), which is written out on the way.  A block is `wide` threads
 // across the columns (8 each) and 256 / wide rows.
 template <ColumnSumOf kOf>
-__global__ void __launch_bounds__(kGeluThreads)
+__global__ void __launch_bounds__(kGeluThreads, kColumnBlocksPerSm<kOf>)
 column_sum_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, bf16* __restrict__ dx,
                   float* __restrict__ partial, int64_t rows, int cols, int wide) {
-  constexpr int U = kOf == kOfInput ? 8 : 4;
+  constexpr int U = kOf == kOfInput ? 8 : kOf == kOfTanhGelu ? 2 : 4;
   const int across = threadIdx.x % wide, down = threadIdx.x / wide, height = kGeluThreads / wide;
   const int c = (blockIdx.x * wide + across) * 8;
   const int64_t stride = (int64_t)gridDim.y * height;
@@ -171,13 +174,13 @@ column_sum_finish_kernel(const float* __restrict__ partial, int strips, int cols
 
 struct ColumnGeometry {
   int wide = 1, tiles, strips;
-  // Blocks for three per SM (80 registers), but at least four rows for a thread: a strip is read again
-  // by the finishing kernel.
-  ColumnGeometry(int64_t rows, int cols, int sm_count) {
+  // As many blocks as are resident, but at least four rows for a thread: a strip is read
+  // again by the finishing kernel.
+  ColumnGeometry(int64_t rows, int cols, int sm_count, int per_sm) {
     while (wide < kGeluThreads && wide * 8 < cols) wide *= 2;
     tiles = (cols / 8 + wide - 1) / wide;
     const int64_t height = kGeluThreads / wide;
-    int64_t n = ((int64_t)sm_count * 3 + tiles - 1) / tiles;
+    int64_t n = ((int64_t)sm_count * per_sm + tiles - 1) / tiles;
     const int64_t most = (rows + 4 * height - 1) / (4 * height);
     strips = (int)(n < most ? n : most);
     if (strips < 1) strips = 1;
@@ -200,12 +203,15 @@ cudaError_t launchGeluForward(const void* x, void* y, int64_t n, bool tanh_form,
   return cudaGetLastError();
 }
 
-int columnSumStrips(int64_t rows, int cols, int sm_count) { return ColumnGeometry(rows, cols, sm_count).strips; }
+int columnSumStrips(int64_t rows, int cols, int sm_count) {
+  return ColumnGeometry(rows, cols, sm_count, kColumnBlocksPerSm<kOfTanhGelu>).strips;  // the largest of the three
+}
 
 cudaError_t launchColumnSum(const void* dy, const void* gelu_x, bool tanh_form, void* dx, float* partial, void* out,
                             bool out_bf16, int64_t rows, int cols, int sm_count, cudaStream_t stream) {
   if (!takes(cols) || rows < 0) return cudaErrorInvalidValue;
-  const ColumnGeometry g(rows, cols, sm_count);
+  const ColumnGeometry g(rows, cols, sm_count,
+                         gelu_x != nullptr && tanh_form ? kColumnBlocksPerSm<kOfTanhGelu> : kColumnBlocksPerSm<kOfInput>);
   auto kernel = gelu_x == nullptr ? column_sum_kernel<kOfInput>
                                   : (tanh_form ? column_sum_kernel<kOfTanhGelu> : column_sum_kernel<kOfErfGelu>);
   kernel<<<dim3(g.tiles, g.strips), kGeluThreads, 0, stream>>>(static_cast<const bf16*>(dy),

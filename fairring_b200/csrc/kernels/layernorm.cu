@@ -43,14 +43,16 @@ __device__ __forceinline__ float warpSum(float v) {
   return v;
 }
 
-// Sum of two values over the block; every thread gets the result.
-__device__ __forceinline__ float2 blockSum2(float a, float b, float2* scratch) {
+// Sum of two values over the block; every thread gets the result.  `scratch` is in
+// two halves that rows alternate between: one barrier per row, which is what the
+// kernels wait for when they do not wait for memory.
+__device__ __forceinline__ float2 blockSum2(float a, float b, float2 (&halves)[2][kLnThreads / 32], int half) {
+  float2* scratch = halves[half];
   for (int o = 16; o > 0; o >>= 1) {
     a += __shfl_xor_sync(0xffffffffu, a, o);
     b += __shfl_xor_sync(0xffffffffu, b, o);
   }
   const int w = threadIdx.x >> 5;
-  __syncthreads();  // scratch may still be read from the previous row
   if ((threadIdx.x & 31) == 0) scratch[w] = make_float2(a, b);
   __syncthreads();
   float2 s = scratch[0];
@@ -67,8 +69,9 @@ __global__ void __launch_bounds__(kLnThreads, ITER == 1 ? 8 : 1)
 layer_norm_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ gamma,
                       const float* __restrict__ beta, TY* __restrict__ y, float* __restrict__ mean_out,
                       float* __restrict__ rstd_out, int64_t rows, int cols, float eps) {
-  __shared__ float2 scratch[kLnThreads / 32];
-  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+  __shared__ float2 scratch[2][kLnThreads / 32];
+  int half = 0;
+  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, half ^= 1) {
     float v[ITER][8];
     float s = 0.f, ss = 0.f;
 #pragma unroll
@@ -83,7 +86,7 @@ layer_norm_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ gamma,
         }
       }
     }
-    const float2 t = blockSum2(s, ss, scratch);
+    const float2 t = blockSum2(s, ss, scratch, half);
     const float mean = t.x / cols;
     const float var = fmaxf(t.y / cols - mean * mean, 0.f);
     const float rstd = rsqrtf(var + eps);
@@ -114,14 +117,15 @@ layer_norm_bwd_kernel(const TY* __restrict__ dy, const TX* __restrict__ x,
                       const float* __restrict__ gamma, const float* __restrict__ mean_in,
                       const float* __restrict__ rstd_in, TX* __restrict__ dx,
                       float* __restrict__ partial, int64_t rows, int cols) {
-  __shared__ float2 scratch[kLnThreads / 32];
+  __shared__ float2 scratch[2][kLnThreads / 32];
+  int half = 0;
   float dg[ITER][8], db[ITER][8];
 #pragma unroll
   for (int it = 0; it < ITER; ++it) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) dg[it][i] = db[it][i] = 0.f;
   }
-  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, half ^= 1) {
     const float mean = mean_in[r], rstd = rstd_in[r];
     float xh[ITER][8], w[ITER][8];
     float s1 = 0.f, s2 = 0.f;
@@ -144,7 +148,7 @@ layer_norm_bwd_kernel(const TY* __restrict__ dy, const TX* __restrict__ x,
         }
       }
     }
-    const float2 t = blockSum2(s1, s2, scratch);
+    const float2 t = blockSum2(s1, s2, scratch, half);
     const float m1 = t.x / cols, m2 = t.y / cols;
 #pragma unroll
     for (int it = 0; it < ITER; ++it) {
@@ -291,7 +295,7 @@ add_layer_norm_fwd_kernel(const float* __restrict__ x, const TB* __restrict__ br
       mean = t.x;
       var = t.y / cols;
     } else {
-      const float2 t = blockSum2(s, ss, scratch[0]);
+      const float2 t = blockSum2(s, ss, scratch, half);
       mean = t.x / cols;
       var = fmaxf(t.y / cols - mean * mean, 0.f);
     }
@@ -327,14 +331,15 @@ add_layer_norm_bwd_kernel(const TY* __restrict__ dy, const float* __restrict__ d
                           const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                           float* __restrict__ dx, __nv_bfloat16* __restrict__ dbranch,
                           float* __restrict__ partial, int64_t rows, int cols) {
-  __shared__ float2 scratch[kLnThreads / 32];
+  __shared__ float2 scratch[2][kLnThreads / 32];
+  int half = 0;
   float dg[ITER][8], db[ITER][8];
 #pragma unroll
   for (int it = 0; it < ITER; ++it) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) dg[it][i] = db[it][i] = 0.f;
   }
-  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, half ^= 1) {
     const float mean = mean_in[r], rstd = rstd_in[r];
     float xh[ITER][8], w[ITER][8];
     float s1 = 0.f, s2 = 0.f;
@@ -365,7 +370,7 @@ add_layer_norm_bwd_kernel(const TY* __restrict__ dy, const float* __restrict__ d
         }
       }
     }
-    const float2 t = blockSum2(s1, s2, scratch);
+    const float2 t = blockSum2(s1, s2, scratch, half);
     const float m1 = t.x / cols, m2 = t.y / cols;
 #pragma unroll
     for (int it = 0; it < ITER; ++it) {
