@@ -46,20 +46,23 @@ cudaError_t launchLayerNormBackward(const void* dy, bool y_bf16, const void* x, 
                                     float* partial, float* dgamma, float* dbeta, int64_t rows, int cols,
                                     int sm_count, cudaStream_t stream);
 
-// xnew = x + branch (x fp32, branch fp32 or bf16), y = LayerNorm(xnew), also in
-// fp32 to `y32` (may be null); the backward takes the gradient of y in its dtype
-// and the fp32 copy's (`dy`, `dy32`: one may be null), adds `gres` (gradient arriving at xnew along the residual path, may
+// xnew = x + branch (x fp32, branch fp32 or bf16), y = LayerNorm(xnew); the
+// backward takes the gradient of y in its dtype and of an fp32 copy of it (`dy`,
+// `dy32`: one may be null), adds `gres` (gradient arriving at xnew along the residual path, may
 // be null) to the LayerNorm gradient and can also write the sum in bf16
 // (`dbranch_bf16`, may be null).
 cudaError_t launchAddLayerNormForward(const float* x, const void* branch, bool branch_bf16,
                                       const float* gamma, const float* beta, float* xnew, void* y,
-                                      bool y_bf16, float* y32, float* mean, float* rstd, int64_t rows, int cols,
+                                      bool y_bf16, float* mean, float* rstd, int64_t rows, int cols,
                                       float eps, int sm_count, cudaStream_t stream);
 cudaError_t launchAddLayerNormBackward(const void* dy, bool y_bf16, const float* dy32, const float* xnew,
                                        const float* gres, const float* gamma, const float* mean, const float* rstd,
                                        float* dx, void* dbranch_bf16, float* partial, float* dgamma,
                                        float* dbeta, int64_t rows, int cols, int sm_count,
                                        cudaStream_t stream);
+
+// out = x + branch: n elements (a multiple of 8), the branch bf16, 16-byte aligned.
+cudaError_t launchAddBranch(const float* x, const void* branch_bf16, float* out, int64_t n, cudaStream_t stream);
 
 // Softmax cross-entropy over [rows, vocab] logits (fp32 or bf16): per-row loss
 // and log-sum-exp; a negative target's row has loss 0, one past the vocabulary

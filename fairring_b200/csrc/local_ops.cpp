@@ -143,11 +143,10 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> layerNormBackward(at::Tensor dy, 
   return std::make_tuple(dx, dgamma, dbeta);
 }
 
-// xnew, y, mean, rstd [, y in fp32] = x + branch, layer_norm(x + branch); x fp32, branch fp32 or
-// bf16.  The last result is undefined unless `want_y32`.
-std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerNormForward(
+// xnew, y, mean, rstd = x + branch, layer_norm(x + branch); x fp32, branch fp32 or bf16.
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerNormForward(
     at::Tensor x, at::Tensor branch, at::Tensor gamma, at::Tensor beta, double eps,
-    at::ScalarType out_dtype, bool want_y32) {
+    at::ScalarType out_dtype) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.scalar_type() == at::kFloat && x.dim() >= 1,
               "x must be a contiguous fp32 CUDA tensor");
   TORCH_CHECK(branch.is_cuda() && branch.is_contiguous() && branch.sizes() == x.sizes() &&
@@ -167,18 +166,33 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerN
   gamma = aligned16(gamma);
   beta = aligned16(beta);
   at::Tensor xnew = at::empty_like(x);
-  at::Tensor y = at::empty(x.sizes(), x.options().dtype(out_dtype)), y32;
-  if (want_y32) y32 = at::empty_like(x);
+  at::Tensor y = at::empty(x.sizes(), x.options().dtype(out_dtype));
   at::Tensor mean = at::empty({rows}, x.options());
   at::Tensor rstd = at::empty({rows}, x.options());
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   cudaError_t e = launchAddLayerNormForward(
       x.data_ptr<float>(), branch.data_ptr(), branch.scalar_type() == at::kBFloat16, gamma.data_ptr<float>(),
       beta.data_ptr<float>(), xnew.data_ptr<float>(), y.data_ptr(), out_dtype == at::kBFloat16,
-      want_y32 ? y32.data_ptr<float>() : nullptr, mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, (int)cols,
-      (float)eps, sms, c10::cuda::getCurrentCUDAStream());
+      mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, (int)cols, (float)eps, sms,
+      c10::cuda::getCurrentCUDAStream());
   TORCH_CHECK(e == cudaSuccess, "add_layer_norm forward launch failed: ", cudaGetErrorString(e));
-  return std::make_tuple(xnew, y, mean, rstd, y32);
+  return std::make_tuple(xnew, y, mean, rstd);
+}
+
+// x + branch in fp32, x fp32 and the branch bf16.
+at::Tensor addBranch(at::Tensor x, at::Tensor branch) {
+  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.scalar_type() == at::kFloat && branch.is_cuda() &&
+                  branch.device() == x.device() && branch.is_contiguous() && branch.scalar_type() == at::kBFloat16 &&
+                  branch.sizes() == x.sizes() && x.numel() % 8 == 0,
+              "x must be contiguous fp32, branch contiguous bf16 and shaped alike, a multiple of 8 elements");
+  c10::cuda::CUDAGuard guard(x.device());
+  x = aligned16(x);
+  branch = aligned16(branch);
+  at::Tensor out = at::empty_like(x);
+  cudaError_t e = launchAddBranch(x.data_ptr<float>(), branch.data_ptr(), out.data_ptr<float>(), x.numel(),
+                                  c10::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(e == cudaSuccess, "residual add launch failed: ", cudaGetErrorString(e));
+  return out;
 }
 
 // dx (fp32), dx in bf16 (or an undefined tensor), dgamma, dbeta.  `dy`: the gradient
@@ -558,8 +572,7 @@ struct LayerNormNode : torch::autograd::Function<LayerNormNode> {
 struct AddLayerNormNode : torch::autograd::Function<AddLayerNormNode> {
   static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& branch,
                                const at::Tensor& gamma, const at::Tensor& beta, double eps, at::ScalarType out_dtype) {
-    auto [xnew, y, mean, rstd, y32] =
-        addLayerNormForward(x.contiguous(), branch.contiguous(), gamma, beta, eps, out_dtype, false);
+    auto [xnew, y, mean, rstd] = addLayerNormForward(x.contiguous(), branch.contiguous(), gamma, beta, eps, out_dtype);
     ctx->set_materialize_grads(false);  // an unused output arrives undefined, not as zeros
     ctx->save_for_backward({xnew, gamma, mean, rstd});
     ctx->saved_data["out"] = static_cast<int64_t>(out_dtype);
@@ -647,7 +660,8 @@ void bindLocalOps(pybind11::module_& m) {
   m.def("cross_entropy_bwd_", &crossEntropyBackwardInPlace, py::arg("logits"), py::arg("targets"),
         py::arg("lse"), py::arg("upstream"), py::arg("scale"), py::arg("count") = py::none());
   m.def("add_layer_norm_fwd", &addLayerNormForward, py::arg("x"), py::arg("branch"), py::arg("weight"),
-        py::arg("bias"), py::arg("eps"), py::arg("out_dtype"), py::arg("want_y32") = false);
+        py::arg("bias"), py::arg("eps"), py::arg("out_dtype"));
+  m.def("add_branch", &addBranch, py::arg("x"), py::arg("branch"));
   m.def("add_layer_norm_bwd", &addLayerNormBackward, py::arg("dy"), py::arg("xnew"), py::arg("weight"),
         py::arg("mean"), py::arg("rstd"), py::arg("gres"), py::arg("want_bf16"), py::arg("dy32") = py::none());
   m.def("gelu_fwd", &geluForward, py::arg("x"), py::arg("tanh_form"));

@@ -50,6 +50,17 @@ class EncoderLayer(nn.Module):
         x = self.ln1(x + self.proj(a.transpose(1, 2).reshape(b, s, d)))
         return self.ln2(x + self.fc2(F.gelu(self.fc1(x))))
 
+    def forward_pair(self, x: torch.Tensor, low: torch.Tensor):
+        """The same layer on the stream and its copy in the autocast dtype, which the linear layers read:
+        takes and returns both, so that each LayerNorm's backward takes both gradients at once."""
+        from ..ops import add_layer_norm_pair, linear, linear_gelu
+
+        b, s, d = x.shape
+        q, k, v = linear(self.qkv, low).view(b, s, 3, self.n_head, d // self.n_head).unbind(2)
+        a = F.scaled_dot_product_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2))
+        x, low = add_layer_norm_pair(self.ln1, x, linear(self.proj, a.transpose(1, 2).reshape(b, s, d)))
+        return add_layer_norm_pair(self.ln2, x, linear(self.fc2, linear_gelu(self.fc1, low)))
+
 
 class EncoderMLM(nn.Module):
     def __init__(self, cfg: EncoderConfig):
@@ -73,19 +84,27 @@ class EncoderMLM(nn.Module):
 
     def forward(self, tokens: torch.Tensor, labels: torch.Tensor | None = None):
         """``labels``: target ids at masked positions, -100 elsewhere."""
+        from ..ops import cross_entropy_keeping_logits, linear_gelu, tied_embedding, vocab_logits
+        from ..ops._plain import plain_module
+
         b, s = tokens.shape
-        x = self.ln_emb(self.tok(tokens) + self.pos(torch.arange(s, device=tokens.device)))
+        x, table = tied_embedding(self.tok, self.pos, tokens, pad_rows=labels is not None)
+        x = self.ln_emb(x)
+        low = x
         for layer in self.layers:
-            x = layer(x)
+            if x.is_cuda and plain_module(layer, EncoderLayer):
+                x, low = layer.forward_pair(x, low)
+            else:
+                x = low = layer(x)
         if labels is None:
             h = self.head_ln(F.gelu(self.head_dense(x)))
-            return F.linear(h, self.tok.weight, self.head_bias)
+            return F.linear(h, table, self.head_bias)
         # Only masked positions go through the vocabulary projection.
         sel = labels.reshape(-1) != -100
-        h = x.reshape(b * s, -1)[sel]
-        h = self.head_ln(F.gelu(self.head_dense(h)))
-        logits = F.linear(h, self.tok.weight, self.head_bias)
-        return F.cross_entropy(logits.float(), labels.reshape(-1)[sel])
+        h = low.reshape(b * s, -1)[sel]
+        h = self.head_ln(linear_gelu(self.head_dense, h))
+        logits = vocab_logits(h, table, self.head_bias)
+        return cross_entropy_keeping_logits(logits, labels.reshape(-1)[sel])
 
 
 def mask_tokens(tokens: torch.Tensor, cfg: EncoderConfig, generator: torch.Generator, mask_id: int = 0):

@@ -16,29 +16,34 @@ class _TiedEmbeddingFn(torch.autograd.Function):
     the table, so that its gradient is built once."""
 
     @staticmethod
-    def forward(ctx, tokens, table, pos):
+    def forward(ctx, tokens, table, pos, rows):
         ctx.save_for_backward(tokens)
         ctx.set_materialize_grads(False)  # an unused output arrives as None, not as zeros
         ctx.vocab, ctx.positions, ctx.d = table.shape[0], pos.shape[0], table.shape[1]
-        return _C.embed_fwd(tokens, table, pos), table.to(torch.bfloat16)
+        low = table.new_empty((rows, ctx.d), dtype=torch.bfloat16)
+        low[: ctx.vocab].copy_(table)
+        low[ctx.vocab:].zero_()
+        return _C.embed_fwd(tokens, table, pos), low
 
     @staticmethod
     def backward(ctx, dx, dlow):
         (tokens,) = ctx.saved_tensors
         if dx is None and dlow is None:
-            return None, None, None
+            return None, None, None, None
+        dlow = None if dlow is None else dlow[: ctx.vocab]
         if torch.is_grad_enabled():  # the graph of this backward is wanted: torch's own ops have one
             scatter = torch.ops.aten.embedding_dense_backward
             dtable = dlow.float() if dlow is not None else None
             if dx is None:
-                return None, dtable, None
+                return None, dtable, None, None
             rows = scatter(dx, tokens, ctx.vocab, -1, False)
             places = torch.arange(tokens.shape[1], device=tokens.device).expand_as(tokens)
-            return None, rows if dtable is None else dtable + rows, scatter(dx, places, ctx.positions, -1, False)
+            dpos = scatter(dx, places, ctx.positions, -1, False)
+            return None, rows if dtable is None else dtable + rows, dpos, None
         dx = None if dx is None else dx.contiguous()
         dlow = None if dlow is None else dlow.contiguous()
         dtable, dpos = _C.embed_bwd(dx, dlow, tokens, ctx.vocab, ctx.positions, ctx.d)
-        return None, dtable, dpos
+        return None, dtable, dpos, None
 
 
 def _plain_table(m: nn.Module) -> bool:
@@ -47,9 +52,10 @@ def _plain_table(m: nn.Module) -> bool:
             and m.weight.is_contiguous() and m.weight.data_ptr() % 16 == 0)
 
 
-def tied_embedding(tok: nn.Embedding, pos: nn.Embedding, tokens: torch.Tensor):
+def tied_embedding(tok: nn.Embedding, pos: nn.Embedding, tokens: torch.Tensor, pad_rows: bool = False):
     """``(tok(tokens) + pos(0, 1, ...), table)``: ``table`` is what the output projection multiplies
-    with, ``tok.weight`` or, where the fused form applies, its bf16 copy.  Fused in training under bf16
+    with, ``tok.weight`` or, where the fused form applies, its bf16 copy, with ``pad_rows`` with rows of
+    zeros behind it up to a multiple of 8 (see :func:`fairring_b200.ops.vocab_logits`).  Fused in training under bf16
     autocast on the GPU.  The rows of equal tokens are added in no fixed order, so under
     ``torch.use_deterministic_algorithms`` the modules are called."""
     if (tokens.is_cuda and tokens.dim() == 2 and tokens.dtype == torch.long and tokens.numel() > 0
@@ -58,5 +64,7 @@ def tied_embedding(tok: nn.Embedding, pos: nn.Embedding, tokens: torch.Tensor):
             and tok.weight.device == pos.weight.device == tokens.device and tok.embedding_dim == pos.embedding_dim
             and tok.embedding_dim % 8 == 0 and tokens.shape[1] <= pos.num_embeddings
             and not torch.are_deterministic_algorithms_enabled() and plain_autograd()):
-        return _TiedEmbeddingFn.apply(tokens.contiguous(), tok.weight, pos.weight)
+        rows = tok.num_embeddings
+        rows = (rows + 7) // 8 * 8 if pad_rows else rows
+        return _TiedEmbeddingFn.apply(tokens.contiguous(), tok.weight, pos.weight, rows)
     return tok(tokens) + pos(torch.arange(tokens.shape[1], device=tokens.device)), tok.weight
