@@ -95,9 +95,10 @@ cudaError_t launchBatchNormForward(const BatchNormShape& s, bool bf16, const voi
                                    float* running_mean, float* running_var, int64_t* tracked, float momentum,
                                    float eps, float* scratch, int sm_count, cudaStream_t stream);
 // `y`, `dz`: given when there was a residual and a ReLU: the output, and where the
-// residual's gradient goes.  Without a ReLU the residual's gradient is dy.
-cudaError_t launchBatchNormBackward(const BatchNormShape& s, bool bf16, const void* dy, const void* x, const void* y,
-                                    void* dz, void* dx, bool relu, const float* gamma, const float* beta,
+// residual's gradient goes.  Without a ReLU the residual's gradient is dy.  `dy2` (may be null,
+// only then): a second gradient of y, added to dy.
+cudaError_t launchBatchNormBackward(const BatchNormShape& s, bool bf16, const void* dy, const void* dy2, const void* x,
+                                    const void* y, void* dz, void* dx, bool relu, const float* gamma, const float* beta,
                                     const float* mean, const float* rstd, float* dgamma, float* dbeta,
                                     float* scratch, int sm_count, cudaStream_t stream);
 

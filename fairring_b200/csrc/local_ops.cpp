@@ -411,10 +411,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> batchNormForward(
 }
 
 // dx, gradient of the residual, dgamma, dbeta.  `y`: the output, given when there
-// was a residual and a ReLU; otherwise the second result is undefined.
+// was a residual and a ReLU; otherwise the second result is undefined.  `dy2`: a second gradient of
+// that output, or nothing.
 std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> batchNormBackward(
     at::Tensor dy, at::Tensor x, std::optional<at::Tensor> y, at::Tensor gamma, at::Tensor beta, at::Tensor mean,
-    at::Tensor rstd, bool relu) {
+    at::Tensor rstd, bool relu, std::optional<at::Tensor> dy2) {
   const BatchNormShape s = batchNormShape(x);
   checkLikeX(dy, x, "dy");
   checkPerChannel(gamma, x, "weight");
@@ -424,6 +425,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> batchNormBackward(
   c10::cuda::CUDAGuard guard(x.device());
   x = aligned16(x);
   dy = aligned16(dy);
+  at::Tensor second;
+  if (dy2.has_value() && dy2->defined()) {
+    checkLikeX(*dy2, x, "dy2");
+    second = aligned16(*dy2);
+  }
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   at::Tensor dz, yt;
   if (y.has_value() && y->defined()) {
@@ -435,7 +441,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> batchNormBackward(
   at::Tensor dgamma = at::empty_like(gamma), dbeta = at::empty_like(gamma);
   at::Tensor scratch = at::empty({batchNormScratchFloats(s, sms)}, gamma.options());
   cudaError_t e = launchBatchNormBackward(
-      s, x.scalar_type() == at::kBFloat16, dy.data_ptr(), x.data_ptr(), yt.defined() ? yt.data_ptr() : nullptr,
+      s, x.scalar_type() == at::kBFloat16, dy.data_ptr(), second.defined() ? second.data_ptr() : nullptr, x.data_ptr(),
+      yt.defined() ? yt.data_ptr() : nullptr,
       dz.defined() ? dz.data_ptr() : nullptr, dx.data_ptr(), relu, gamma.data_ptr<float>(), beta.data_ptr<float>(),
       mean.data_ptr<float>(), rstd.data_ptr<float>(), dgamma.data_ptr<float>(), dbeta.data_ptr<float>(),
       scratch.data_ptr<float>(), sms, c10::cuda::getCurrentCUDAStream());
@@ -671,7 +678,7 @@ void bindLocalOps(pybind11::module_& m) {
         py::arg("running_mean"), py::arg("running_var"), py::arg("tracked"), py::arg("momentum"), py::arg("eps"),
         py::arg("relu"));
   m.def("batch_norm_bwd", &batchNormBackward, py::arg("dy"), py::arg("x"), py::arg("y"), py::arg("weight"),
-        py::arg("bias"), py::arg("mean"), py::arg("rstd"), py::arg("relu"));
+        py::arg("bias"), py::arg("mean"), py::arg("rstd"), py::arg("relu"), py::arg("dy2") = py::none());
   m.def("max_pool_fwd", &maxPoolForward, py::arg("x"), py::arg("window"), py::arg("stride"), py::arg("pad"));
   m.def("max_pool_bwd", &maxPoolBackward, py::arg("dy"), py::arg("x"), py::arg("chosen"), py::arg("window"),
         py::arg("stride"), py::arg("pad"));

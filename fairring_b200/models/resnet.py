@@ -27,12 +27,17 @@ class Bottleneck(nn.Module):
         self.downsample = downsample
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        return self.forward_pair(x, x)[0]
+
+    def forward_pair(self, x: torch.Tensor, shortcut: torch.Tensor):
+        """The block on an input that comes twice, for its convolutions and for its shortcut; so does
+        the output, whose two gradients the backward then adds inside the BatchNorm."""
         from ..ops import batch_norm_act
 
-        identity = x if self.downsample is None else self.downsample(x)
+        identity = shortcut if self.downsample is None else self.downsample(shortcut)
         out = batch_norm_act(self.bn1, self.conv1(x), relu=self.relu)
         out = batch_norm_act(self.bn2, self.conv2(out), relu=self.relu)
-        return batch_norm_act(self.bn3, self.conv3(out), residual=identity, relu=self.relu)
+        return batch_norm_act(self.bn3, self.conv3(out), residual=identity, relu=self.relu, twice=True)
 
 
 class Downsample(nn.Sequential):
@@ -85,9 +90,16 @@ class ResNet50(nn.Module):
 
     def forward(self, images: torch.Tensor, labels: torch.Tensor | None = None):
         from ..ops import batch_norm_act, max_pool
+        from ..ops._plain import plain_module
 
         x = max_pool(self.maxpool, batch_norm_act(self.bn1, self.conv1(images), relu=self.relu))
-        x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
+        shortcut = x
+        for stage in (self.layer1, self.layer2, self.layer3, self.layer4):
+            if plain_module(stage, nn.Sequential) and all(plain_module(block, Bottleneck) for block in stage):
+                for block in stage:
+                    x, shortcut = block.forward_pair(x, shortcut)
+            else:
+                x = shortcut = stage(x)
         logits = self.fc(torch.flatten(self.avgpool(x), 1))
         if labels is None:
             return logits

@@ -19,32 +19,44 @@ from ._plain import plain_autograd, plain_module
 
 class _BatchNormActFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, residual, weight, bias, running_mean, running_var, tracked, momentum, eps, relu):
+    def forward(ctx, x, residual, weight, bias, running_mean, running_var, tracked, momentum, eps, relu, twice):
         y, mean, rstd = _C.batch_norm_fwd(x, residual, weight, bias, running_mean, running_var, tracked, momentum,
                                           eps, relu)
         torch.autograd.graph.increment_version(tracked)  # as torch's own layer does, which adds 1 in place
         ctx.relu, ctx.eps, ctx.has_residual = relu, eps, residual is not None
         ctx.save_for_backward(x, weight, bias, mean, rstd, residual, y if relu and residual is not None else None)
-        return y
+        if not twice:
+            return y
+        ctx.set_materialize_grads(False)  # an unused output arrives as None, not as zeros
+        return y, y.view_as(y)
 
     @staticmethod
-    def backward(ctx, dy):
+    def backward(ctx, dy, dy2=None):
+        if dy is None:
+            dy, dy2 = dy2, None
+        if dy is None:
+            return (None,) * 11
         x, weight, bias, mean, rstd, residual, y = ctx.saved_tensors
         if torch.is_grad_enabled():  # the graph of this backward is wanted: torch's own ops have one
             inputs = (x, weight, bias) if residual is None else (x, weight, bias, residual)
             wanted = [t for t in inputs if t.requires_grad]
             with torch.enable_grad():
+                dy = dy if dy2 is None else dy + dy2
                 out = F.batch_norm(x, None, None, weight, bias, True, 0.0, ctx.eps)
                 out = out if residual is None else out + residual
                 out = F.relu(out) if ctx.relu else out
                 grads = iter(torch.autograd.grad(out, wanted, dy, create_graph=True))
             got = [next(grads) if t.requires_grad else None for t in inputs] + [None]
-            return got[0], got[3], got[1], got[2], None, None, None, None, None, None
+            return got[0], got[3], got[1], got[2], None, None, None, None, None, None, None
         dy = dy.contiguous(memory_format=torch.channels_last)
-        dx, dres, dgamma, dbeta = _C.batch_norm_bwd(dy, x, y, weight, bias, mean, rstd, ctx.relu)
+        if dy2 is not None:
+            dy2 = dy2.contiguous(memory_format=torch.channels_last)
+            if y is None:
+                dy, dy2 = dy + dy2, None
+        dx, dres, dgamma, dbeta = _C.batch_norm_bwd(dy, x, y, weight, bias, mean, rstd, ctx.relu, dy2)
         if ctx.has_residual and not ctx.relu:
             dres = dy
-        return dx, dres if ctx.has_residual else None, dgamma, dbeta, None, None, None, None, None, None
+        return dx, dres if ctx.has_residual else None, dgamma, dbeta, None, None, None, None, None, None, None
 
 
 def _channels_last(t: torch.Tensor) -> bool:
@@ -71,15 +83,18 @@ def _fusable(bn: nn.BatchNorm2d, x: torch.Tensor, residual: torch.Tensor | None)
 
 
 def batch_norm_act(bn: nn.Module, x: torch.Tensor, residual: torch.Tensor | None = None,
-                   relu: nn.Module | None = None) -> torch.Tensor:
-    """``relu(bn(x) + residual)``; ``residual`` and ``relu`` may be left out.  Fused for an
+                   relu: nn.Module | None = None, twice: bool = False):
+    """``relu(bn(x) + residual)``; ``residual`` and ``relu`` may be left out.  With ``twice`` the result
+    comes as a pair, for a caller that uses it in two places: the two gradients are then added inside
+    the backward.  Fused for an
     ``nn.BatchNorm2d`` in training mode and a channels-last fp32 or bf16 ``x`` on the GPU with a
     power of two from 8 to 2048 channels; otherwise, and when one of the modules carries hooks or
     has been replaced, the modules are called."""
     if (relu is None or plain_module(relu, nn.ReLU)) and _fusable(bn, x, residual):
         return _BatchNormActFn.apply(x, residual, bn.weight, bn.bias, bn.running_mean, bn.running_var,
-                                     bn.num_batches_tracked, bn.momentum, bn.eps, relu is not None)
+                                     bn.num_batches_tracked, bn.momentum, bn.eps, relu is not None, twice)
     y = bn(x)
     if residual is not None:
         y = y + residual
-    return y if relu is None else relu(y)
+    y = y if relu is None else relu(y)
+    return (y, y) if twice else y

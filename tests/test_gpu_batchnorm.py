@@ -125,3 +125,29 @@ def test_second_derivative():
         (g,) = torch.autograd.grad((y ** 3).sum(), x, create_graph=True)
         got.append(torch.autograd.grad((g ** 2).sum(), x)[0])
     torch.testing.assert_close(got[0], got[1], rtol=1e-3, atol=1e-4 * float(got[1].abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("residual,relu", [(True, True), (False, True), (True, False)])
+@pytest.mark.parametrize("use", ["both", "first", "second"])
+def test_two_uses_of_the_output(dtype, residual, relu, use):
+    _need_gpu()
+    from fairring_b200.ops import batch_norm_act
+
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda: torch.randn(4, 64, 13, 11, device="cuda", generator=gen).to(  # noqa: E731
+        dtype=dtype, memory_format=torch.channels_last)
+    x, res, dy, dy2 = rand().requires_grad_(True), rand().requires_grad_(True) if residual else None, rand(), rand()
+    bn, act = nn.BatchNorm2d(64, device="cuda"), nn.ReLU() if relu else None
+    inputs = [x, bn.weight, bn.bias] + ([res] if residual else [])
+    pair = batch_norm_act(bn, x, res, act, twice=True)
+    outs = {"both": (list(pair), [dy, dy2]), "first": ([pair[0]], [dy]), "second": ([pair[1]], [dy2])}[use]
+    got = torch.autograd.grad(outs[0], inputs, outs[1])
+    y = batch_norm_act(bn, x, res, act)
+    assert torch.equal(pair[0], y) and torch.equal(pair[1], y)
+    total = sum(d.double() for d in outs[1])
+    want = _reference(x, res, bn, relu, total)[2]
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22
+    far = 2.0 ** -7 if dtype == torch.bfloat16 else 1e-5  # the sum of two gradients is rounded before it is used
+    for g, w in zip(got, want):
+        assert float((g.double() - w).norm()) <= (eps + far) * float(w.norm())
