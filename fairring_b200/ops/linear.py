@@ -16,6 +16,30 @@ from .. import _C
 from ._plain import plain_autograd, plain_module
 
 
+class _LowWeightFn(torch.autograd.Function):
+    """The weight's bf16 copy, which autocast would make as well; its gradient is widened by this
+    package's kernel (19 us for 12.6 M elements, torch's cast takes 32 us)."""
+
+    @staticmethod
+    def forward(ctx, weight):
+        return weight.to(torch.bfloat16)
+
+    @staticmethod
+    def backward(ctx, g):
+        if torch.is_grad_enabled() or not g.is_contiguous() or g.data_ptr() % 16:
+            return g.float()
+        out = torch.empty_like(g, dtype=torch.float32)
+        _C.bf16_grad_to_f32_(out, g)
+        return out
+
+
+def _product(fc: nn.Linear, x: torch.Tensor) -> torch.Tensor:
+    weight = fc.weight
+    if weight.dtype == torch.float32 and weight.requires_grad:
+        weight = _LowWeightFn.apply(weight)
+    return F.linear(x, weight, fc.bias.detach())
+
+
 class _BiasGradFn(torch.autograd.Function):
     """The layer's output as it is; its backward gives the bias its gradient."""
 
@@ -77,7 +101,7 @@ def linear(fc: nn.Linear, x: torch.Tensor) -> torch.Tensor:
     """``fc(x)``, with the bias gradient summed by one kernel where the output is bf16."""
     if not _fusable(fc, x):
         return fc(x)
-    return _BiasGradFn.apply(F.linear(x, fc.weight, fc.bias.detach()), fc.bias)
+    return _BiasGradFn.apply(_product(fc, x), fc.bias)
 
 
 def linear_gelu(fc: nn.Linear, x: torch.Tensor, approximate: str = "none") -> torch.Tensor:
@@ -85,7 +109,7 @@ def linear_gelu(fc: nn.Linear, x: torch.Tensor, approximate: str = "none") -> to
     each way and its backward also sums the bias gradient."""
     if approximate not in ("none", "tanh") or not _fusable(fc, x):
         return F.gelu(fc(x), approximate=approximate)
-    return _GeluFn.apply(F.linear(x, fc.weight, fc.bias.detach()), fc.bias, approximate == "tanh")
+    return _GeluFn.apply(_product(fc, x), fc.bias, approximate == "tanh")
 
 
 class _PaddedHeadFn(torch.autograd.Function):
