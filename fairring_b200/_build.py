@@ -47,6 +47,7 @@ SOURCES = [
     "kernels/cross_entropy.cu",
     "kernels/batchnorm.cu",
     "kernels/maxpool.cu",
+    "kernels/stem.cu",
     "kernels/gelu.cu",
     "kernels/embedding.cu",
     "kernels/noalloc_allreduce.cu",

@@ -129,6 +129,11 @@ cudaError_t launchEmbedForward(const int64_t* tokens, const float* table, const 
 cudaError_t launchEmbedBackward(const float* dx, const int64_t* tokens, float* dtable, float* dpos, int batch, int seq,
                                 int64_t vocab, int d, cudaStream_t stream);
 
+// Channels-last [images, 3, height, width] (fp32 or bf16) to channels-last bf16 [images, 16, rows, cols]:
+// the 2 x 2 pixel blocks from row and column -4 on, 4 x 3 channels and 4 zeros; zero outside the image.
+cudaError_t launchStemFold(const void* image, bool bf16, void* out, int images, int height, int width, int rows,
+                           int cols, cudaStream_t stream);
+
 uint64_t localLaunchCountImpl();
 void noteLocalLaunch();
 

@@ -89,10 +89,10 @@ class ResNet50(nn.Module):
         return sum(p.numel() for p in self.parameters())
 
     def forward(self, images: torch.Tensor, labels: torch.Tensor | None = None):
-        from ..ops import batch_norm_act, max_pool
+        from ..ops import batch_norm_act, max_pool, stem_conv
         from ..ops._plain import plain_module
 
-        x = max_pool(self.maxpool, batch_norm_act(self.bn1, self.conv1(images), relu=self.relu))
+        x = max_pool(self.maxpool, batch_norm_act(self.bn1, stem_conv(self.conv1, images), relu=self.relu))
         shortcut = x
         for stage in (self.layer1, self.layer2, self.layer3, self.layer4):
             if plain_module(stage, nn.Sequential) and all(plain_module(block, Bottleneck) for block in stage):

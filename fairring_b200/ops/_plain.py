@@ -11,9 +11,9 @@ from torch.nn.modules import module as _module
 def plain_autograd() -> bool:
     """False inside the transforms that look through torch's own ops but not through an
     ``autograd.Function`` around a native kernel: functorch (``vmap``, ``grad``, ``jvp``),
-    forward-mode differentiation, tracing and compilation."""
-    return not (torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0
-                or torch.compiler.is_compiling() or torch.jit.is_tracing())
+    forward-mode differentiation, tracing and compilation; and in inference mode."""
+    return not (torch.is_inference_mode_enabled() or torch._C._are_functorch_transforms_active()
+                or forward_ad._current_level >= 0 or torch.compiler.is_compiling() or torch.jit.is_tracing())
 
 
 def plain_module(m: nn.Module, cls: type) -> bool:
