@@ -84,7 +84,7 @@ def main(argv=None) -> int:
             loss, lse = C.cross_entropy_fwd(logits, targets)
             C.cross_entropy_bwd_(logits, targets, lse, one, 1.0 / rows)
 
-        # forward: read the logits once (the second sweep of a row hits L2); backward: read + write
+        # forward: read the logits once; backward: read + write
         algo_bytes = rows * vocab * 2 * 3
         pattern = "cross_entropy_fwd_kernel|cross_entropy_bwd_kernel"
     elif args.kernel == "pipe":

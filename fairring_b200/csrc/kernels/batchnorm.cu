@@ -19,12 +19,14 @@
 //
 // ResNet-50, 256 images of 224 x 224 in bf16 (53 BatchNorms): torch's statistics,
 // transform, reduction and gradient kernels took 31.4 ms of a step, its ReLU and add
-// passes around them another 4.9 ms; the kernels here take 9.4 ms for all of it, at
+// passes around them another 4.9 ms; the kernels here take 9.0 ms for all of it, at
 // 4.5 to 6 TB/s in the large layers (a copy moves 6.5), and the step went from 54.3
-// to 27.5 ms.
+// to 27.5 ms (22.3 ms with the later steps around it).
 //
 // The two small kernels between the passes read one partial result per block of
-// the first pass: all of a thread's partials are loaded before the first is used.
+// the first pass: 8 channels and 128 results side by side, all of a thread's loads in
+// flight (5.4 and 3.7 us on average; with 32 channels a block and up to 20 results a
+// thread 10.6 and 7.5 us).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -37,9 +39,11 @@ namespace fairring {
 namespace {
 
 constexpr int kBnThreads = 256;
-constexpr int kBnFinishWarps = 32;
-constexpr int kBnFinishLoads = 20;
-constexpr int kBnMaxBlocks = kBnFinishWarps * kBnFinishLoads;
+// The small kernels: 8 channels (a 32-byte sector) and 128 partial results side by side.
+constexpr int kBnFinishThreads = 1024;
+constexpr int kBnFinishRows = kBnFinishThreads / 8;
+constexpr int kBnFinishLoads = 5;
+constexpr int kBnMaxBlocks = kBnFinishRows * kBnFinishLoads;
 
 __device__ __forceinline__ void loadChannels(const float* p, int group, float (&v)[8]) {
   Raw8<float> r;
@@ -120,57 +124,56 @@ bn_stats_kernel(const T* __restrict__ x, int64_t nvec, int groups, float* __rest
   }
 }
 
-// Sum over the 32 warps of a block of what each lane holds for its column: warp w
-// gets column w's.
-__device__ __forceinline__ double sumOfColumn(double v, double (&sm)[kBnFinishWarps][33]) {
+// Sum over the block of what each thread holds for channel threadIdx.x % 8: warp w < 8
+// gets channel w's.
+__device__ __forceinline__ double sumOfChannel(double v, double (&sm)[kBnFinishThreads / 32][9]) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  v += __shfl_xor_sync(0xffffffffu, v, 8);
+  v += __shfl_xor_sync(0xffffffffu, v, 16);
   __syncthreads();
-  sm[w][lane] = v;
+  if (lane < 8) sm[w][lane] = v;
   __syncthreads();
-  double t = sm[lane][w];
+  double t = w < 8 ? sm[lane][w] : 0.0;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   return t;
 }
 
-// Merges the blocks' statistics, 32 channels per block, and updates the running ones.
+// Merges the blocks' statistics, 8 channels per block, and updates the running ones.
 // `members`: rows that a block of the first pass visits at a time.
-__global__ void __launch_bounds__(kBnFinishWarps * 32, 1)
+__global__ void __launch_bounds__(kBnFinishThreads, 1)
 bn_finish_stats_kernel(const float* __restrict__ part, int nparts, int members, int channels, int64_t rows,
                        float eps, float momentum, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                        float* __restrict__ running_mean, float* __restrict__ running_var,
                        int64_t* __restrict__ tracked) {
-  __shared__ double sm[kBnFinishWarps][33];
+  __shared__ double sm[kBnFinishThreads / 32][9];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;
-  const float first = c < channels ? part[c] : 0.f;  // block 0's mean: what the others are merged around
+  const int c = blockIdx.x * 8 + (threadIdx.x & 7), row = threadIdx.x >> 3;
+  const float first = part[c];  // block 0's mean: what the others are merged around
+  float mean[kBnFinishLoads], m2[kBnFinishLoads];
+#pragma unroll
+  for (int j = 0; j < kBnFinishLoads; ++j) {
+    const int b = row + j * kBnFinishRows;
+    mean[j] = b < nparts ? part[(size_t)b * 2 * channels + c] : 0.f;
+    m2[j] = b < nparts ? part[((size_t)b * 2 + 1) * channels + c] : 0.f;
+  }
   // Rows of block b: whole rounds of the grid, and its share of the last one.
   const int64_t round = (int64_t)nparts * members;
   const int whole = (int)(rows / round) * members, rest = (int)(rows % round);
   double d = 0.0, q = 0.0;
-  for (int b0 = w; b0 < nparts; b0 += kBnFinishLoads / 2 * kBnFinishWarps) {
-    float mean[kBnFinishLoads / 2], m2[kBnFinishLoads / 2];
 #pragma unroll
-    for (int j = 0; j < kBnFinishLoads / 2; ++j) {
-      const int b = b0 + j * kBnFinishWarps;
-      const bool in = b < nparts && c < channels;
-      mean[j] = in ? part[(size_t)b * 2 * channels + c] : 0.f;
-      m2[j] = in ? part[((size_t)b * 2 + 1) * channels + c] : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < kBnFinishLoads / 2; ++j) {
-      const int b = b0 + j * kBnFinishWarps;
-      if (b < nparts) {
-        const double n = whole + min(members, max(0, rest - b * members)), e = (double)mean[j] - (double)first;
-        d += n * e;
-        q += (double)m2[j] + n * e * e;
-      }
+  for (int j = 0; j < kBnFinishLoads; ++j) {
+    const int b = row + j * kBnFinishRows;
+    if (b < nparts) {
+      const double n = whole + min(members, max(0, rest - b * members)), e = (double)mean[j] - (double)first;
+      d += n * e;
+      q += (double)m2[j] + n * e * e;
     }
   }
-  d = sumOfColumn(d, sm) / (double)rows;
-  q = sumOfColumn(q, sm) / (double)rows;
-  const int mine = blockIdx.x * 32 + w;
-  if (lane == 0 && mine < channels) {
+  d = sumOfChannel(d, sm) / (double)rows;
+  q = sumOfChannel(q, sm) / (double)rows;
+  const int mine = blockIdx.x * 8 + w;
+  if (lane == 0 && w < 8) {
     const float mu = (float)((double)part[mine] + d);
     double var = q - d * d;
     if (var < 0.0) var = 0.0;  // NaN stays
@@ -183,7 +186,9 @@ bn_finish_stats_kernel(const float* __restrict__ part, int nparts, int members, 
   if (blockIdx.x == 0 && threadIdx.x == 0) *tracked += 1;
 }
 
-// y = (x - mean) * rstd * gamma + beta [+ residual] [, negative values to zero]
+// y = (x - mean) * rstd * gamma + beta [+ residual] [, negative values to zero].  From
+// the end to the start, as the dx pass below: the end of x is what the pass before
+// left in L2 (2 to 3 % of either).
 template <typename T, bool kRelu, bool kResidual>
 __global__ void __launch_bounds__(kBnThreads, 4)
 bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ residual, T* __restrict__ y,
@@ -217,18 +222,19 @@ bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ residual, T* __re
     out.set(o);
     out.store(y + at * 8);
   };
-  int64_t i = (int64_t)blockIdx.x * kBnThreads + threadIdx.x;
-  for (; i + (U - 1) * stride < nvec; i += U * stride) {
+  const int64_t first = (int64_t)blockIdx.x * kBnThreads + threadIdx.x;
+  int64_t i = first < nvec ? first + (nvec - 1 - first) / stride * stride : -1;  // the thread's last vector
+  for (; i - (U - 1) * stride >= 0; i -= U * stride) {
     Raw8<T> rx[U], rr[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      rx[u].load(x + (i + u * stride) * 8);
-      if constexpr (kResidual) rr[u].load(residual + (i + u * stride) * 8);
+      rx[u].load(x + (i - u * stride) * 8);
+      if constexpr (kResidual) rr[u].load(residual + (i - u * stride) * 8);
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) one(rx[u], rr[u], i + u * stride);
+    for (int u = 0; u < U; ++u) one(rx[u], rr[u], i - u * stride);
   }
-  for (; i < nvec; i += stride) {
+  for (; i >= 0; i -= stride) {
     Raw8<T> rx, rr;
     rx.load(x + i * 8);
     if constexpr (kResidual) rr.load(residual + i * 8);
@@ -331,20 +337,19 @@ bn_bwd_sums_kernel(const T* __restrict__ dy, const T* __restrict__ dy2, const T*
 
 // Adds the blocks' sums: the affine gradients, and what the last pass subtracts,
 // coef[0][c] = mean of dz and coef[1][c] = mean of dz * xhat * rstd.
-__global__ void __launch_bounds__(kBnFinishWarps * 32, 1)
+__global__ void __launch_bounds__(kBnFinishThreads, 1)
 bn_finish_sums_kernel(const float* __restrict__ part, int nparts, int channels, int64_t rows,
                       const float* __restrict__ rstd, float* __restrict__ dgamma, float* __restrict__ dbeta,
                       float* __restrict__ coef) {
-  __shared__ double sm[kBnFinishWarps][33];
+  __shared__ double sm[kBnFinishThreads / 32][9];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;
+  const int c = blockIdx.x * 8 + (threadIdx.x & 7), row = threadIdx.x >> 3;
   float v1[kBnFinishLoads], v2[kBnFinishLoads];
 #pragma unroll
   for (int j = 0; j < kBnFinishLoads; ++j) {
-    const int b = w + j * kBnFinishWarps;
-    const bool in = b < nparts && c < channels;
-    v1[j] = in ? part[(size_t)b * 2 * channels + c] : 0.f;
-    v2[j] = in ? part[((size_t)b * 2 + 1) * channels + c] : 0.f;
+    const int b = row + j * kBnFinishRows;
+    v1[j] = b < nparts ? part[(size_t)b * 2 * channels + c] : 0.f;
+    v2[j] = b < nparts ? part[((size_t)b * 2 + 1) * channels + c] : 0.f;
   }
   double t1 = 0.0, t2 = 0.0;
 #pragma unroll
@@ -352,10 +357,10 @@ bn_finish_sums_kernel(const float* __restrict__ part, int nparts, int channels, 
     t1 += v1[j];
     t2 += v2[j];
   }
-  t1 = sumOfColumn(t1, sm);
-  t2 = sumOfColumn(t2, sm);
-  const int mine = blockIdx.x * 32 + w;
-  if (lane == 0 && mine < channels) {
+  t1 = sumOfChannel(t1, sm);
+  t2 = sumOfChannel(t2, sm);
+  const int mine = blockIdx.x * 8 + w;
+  if (lane == 0 && w < 8) {
     const double r = rstd[mine];
     dbeta[mine] = (float)t1;
     dgamma[mine] = (float)(t2 * r);
@@ -401,18 +406,19 @@ bn_bwd_dx_kernel(const T* __restrict__ dz, const T* __restrict__ x, T* __restric
     out.set(v);
     out.store(dx + at * 8);
   };
-  int64_t i = (int64_t)blockIdx.x * kBnThreads + threadIdx.x;
-  for (; i + (U - 1) * stride < nvec; i += U * stride) {
+  const int64_t first = (int64_t)blockIdx.x * kBnThreads + threadIdx.x;
+  int64_t i = first < nvec ? first + (nvec - 1 - first) / stride * stride : -1;  // the thread's last vector
+  for (; i - (U - 1) * stride >= 0; i -= U * stride) {
     Raw8<T> rd[U], rx[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      rd[u].load(dz + (i + u * stride) * 8);
-      rx[u].load(x + (i + u * stride) * 8);
+      rd[u].load(dz + (i - u * stride) * 8);
+      rx[u].load(x + (i - u * stride) * 8);
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) one(rd[u], rx[u], i + u * stride);
+    for (int u = 0; u < U; ++u) one(rd[u], rx[u], i - u * stride);
   }
-  for (; i < nvec; i += stride) {
+  for (; i >= 0; i -= stride) {
     Raw8<T> rd, rx;
     rd.load(dz + i * 8);
     rx.load(x + i * 8);
@@ -437,7 +443,7 @@ cudaError_t forwardOf(const BatchNormShape& s, const void* x, const void* residu
   const T* rt = static_cast<const T*>(residual);
   T* yt = static_cast<T*>(y);
   bn_stats_kernel<T><<<nparts, kBnThreads, 0, stream>>>(xt, nvec, groups, part);
-  bn_finish_stats_kernel<<<(s.channels + 31) / 32, kBnFinishWarps * 32, 0, stream>>>(
+  bn_finish_stats_kernel<<<s.channels / 8, kBnFinishThreads, 0, stream>>>(
       part, nparts, kBnThreads / groups, s.channels, s.rows, eps, momentum, mean, rstd, running_mean, running_var, tracked);
   const unsigned blocks = streamBlocks(nvec, 4, sm_count);
 #define FR_BN_APPLY(R, A) \
@@ -473,7 +479,7 @@ cudaError_t backwardOf(const BatchNormShape& s, const void* dy, const void* dy2,
   else if (dy2t == nullptr) FR_BN_SUMS(kBnFromY);
   else FR_BN_SUMS(kBnFromY, true);
 #undef FR_BN_SUMS
-  bn_finish_sums_kernel<<<(s.channels + 31) / 32, kBnFinishWarps * 32, 0, stream>>>(
+  bn_finish_sums_kernel<<<s.channels / 8, kBnFinishThreads, 0, stream>>>(
       part, nparts, s.channels, s.rows, rstd, dgamma, dbeta, coef);
   const unsigned blocks = streamBlocks(nvec, 3, sm_count);
   if (relu && yt == nullptr)
