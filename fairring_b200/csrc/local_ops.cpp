@@ -74,14 +74,14 @@ void bf16GradToF32(at::Tensor dst, at::Tensor src, bool accumulate) {
   TORCH_CHECK(e == cudaSuccess, "bf16_grad_to_f32 launch failed: ", cudaGetErrorString(e));
 }
 
-// Sum of squares of a flat fp32 buffer, as a 1-element device tensor.
-at::Tensor sumSq(at::Tensor x) {
+// Sum of squares of a flat fp32 buffer, or its square root, as a 1-element device tensor.
+at::Tensor sumSq(at::Tensor x, bool root) {
   checkFlat(x, "input");
   c10::cuda::CUDAGuard guard(x.device());
-  at::Tensor out = at::zeros({1}, x.options());
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  cudaError_t e = launchSumSq(x.data_ptr<float>(), x.numel(), out.data_ptr<float>(), sms,
-                              c10::cuda::getCurrentCUDAStream());
+  at::Tensor out = at::empty({1}, x.options()), partial = at::empty({sumSqBlocks(x.numel(), sms)}, x.options());
+  cudaError_t e = launchSumSq(x.data_ptr<float>(), x.numel(), partial.data_ptr<float>(), out.data_ptr<float>(), root,
+                              sms, c10::cuda::getCurrentCUDAStream());
   TORCH_CHECK(e == cudaSuccess, "sumsq launch failed: ", cudaGetErrorString(e));
   return out;
 }
@@ -676,7 +676,7 @@ void bindLocalOps(pybind11::module_& m) {
   m.def("add_layer_norm", &addLayerNorm, py::arg("x"), py::arg("branch"), py::arg("weight"), py::arg("bias"),
         py::arg("eps"), py::arg("out_dtype"));
   m.def("cross_entropy", &crossEntropy, py::arg("logits"), py::arg("targets"), py::arg("keep"));
-  m.def("sumsq", &sumSq, py::arg("x"));
+  m.def("sumsq", &sumSq, py::arg("x"), py::arg("root") = false);
   m.def("cross_entropy_fwd", &crossEntropyForward, py::arg("logits"), py::arg("targets"),
         py::arg("bad_target") = 0.0);
   m.def("cross_entropy_mean", &crossEntropyMean, py::arg("losses"), py::arg("targets"), py::arg("least"));

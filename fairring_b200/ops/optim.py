@@ -46,7 +46,7 @@ class FlatAdamW:
         if tail is not None:
             for w in tail[1]:
                 w.wait()
-        return _C.sumsq(self.grad).sqrt()
+        return _C.sumsq(self.grad, root=True)
 
     @torch.no_grad()
     def step(self, grad_scale: float = 1.0) -> None:
