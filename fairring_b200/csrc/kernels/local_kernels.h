@@ -26,10 +26,11 @@ cudaError_t launchAdamWFlat(float* p, const float* g, float* m, float* v, void* 
 // dst (fp32, 16-byte aligned) = or += src (bf16, 16-byte aligned), n elements.
 cudaError_t launchBf16GradToF32(float* dst, const void* src_bf16, int64_t n, bool accumulate,
                                 int sm_count, cudaStream_t stream);
-// *out = sum(x^2), or its square root; `partial`: scratch of sumSqBlocks(n, sm_count) floats.
+// *out = sum(x^2), or its square root; `partial`: scratch of sumSqBlocks(n, sm_count) floats,
+// `done`: of one word.
 int sumSqBlocks(int64_t n, int sm_count);
-cudaError_t launchSumSq(const float* x, int64_t n, float* partial, float* out, bool root, int sm_count,
-                        cudaStream_t stream);
+cudaError_t launchSumSq(const float* x, int64_t n, float* partial, unsigned* done, float* out, bool root,
+                        int sm_count, cudaStream_t stream);
 
 // Device-to-device copy by a kernel of at most `blocks` blocks (falls back to
 // cudaMemcpyAsync when a pointer is not 16-byte aligned).

@@ -79,9 +79,11 @@ at::Tensor sumSq(at::Tensor x, bool root) {
   checkFlat(x, "input");
   c10::cuda::CUDAGuard guard(x.device());
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  at::Tensor out = at::empty({1}, x.options()), partial = at::empty({sumSqBlocks(x.numel(), sms)}, x.options());
-  cudaError_t e = launchSumSq(x.data_ptr<float>(), x.numel(), partial.data_ptr<float>(), out.data_ptr<float>(), root,
-                              sms, c10::cuda::getCurrentCUDAStream());
+  const int blocks = sumSqBlocks(x.numel(), sms);
+  at::Tensor out = at::empty({1}, x.options()), scratch = at::empty({blocks + 1}, x.options());
+  float* partial = scratch.data_ptr<float>();
+  cudaError_t e = launchSumSq(x.data_ptr<float>(), x.numel(), partial, reinterpret_cast<unsigned*>(partial + blocks),
+                              out.data_ptr<float>(), root, sms, c10::cuda::getCurrentCUDAStream());
   TORCH_CHECK(e == cudaSuccess, "sumsq launch failed: ", cudaGetErrorString(e));
   return out;
 }
