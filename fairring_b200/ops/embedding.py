@@ -22,7 +22,8 @@ class _TiedEmbeddingFn(torch.autograd.Function):
         ctx.vocab, ctx.positions, ctx.d = table.shape[0], pos.shape[0], table.shape[1]
         low = table.new_empty((rows, ctx.d), dtype=torch.bfloat16)
         low[: ctx.vocab].copy_(table)
-        low[ctx.vocab:].zero_()
+        if rows > ctx.vocab:
+            low[ctx.vocab:].zero_()
         return _C.embed_fwd(tokens, table, pos), low
 
     @staticmethod
@@ -52,10 +53,14 @@ def _plain_table(m: nn.Module) -> bool:
             and m.weight.is_contiguous() and m.weight.data_ptr() % 16 == 0)
 
 
+# Table elements from which rows are padded: below, the head's products are bound by their launches.
+_PAD_FROM = 1 << 22
+
+
 def tied_embedding(tok: nn.Embedding, pos: nn.Embedding, tokens: torch.Tensor, pad_rows: bool = False):
     """``(tok(tokens) + pos(0, 1, ...), table)``: ``table`` is what the output projection multiplies
-    with, ``tok.weight`` or, where the fused form applies, its bf16 copy, with ``pad_rows`` with rows of
-    zeros behind it up to a multiple of 8 (see :func:`fairring_b200.ops.vocab_logits`).  Fused in training under bf16
+    with, ``tok.weight`` or, where the fused form applies, its bf16 copy, with ``pad_rows`` and a large table
+    with rows of zeros behind it up to a multiple of 8 (see :func:`fairring_b200.ops.vocab_logits`).  Fused in training under bf16
     autocast on the GPU.  The rows of equal tokens are added in no fixed order, so under
     ``torch.use_deterministic_algorithms`` the modules are called."""
     if (tokens.is_cuda and tokens.dim() == 2 and tokens.dtype == torch.long and tokens.numel() > 0
@@ -65,6 +70,6 @@ def tied_embedding(tok: nn.Embedding, pos: nn.Embedding, tokens: torch.Tensor, p
             and tok.embedding_dim % 8 == 0 and tokens.shape[1] <= pos.num_embeddings
             and not torch.are_deterministic_algorithms_enabled() and plain_autograd()):
         rows = tok.num_embeddings
-        rows = (rows + 7) // 8 * 8 if pad_rows else rows
+        rows = (rows + 7) // 8 * 8 if pad_rows and tok.weight.numel() >= _PAD_FROM else rows
         return _TiedEmbeddingFn.apply(tokens.contiguous(), tok.weight, pos.weight, rows)
     return tok(tokens) + pos(torch.arange(tokens.shape[1], device=tokens.device)), tok.weight
