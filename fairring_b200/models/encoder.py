@@ -85,14 +85,15 @@ class EncoderMLM(nn.Module):
     def forward(self, tokens: torch.Tensor, labels: torch.Tensor | None = None):
         """``labels``: target ids at masked positions, -100 elsewhere."""
         from ..ops import cross_entropy_keeping_logits, linear_gelu, tied_embedding, vocab_logits
-        from ..ops._plain import plain_module
+        from ..ops._plain import FUSE_FROM, plain_module
 
         b, s = tokens.shape
         x, table = tied_embedding(self.tok, self.pos, tokens, pad_rows=labels is not None)
         x = self.ln_emb(x)
         low = x
+        large = x.is_cuda and b * s * self.cfg.d_ff >= FUSE_FROM  # else nothing in forward_pair() is fused
         for layer in self.layers:
-            if x.is_cuda and plain_module(layer, EncoderLayer):
+            if large and plain_module(layer, EncoderLayer):
                 x, low = layer.forward_pair(x, low)
             else:
                 x = low = layer(x)

@@ -8,6 +8,11 @@ from torch.autograd import forward_ad
 from torch.nn.modules import module as _module
 
 
+# Elements from which the Python nodes of this package are used.  Below, torch's kernels are bound by
+# their launches just as the package's are, and a Python node costs the host more than it saves.
+FUSE_FROM = 1 << 22
+
+
 def plain_autograd() -> bool:
     """False inside the transforms that look through torch's own ops but not through an
     ``autograd.Function`` around a native kernel: functorch (``vmap``, ``grad``, ``jvp``),

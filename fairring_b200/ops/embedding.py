@@ -8,7 +8,7 @@ import torch
 import torch.nn as nn
 
 from .. import _C
-from ._plain import plain_autograd, plain_module
+from ._plain import FUSE_FROM, plain_autograd, plain_module
 
 
 class _TiedEmbeddingFn(torch.autograd.Function):
@@ -54,7 +54,7 @@ def _plain_table(m: nn.Module) -> bool:
 
 
 # Table elements from which rows are padded: below, the head's products are bound by their launches.
-_PAD_FROM = 1 << 22
+_PAD_FROM = FUSE_FROM
 
 
 def tied_embedding(tok: nn.Embedding, pos: nn.Embedding, tokens: torch.Tensor, pad_rows: bool = False):

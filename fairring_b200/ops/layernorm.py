@@ -17,7 +17,7 @@ import torch.nn as nn
 from torch.autograd.function import once_differentiable
 
 from .. import _C
-from ._plain import plain_autograd, plain_module
+from ._plain import FUSE_FROM, plain_autograd, plain_module
 
 
 # The nodes below are used where torch looks into an autograd function (tracing, compilation) or
@@ -141,10 +141,9 @@ class _AddLayerNormPairFn(torch.autograd.Function):
         return dx, (dbr if want_bf16 else dx), dgamma, dbeta, None, None
 
 
-# Elements from which the pair's node is used.  Below, torch's kernels are bound by their launches too, and the
-# Python node costs the host more than it saves: an encoder step of 1104 x 256 took 2370 us without it and
-# the padded head, 2570 us with them; from 8192 x 2048 on the node halves the device time.
-_PAIR_FROM = 1 << 22
+# Elements from which the pair's node is used: an encoder step of 1104 x 256 took 2370 us without it and the
+# padded head, 2570 us with them; from 8192 x 2048 on the node halves the device time.
+_PAIR_FROM = FUSE_FROM
 
 
 def add_layer_norm_pair(norm: nn.LayerNorm, x: torch.Tensor, branch: torch.Tensor):
@@ -153,10 +152,10 @@ def add_layer_norm_pair(norm: nn.LayerNorm, x: torch.Tensor, branch: torch.Tenso
     for an ``nn.LayerNorm`` and an fp32 ``x`` on the GPU under bf16 autocast; otherwise both are
     what ``norm`` returns."""
     d = x.shape[-1]
-    if (x.is_cuda and plain_module(norm, nn.LayerNorm) and torch.is_autocast_enabled("cuda")
+    if (x.is_cuda and x.numel() >= max(1, _PAIR_FROM) and plain_module(norm, nn.LayerNorm) and torch.is_autocast_enabled("cuda")
             and torch.get_autocast_dtype("cuda") == torch.bfloat16 and x.dtype == torch.float32
             and branch.dtype in (torch.float32, torch.bfloat16) and branch.shape == x.shape
-            and branch.device == x.device and x.numel() >= max(1, _PAIR_FROM) and norm.normalized_shape == (d,) and d % 8 == 0
+            and branch.device == x.device and norm.normalized_shape == (d,) and d % 8 == 0
             and d <= 8192 and norm.weight is not None and norm.bias is not None
             and norm.weight.dtype == norm.bias.dtype == torch.float32 and norm.weight.device == x.device
             and plain_autograd()):

@@ -13,7 +13,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _C
-from ._plain import plain_autograd, plain_module
+from ._plain import FUSE_FROM, plain_autograd, plain_module
 
 
 class _LowWeightFn(torch.autograd.Function):
@@ -74,11 +74,9 @@ class _GeluFn(torch.autograd.Function):
         return dh, db, None
 
 
-# Output elements from which the fused forms are used.  Below, torch's kernels are bound by their
-# launches just as these are, and the host time of a Python autograd function costs more than they
-# save: a two-layer model of width 128 (0.1 M elements) takes 2465 us a step without and 2640 us
-# with them, while at 6 M elements the sum alone is 28 us against 12 us.
-_FUSE_FROM = 1 << 22
+# Output elements from which the fused forms are used: a two-layer model of width 128 (0.1 M elements) takes
+# 2465 us a step without and 2640 us with them, while at 6 M elements the sum alone is 28 us against 12 us.
+_FUSE_FROM = FUSE_FROM
 
 
 def _fusable(fc: nn.Linear, x: torch.Tensor) -> bool:

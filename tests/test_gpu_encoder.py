@@ -17,6 +17,7 @@ def _small_sizes_too(monkeypatch):
 
     monkeypatch.setattr(sys.modules["fairring_b200.ops.layernorm"], "_PAIR_FROM", 0)
     monkeypatch.setattr(sys.modules["fairring_b200.ops.embedding"], "_PAD_FROM", 0)
+    monkeypatch.setattr(sys.modules["fairring_b200.ops._plain"], "FUSE_FROM", 0)
 
 
 def _need_gpu():
