@@ -128,9 +128,10 @@ cudaError_t launchMaxPoolBackward(const PoolShape& s, bool bf16, const void* dy,
 // x[b][s] = table[tokens[b][s]] + pos[s], rows of d floats (a multiple of 4), 16-byte aligned.
 cudaError_t launchEmbedForward(const int64_t* tokens, const float* table, const float* pos, float* x, int batch, int seq,
                                int64_t vocab, int d, cudaStream_t stream);
-// dtable[tokens[b][s]] += dx[b][s]; dpos[s] = sum over b of dx[b][s].
+// dtable[tokens[b][s]] += dx[b][s]; dpos[s] = sum over b of dx[b][s].  The order of the additions depends on
+// the tokens and the sizes alone.
 cudaError_t launchEmbedBackward(const float* dx, const int64_t* tokens, float* dtable, float* dpos, int batch, int seq,
-                                int64_t vocab, int d, cudaStream_t stream);
+                                int64_t vocab, int d, int sm_count, cudaStream_t stream);
 
 // Channels-last [images, 3, height, width] (fp32 or bf16) to channels-last bf16 [images, 16, rows, cols]:
 // the 2 x 2 pixel blocks from row and column -4 on, 4 x 3 channels and 4 zeros; zero outside the image.

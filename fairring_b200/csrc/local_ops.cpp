@@ -547,7 +547,7 @@ std::tuple<at::Tensor, at::Tensor> embedBackward(std::optional<at::Tensor> dx, s
   const at::Tensor g = aligned16(*dx);
   at::Tensor dpos = tokens.size(1) < positions ? at::zeros({positions, d}, fopt) : at::empty({positions, d}, fopt);
   cudaError_t e = launchEmbedBackward(g.data_ptr<float>(), tokens.data_ptr<int64_t>(), dtable.data_ptr<float>(),
-                                      dpos.data_ptr<float>(), (int)tokens.size(0), (int)tokens.size(1), vocab, (int)d,
+                                      dpos.data_ptr<float>(), (int)tokens.size(0), (int)tokens.size(1), vocab, (int)d, sms,
                                       stream);
   TORCH_CHECK(e == cudaSuccess, "embedding backward launch failed: ", cudaGetErrorString(e));
   return std::make_tuple(dtable, dpos);

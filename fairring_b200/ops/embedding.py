@@ -61,14 +61,14 @@ def tied_embedding(tok: nn.Embedding, pos: nn.Embedding, tokens: torch.Tensor, p
     """``(tok(tokens) + pos(0, 1, ...), table)``: ``table`` is what the output projection multiplies
     with, ``tok.weight`` or, where the fused form applies, its bf16 copy, with ``pad_rows`` and a large table
     with rows of zeros behind it up to a multiple of 8 (see :func:`fairring_b200.ops.vocab_logits`).  Fused in training under bf16
-    autocast on the GPU.  The rows of equal tokens are added in no fixed order, so under
-    ``torch.use_deterministic_algorithms`` the modules are called."""
+    autocast on the GPU.  The gradients of equal tokens are added in an order that the tokens fix: a step
+    repeats itself bit for bit."""
     if (tokens.is_cuda and tokens.dim() == 2 and tokens.dtype == torch.long and tokens.numel() > 0
             and torch.is_grad_enabled() and torch.is_autocast_enabled("cuda")
             and torch.get_autocast_dtype("cuda") == torch.bfloat16 and _plain_table(tok) and _plain_table(pos)
             and tok.weight.device == pos.weight.device == tokens.device and tok.embedding_dim == pos.embedding_dim
             and tok.embedding_dim % 8 == 0 and tokens.shape[1] <= pos.num_embeddings
-            and not torch.are_deterministic_algorithms_enabled() and plain_autograd()):
+            and plain_autograd()):
         rows = tok.num_embeddings
         rows = (rows + 7) // 8 * 8 if pad_rows and tok.weight.numel() >= _PAD_FROM else rows
         return _TiedEmbeddingFn.apply(tokens.contiguous(), tok.weight, pos.weight, rows)

@@ -47,6 +47,38 @@ def test_matches_torch(d, batch, seq, positions, use):
         assert float((a - b).abs().max()) <= 2e-6 * (batch * seq) ** 0.5 * max(1.0, float(b.abs().max()))
 
 
+# less than a round of the token lists, two rounds and a ragged third; tokens of one occurrence, of a warp's
+# share, of all warps' (32 and more within a round) and a batch of nothing else
+@pytest.mark.parametrize("d", [8, 136, 2048])
+@pytest.mark.parametrize("batch,seq", [(1, 7), (3, 700), (5, 1001)])
+@pytest.mark.parametrize("mix", ["spread", "frequent", "one"])
+def test_the_gradient_repeats_itself(d, batch, seq, mix):
+    _need_gpu()
+    from fairring_b200 import _C
+
+    vocab, n = 613, batch * seq
+    gen = torch.Generator(device="cuda").manual_seed(d + n)
+    tokens = torch.randint(0, vocab, (batch, seq), device="cuda", generator=gen)
+    if mix == "frequent":
+        tokens[torch.rand(batch, seq, device="cuda", generator=gen) < 0.4] = 612
+        tokens[:, ::9] = 3
+    elif mix == "one":
+        tokens[:] = 5
+    dx = torch.randn(batch, seq, d, device="cuda", generator=gen)
+    dlow = torch.randn(vocab, d, device="cuda", generator=gen).bfloat16()
+    dtable, dpos = _C.embed_bwd(dx, dlow, tokens, vocab, seq + 2, d)
+    rows = dx.view(n, d).double()
+    want = dlow.double().index_add_(0, tokens.view(-1), rows)
+    most = dlow.double().abs().index_add_(0, tokens.view(-1), rows.abs())  # a rounding for each term at the most
+    times = torch.bincount(tokens.view(-1), minlength=vocab).view(-1, 1) + 1
+    assert ((dtable.double() - want).abs() <= 2.0 ** -24 * times * most).all()
+    assert ((dpos[:seq].double() - dx.double().sum(0)).abs() <= 2.0 ** -24 * batch * dx.double().abs().sum(0)).all()
+    assert not dpos[seq:].any()
+    for _ in range(3):
+        again = _C.embed_bwd(dx, dlow, tokens, vocab, seq + 2, d)
+        assert torch.equal(again[0], dtable) and torch.equal(again[1], dpos)
+
+
 def test_calls_the_modules_where_they_cannot_be_skipped():
     _need_gpu()
     from fairring_b200.ops import tied_embedding
