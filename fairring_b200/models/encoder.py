@@ -12,6 +12,9 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops import add_layer_norm_pair, cross_entropy_keeping_logits, linear, linear_gelu, tied_embedding, vocab_logits
+from ..ops._plain import FUSE_FROM, native, plain_module
+
 
 @dataclass
 class EncoderConfig:
@@ -53,8 +56,6 @@ class EncoderLayer(nn.Module):
     def forward_pair(self, x: torch.Tensor, low: torch.Tensor):
         """The same layer on the stream and its copy in the autocast dtype, which the linear layers read:
         takes and returns both, so that each LayerNorm's backward takes both gradients at once."""
-        from ..ops import add_layer_norm_pair, linear, linear_gelu
-
         b, s, d = x.shape
         q, k, v = linear(self.qkv, low).view(b, s, 3, self.n_head, d // self.n_head).unbind(2)
         a = F.scaled_dot_product_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2))
@@ -84,14 +85,30 @@ class EncoderMLM(nn.Module):
 
     def forward(self, tokens: torch.Tensor, labels: torch.Tensor | None = None):
         """``labels``: target ids at masked positions, -100 elsewhere."""
-        from ..ops import cross_entropy_keeping_logits, linear_gelu, tied_embedding, vocab_logits
-        from ..ops._plain import FUSE_FROM, plain_module
+        if not torch.jit.is_scripting():
+            if native(tokens):
+                return self._forward_native(tokens, labels)
+        b, s = tokens.shape
+        x = self.ln_emb(self.tok(tokens) + self.pos(torch.arange(s, device=tokens.device)))
+        for layer in self.layers:
+            x = layer(x)
+        if labels is None:
+            h = self.head_ln(F.gelu(self.head_dense(x)))
+            return F.linear(h, self.tok.weight, self.head_bias)
+        # Only masked positions go through the vocabulary projection.
+        sel = labels.reshape(-1) != -100
+        h = x.reshape(b * s, -1)[sel]
+        h = self.head_ln(F.gelu(self.head_dense(h)))
+        logits = F.linear(h, self.tok.weight, self.head_bias)
+        return F.cross_entropy(logits.float(), labels.reshape(-1)[sel])
 
+    def _forward_native(self, tokens: torch.Tensor, labels: torch.Tensor | None):
+        """The same on the ops of this package."""
         b, s = tokens.shape
         x, table = tied_embedding(self.tok, self.pos, tokens, pad_rows=labels is not None)
         x = self.ln_emb(x)
         low = x
-        large = x.is_cuda and b * s * self.cfg.d_ff >= FUSE_FROM  # else nothing in forward_pair() is fused
+        large = x.is_cuda and b * s * self.cfg.d_ff >= FUSE_FROM
         for layer in self.layers:
             if large and plain_module(layer, EncoderLayer):
                 x, low = layer.forward_pair(x, low)
@@ -100,7 +117,6 @@ class EncoderMLM(nn.Module):
         if labels is None:
             h = self.head_ln(F.gelu(self.head_dense(x)))
             return F.linear(h, table, self.head_bias)
-        # Only masked positions go through the vocabulary projection.
         sel = labels.reshape(-1) != -100
         h = low.reshape(b * s, -1)[sel]
         h = self.head_ln(linear_gelu(self.head_dense, h))

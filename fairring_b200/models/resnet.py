@@ -11,6 +11,9 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from ..ops import batch_norm_act, max_pool, stem_conv
+from ..ops._plain import native, plain_module
+
 
 class Bottleneck(nn.Module):
     expansion = 4
@@ -27,29 +30,26 @@ class Bottleneck(nn.Module):
         self.downsample = downsample
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return self.forward_pair(x, x)[0]
+        if not torch.jit.is_scripting():
+            if native(x):
+                return self.forward_pair(x, x)[0]
+        identity = x if self.downsample is None else self.downsample(x)
+        out = self.relu(self.bn1(self.conv1(x)))
+        out = self.relu(self.bn2(self.conv2(out)))
+        out = self.bn3(self.conv3(out))
+        return self.relu(out + identity)
 
     def forward_pair(self, x: torch.Tensor, shortcut: torch.Tensor):
         """The block on an input that comes twice, for its convolutions and for its shortcut; so does
         the output, whose two gradients the backward then adds inside the BatchNorm."""
-        from ..ops import batch_norm_act
-
-        identity = shortcut if self.downsample is None else self.downsample(shortcut)
+        identity, down = shortcut, self.downsample
+        if down is not None and plain_module(down, nn.Sequential) and len(down) == 2:
+            identity = batch_norm_act(down[1], down[0](shortcut))
+        elif down is not None:
+            identity = down(shortcut)
         out = batch_norm_act(self.bn1, self.conv1(x), relu=self.relu)
         out = batch_norm_act(self.bn2, self.conv2(out), relu=self.relu)
         return batch_norm_act(self.bn3, self.conv3(out), residual=identity, relu=self.relu, twice=True)
-
-
-class Downsample(nn.Sequential):
-    """Strided 1x1 convolution and BatchNorm of a block's shortcut."""
-
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
-        from ..ops import batch_norm_act
-
-        if len(self) != 2:
-            return super().forward(x)
-        conv, bn = self
-        return batch_norm_act(bn, conv(x))
 
 
 class ResNet50(nn.Module):
@@ -76,7 +76,7 @@ class ResNet50(nn.Module):
     def _make_layer(self, planes: int, blocks: int, stride: int = 1) -> nn.Sequential:
         downsample = None
         if stride != 1 or self.inplanes != planes * Bottleneck.expansion:
-            downsample = Downsample(
+            downsample = nn.Sequential(
                 nn.Conv2d(self.inplanes, planes * Bottleneck.expansion, 1, stride=stride, bias=False),
                 nn.BatchNorm2d(planes * Bottleneck.expansion),
             )
@@ -89,9 +89,15 @@ class ResNet50(nn.Module):
         return sum(p.numel() for p in self.parameters())
 
     def forward(self, images: torch.Tensor, labels: torch.Tensor | None = None):
-        from ..ops import batch_norm_act, max_pool, stem_conv
-        from ..ops._plain import plain_module
+        if not torch.jit.is_scripting():
+            if native(images):
+                return self._head(self._stages(images), labels)
+        x = self.maxpool(self.relu(self.bn1(self.conv1(images))))
+        x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
+        return self._head(x, labels)
 
+    def _stages(self, images: torch.Tensor) -> torch.Tensor:
+        """What stands in front of the pooling, on the ops of this package."""
         x = max_pool(self.maxpool, batch_norm_act(self.bn1, stem_conv(self.conv1, images), relu=self.relu))
         shortcut = x
         for stage in (self.layer1, self.layer2, self.layer3, self.layer4):
@@ -100,6 +106,9 @@ class ResNet50(nn.Module):
                     x, shortcut = block.forward_pair(x, shortcut)
             else:
                 x = shortcut = stage(x)
+        return x
+
+    def _head(self, x: torch.Tensor, labels: torch.Tensor | None = None):
         logits = self.fc(torch.flatten(self.avgpool(x), 1))
         if labels is None:
             return logits

@@ -14,11 +14,25 @@ FUSE_FROM = 1 << 22
 
 
 def plain_autograd() -> bool:
-    """False inside the transforms that look through torch's own ops but not through an
-    ``autograd.Function`` around a native kernel: functorch (``vmap``, ``grad``, ``jvp``),
-    forward-mode differentiation, tracing and compilation; and in inference mode."""
-    return not (torch.is_inference_mode_enabled() or torch._C._are_functorch_transforms_active()
-                or forward_ad._current_level >= 0 or torch.compiler.is_compiling() or torch.jit.is_tracing())
+    """False inside what looks through torch's own ops but not through a native kernel: tracing and
+    compilation, dispatch modes (``make_fx``, fake tensors, FLOP counting), functorch (``vmap``,
+    ``grad``, ``jvp``), forward-mode differentiation; and in inference mode."""
+    if torch.compiler.is_compiling():  # asked first: Dynamo refuses some of the questions below
+        return False
+    return not (torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0
+                or torch.is_inference_mode_enabled() or torch._C._are_functorch_transforms_active()
+                or forward_ad._current_level >= 0)
+
+
+def ordinary(x) -> bool:
+    """Neither a tracer's stand-in nor a tensor subclass, which may have no memory of its own."""
+    return type(x) in (torch.Tensor, nn.Parameter)
+
+
+def native(x) -> bool:
+    """Whether a kernel may be handed ``x``: an ordinary tensor on the GPU, where nothing is traced.  To be
+    asked before any other property of ``x``, which a tracer's stand-in does not answer."""
+    return ordinary(x) and plain_autograd() and x.is_cuda
 
 
 def plain_module(m: nn.Module, cls: type) -> bool:

@@ -14,7 +14,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _C
-from ._plain import plain_autograd, plain_module
+from ._plain import native, ordinary, plain_module
 
 
 class _BatchNormActFn(torch.autograd.Function):
@@ -64,22 +64,22 @@ def _channels_last(t: torch.Tensor) -> bool:
 
 
 def _fusable(bn: nn.BatchNorm2d, x: torch.Tensor, residual: torch.Tensor | None) -> bool:
-    if not (bn.training and plain_module(bn, nn.BatchNorm2d) and x.is_cuda and x.dim() == 4):
+    if not (native(x) and bn.training and plain_module(bn, nn.BatchNorm2d) and x.dim() == 4):
         return False
     c = x.shape[1]
     params = (bn.weight, bn.bias, bn.running_mean, bn.running_var)
     if bn.momentum is None or bn.num_batches_tracked is None or any(
-            p is None or p.dtype != torch.float32 or p.device != x.device or p.numel() != c or not p.is_contiguous()
+            p is None or not ordinary(p) or p.dtype != torch.float32 or p.device != x.device or p.numel() != c or not p.is_contiguous()
             or p.data_ptr() % 16 for p in params):
         return False
     if bn.num_batches_tracked.device != x.device or bn.num_batches_tracked.dtype != torch.long:
         return False
     if x.dtype not in (torch.float32, torch.bfloat16) or not 8 <= c <= 2048 or c & (c - 1) or x.numel() <= c:
         return False
-    if residual is not None and (residual.dtype != x.dtype or residual.shape != x.shape or residual.device != x.device
+    if residual is not None and (not ordinary(residual) or residual.dtype != x.dtype or residual.shape != x.shape or residual.device != x.device
                                  or not _channels_last(residual)):
         return False
-    return _channels_last(x) and plain_autograd()
+    return _channels_last(x)
 
 
 def batch_norm_act(bn: nn.Module, x: torch.Tensor, residual: torch.Tensor | None = None,
@@ -90,7 +90,7 @@ def batch_norm_act(bn: nn.Module, x: torch.Tensor, residual: torch.Tensor | None
     ``nn.BatchNorm2d`` in training mode and a channels-last fp32 or bf16 ``x`` on the GPU with a
     power of two from 8 to 2048 channels; otherwise, and when one of the modules carries hooks or
     has been replaced, the modules are called."""
-    if (relu is None or plain_module(relu, nn.ReLU)) and _fusable(bn, x, residual):
+    if _fusable(bn, x, residual) and (relu is None or plain_module(relu, nn.ReLU)):
         return _BatchNormActFn.apply(x, residual, bn.weight, bn.bias, bn.running_mean, bn.running_var,
                                      bn.num_batches_tracked, bn.momentum, bn.eps, relu is not None, twice)
     y = bn(x)

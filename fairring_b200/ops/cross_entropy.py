@@ -14,7 +14,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import _C
-from ._plain import plain_autograd
+from ._plain import native, plain_autograd
 
 
 class _FusedCrossEntropyFn(torch.autograd.Function):
@@ -53,9 +53,9 @@ def fused_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Te
 def cross_entropy_keeping_logits(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
     """``F.cross_entropy(logits.float(), targets)`` (negative targets are ignored) by the same kernels;
     the logits stay as they are whatever the vocabulary."""
-    if (logits.is_cuda and logits.dim() == 2 and logits.is_contiguous() and logits.shape[1] > 0
+    if (native(logits) and logits.dim() == 2 and logits.is_contiguous() and logits.shape[1] > 0
             and logits.dtype in (torch.float32, torch.bfloat16) and logits.data_ptr() % 16 == 0
             and targets.dtype == torch.long and targets.shape == logits.shape[:1]
-            and targets.device == logits.device and plain_autograd()):
+            and targets.device == logits.device):
         return _C.cross_entropy(logits, targets.contiguous(), True)
     return F.cross_entropy(logits.float(), targets, ignore_index=-100)

@@ -8,7 +8,7 @@ import torch
 import torch.nn as nn
 
 from .. import _C
-from ._plain import FUSE_FROM, plain_autograd, plain_module
+from ._plain import FUSE_FROM, native, ordinary, plain_module
 
 
 class _TiedEmbeddingFn(torch.autograd.Function):
@@ -48,7 +48,7 @@ class _TiedEmbeddingFn(torch.autograd.Function):
 
 
 def _plain_table(m: nn.Module) -> bool:
-    return (plain_module(m, nn.Embedding) and m.padding_idx is None and m.max_norm is None and not m.sparse
+    return (plain_module(m, nn.Embedding) and ordinary(m.weight) and m.padding_idx is None and m.max_norm is None and not m.sparse
             and not m.scale_grad_by_freq and m.weight.requires_grad and m.weight.dtype == torch.float32
             and m.weight.is_contiguous() and m.weight.data_ptr() % 16 == 0)
 
@@ -63,12 +63,11 @@ def tied_embedding(tok: nn.Embedding, pos: nn.Embedding, tokens: torch.Tensor, p
     with rows of zeros behind it up to a multiple of 8 (see :func:`fairring_b200.ops.vocab_logits`).  Fused in training under bf16
     autocast on the GPU.  The gradients of equal tokens are added in an order that the tokens fix: a step
     repeats itself bit for bit."""
-    if (tokens.is_cuda and tokens.dim() == 2 and tokens.dtype == torch.long and tokens.numel() > 0
+    if (native(tokens) and tokens.dim() == 2 and tokens.dtype == torch.long and tokens.numel() > 0
             and torch.is_grad_enabled() and torch.is_autocast_enabled("cuda")
             and torch.get_autocast_dtype("cuda") == torch.bfloat16 and _plain_table(tok) and _plain_table(pos)
             and tok.weight.device == pos.weight.device == tokens.device and tok.embedding_dim == pos.embedding_dim
-            and tok.embedding_dim % 8 == 0 and tokens.shape[1] <= pos.num_embeddings
-            and plain_autograd()):
+            and tok.embedding_dim % 8 == 0 and tokens.shape[1] <= pos.num_embeddings):
         rows = tok.num_embeddings
         rows = (rows + 7) // 8 * 8 if pad_rows and tok.weight.numel() >= _PAD_FROM else rows
         return _TiedEmbeddingFn.apply(tokens.contiguous(), tok.weight, pos.weight, rows)

@@ -17,7 +17,7 @@ import torch.nn as nn
 from torch.autograd.function import once_differentiable
 
 from .. import _C
-from ._plain import FUSE_FROM, plain_autograd, plain_module
+from ._plain import FUSE_FROM, native, plain_autograd, plain_module
 
 
 # The nodes below are used where torch looks into an autograd function (tracing, compilation) or
@@ -152,13 +152,12 @@ def add_layer_norm_pair(norm: nn.LayerNorm, x: torch.Tensor, branch: torch.Tenso
     for an ``nn.LayerNorm`` and an fp32 ``x`` on the GPU under bf16 autocast; otherwise both are
     what ``norm`` returns."""
     d = x.shape[-1]
-    if (x.is_cuda and x.numel() >= max(1, _PAIR_FROM) and plain_module(norm, nn.LayerNorm) and torch.is_autocast_enabled("cuda")
+    if (native(x) and x.numel() >= max(1, _PAIR_FROM) and plain_module(norm, nn.LayerNorm) and torch.is_autocast_enabled("cuda")
             and torch.get_autocast_dtype("cuda") == torch.bfloat16 and x.dtype == torch.float32
             and branch.dtype in (torch.float32, torch.bfloat16) and branch.shape == x.shape
             and branch.device == x.device and norm.normalized_shape == (d,) and d % 8 == 0
             and d <= 8192 and norm.weight is not None and norm.bias is not None
-            and norm.weight.dtype == norm.bias.dtype == torch.float32 and norm.weight.device == x.device
-            and plain_autograd()):
+            and norm.weight.dtype == norm.bias.dtype == torch.float32 and norm.weight.device == x.device):
         return _AddLayerNormPairFn.apply(x, branch, norm.weight, norm.bias, norm.eps, torch.bfloat16)
     y = norm(x + branch)
     return y, y

@@ -13,7 +13,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _C
-from ._plain import FUSE_FROM, plain_autograd, plain_module
+from ._plain import FUSE_FROM, native, ordinary, plain_module
 
 
 class _LowWeightFn(torch.autograd.Function):
@@ -81,9 +81,9 @@ _FUSE_FROM = FUSE_FROM
 
 def _fusable(fc: nn.Linear, x: torch.Tensor) -> bool:
     """Whether the layer's output will be bf16 on the GPU and large, and its bias wants a gradient."""
-    if x.dim() < 2 or x.numel() // max(1, x.shape[-1]) * fc.out_features < _FUSE_FROM:
+    if not native(x) or x.dim() < 2 or x.numel() // max(1, x.shape[-1]) * fc.out_features < _FUSE_FROM:
         return False
-    if not (plain_module(fc, nn.Linear) and x.is_cuda and fc.bias is not None
+    if not (plain_module(fc, nn.Linear) and ordinary(fc.weight) and fc.bias is not None
             and fc.bias.requires_grad and torch.is_grad_enabled() and fc.out_features % 8 == 0
             and fc.bias.dtype in (torch.float32, torch.bfloat16) and fc.bias.device == x.device):
         return False
@@ -92,7 +92,7 @@ def _fusable(fc: nn.Linear, x: torch.Tensor) -> bool:
         bf16 = bf16 and x.dtype in (torch.float32, torch.bfloat16) and fc.weight.dtype in (torch.float32, torch.bfloat16)
     else:
         bf16 = x.dtype == fc.weight.dtype == fc.bias.dtype == torch.bfloat16
-    return bf16 and plain_autograd()
+    return bf16
 
 
 def linear(fc: nn.Linear, x: torch.Tensor) -> torch.Tensor:

@@ -8,7 +8,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _C
-from ._plain import plain_autograd, plain_module
+from ._plain import native, plain_module
 
 
 class _MaxPoolFn(torch.autograd.Function):
@@ -38,12 +38,12 @@ def _square(v) -> int | None:
 def max_pool(pool: nn.Module, x: torch.Tensor) -> torch.Tensor:
     """``pool(x)``; for an ``nn.MaxPool2d`` with a square window and a channels-last fp32 or bf16 ``x``
     on the GPU that wants a gradient, by the kernels of this package."""
-    if (plain_module(pool, nn.MaxPool2d) and x.is_cuda and x.dim() == 4 and x.requires_grad and torch.is_grad_enabled()
+    if (native(x) and plain_module(pool, nn.MaxPool2d) and x.dim() == 4 and x.requires_grad and torch.is_grad_enabled()
             and x.dtype in (torch.float32, torch.bfloat16) and x.shape[1] % 8 == 0 and 0 < x.numel() // 8 < 2 ** 31 - 1
             and x.is_contiguous(memory_format=torch.channels_last) and x.data_ptr() % 16 == 0
             and _square(pool.dilation) == 1 and not pool.ceil_mode and not pool.return_indices):
         window, stride, pad = _square(pool.kernel_size), _square(pool.stride), _square(pool.padding)
         if (None not in (window, stride, pad) and 1 <= window <= 16 and stride >= 1 and 0 <= 2 * pad <= window
-                and min(x.shape[2:]) + 2 * pad >= window and plain_autograd()):
+                and min(x.shape[2:]) + 2 * pad >= window):
             return _MaxPoolFn.apply(x, window, stride, pad)
     return pool(x)

@@ -9,7 +9,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _C
-from ._plain import plain_autograd, plain_module
+from ._plain import native, plain_module
 
 # Output pixels from which the fold pays: below, the launches that fold the weight cost the host more
 # than the 0.35 ms per million pixels that the convolution gains.
@@ -40,7 +40,7 @@ class _StemConvFn(torch.autograd.Function):
 def stem_conv(conv: nn.Module, images: torch.Tensor) -> torch.Tensor:
     """``conv(images)``; folded for a plain 7 x 7, stride 2, padding 3 convolution of channels-last images
     that want no gradient, in training under bf16 autocast on the GPU."""
-    if (images.is_cuda and images.dim() == 4 and images.shape[1] == 3 and not images.requires_grad
+    if (native(images) and images.dim() == 4 and images.shape[1] == 3 and not images.requires_grad
             and plain_module(conv, nn.Conv2d) and conv.in_channels == 3 and conv.kernel_size == (7, 7)
             and conv.stride == (2, 2) and conv.padding == (3, 3) and conv.dilation == (1, 1) and conv.groups == 1
             and conv.bias is None and conv.padding_mode == "zeros" and conv.out_channels % 8 == 0
@@ -48,6 +48,6 @@ def stem_conv(conv: nn.Module, images: torch.Tensor) -> torch.Tensor:
             and conv.weight.device == images.device and conv.weight.requires_grad and torch.is_grad_enabled()
             and images.is_contiguous(memory_format=torch.channels_last) and torch.is_autocast_enabled("cuda")
             and torch.get_autocast_dtype("cuda") == torch.bfloat16
-            and images.numel() // 12 >= _FOLD_FROM and images.numel() < 2 ** 31 and plain_autograd()):
+            and images.numel() // 12 >= _FOLD_FROM and images.numel() < 2 ** 31):
         return _StemConvFn.apply(images, conv.weight)
     return conv(images)
