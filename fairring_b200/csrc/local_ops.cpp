@@ -574,20 +574,45 @@ at::Tensor stemFold(at::Tensor image) {
 // ---- autograd nodes ------------------------------------------------------------
 // LayerNorm and the loss as native nodes: one call from Python forward and none backward.  For
 // 777 x 4104 rows the kernels take 27 us of a pass that took 110 us with Python nodes.
+// Where the graph of a backward is itself wanted, it is made of torch's ops (the two functions below).
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
+
+// dx, dgamma, dbeta of LayerNorm, differentiable.
+std::tuple<at::Tensor, at::Tensor, at::Tensor> layerNormBackwardGraph(const at::Tensor& dy, const at::Tensor& x,
+                                                                      const at::Tensor& gamma, const at::Tensor& mean,
+                                                                      const at::Tensor& rstd) {
+  const at::Tensor g = dy.to(at::kFloat);
+  const auto [dx, dgamma, unused] = at::native_layer_norm_backward(g, x.to(at::kFloat), {x.size(-1)}, mean, rstd, gamma,
+                                                                   std::nullopt, {true, true, false});
+  return std::make_tuple(dx.to(x.scalar_type()), dgamma, g.reshape({-1, x.size(-1)}).sum(0));
+}
+
+// The gradient of the mean cross-entropy, differentiable; the logits stay as they are.
+at::Tensor crossEntropyBackwardGraph(const at::Tensor& logits, const at::Tensor& targets, const at::Tensor& upstream,
+                                     const at::Tensor& count) {
+  const at::Tensor counts = targets.ge(0).logical_and(targets.lt(logits.size(1))).unsqueeze(1);
+  const at::Tensor at = at::where(counts, targets.unsqueeze(1), at::zeros_like(targets).unsqueeze(1));
+  const at::Tensor p = at::softmax(logits.to(at::kFloat), 1);
+  const at::Tensor d = p - at::zeros_like(p).scatter_(1, at, 1.0);
+  const at::Tensor grad = at::where(counts, d * (upstream.to(at::kFloat) / count), at::zeros_like(p));
+  return grad.to(logits.scalar_type());
+}
 
 struct LayerNormNode : torch::autograd::Function<LayerNormNode> {
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& gamma, const at::Tensor& beta,
                             double eps, at::ScalarType out_dtype) {
-    const at::Tensor xc = x.contiguous();
-    auto [y, mean, rstd] = layerNormForward(xc, gamma, beta, eps, out_dtype);
-    ctx->save_for_backward({xc, gamma, mean, rstd});
+    auto [y, mean, rstd] = layerNormForward(x, gamma, beta, eps, out_dtype);
+    ctx->save_for_backward({x, gamma, mean, rstd});
     ctx->saved_data["out"] = static_cast<int64_t>(out_dtype);
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
+    if (at::GradMode::is_enabled()) {
+      auto [dx, dgamma, dbeta] = layerNormBackwardGraph(grads[0], saved[0], saved[1], saved[2], saved[3]);
+      return {dx, dgamma, dbeta, at::Tensor(), at::Tensor()};
+    }
     const at::Tensor dy = grads[0].to(static_cast<at::ScalarType>(ctx->saved_data["out"].toInt())).contiguous();
     auto [dx, dgamma, dbeta] = layerNormBackward(dy, saved[0], saved[1], saved[2], saved[3]);
     return {dx, dgamma, dbeta, at::Tensor(), at::Tensor()};
@@ -614,6 +639,11 @@ struct AddLayerNormNode : torch::autograd::Function<AddLayerNormNode> {
       const at::Tensor g = grads[0].defined() ? grads[0] : at::zeros_like(xnew);
       return {g, g.to(branch_dtype), at::zeros_like(gamma), at::zeros_like(gamma), at::Tensor(), at::Tensor()};
     }
+    if (at::GradMode::is_enabled()) {  // xnew, an output of this node, carries the graph of both addends
+      auto [dx, dgamma, dbeta] = layerNormBackwardGraph(grads[1], xnew, gamma, saved[2], saved[3]);
+      if (grads[0].defined()) dx = dx + grads[0];
+      return {dx, dx.to(branch_dtype), dgamma, dbeta, at::Tensor(), at::Tensor()};
+    }
     const at::Tensor dy = grads[1].to(static_cast<at::ScalarType>(ctx->saved_data["out"].toInt())).contiguous();
     std::optional<at::Tensor> gres;
     if (grads[0].defined()) gres = grads[0].to(at::kFloat).contiguous();
@@ -638,11 +668,8 @@ struct CrossEntropyNode : torch::autograd::Function<CrossEntropyNode> {
     const auto saved = ctx->get_saved_variables();
     const at::Tensor &logits = saved[0], &targets = saved[1];
     const bool keep = ctx->saved_data["keep"].toBool();
-    if (keep && at::GradMode::is_enabled()) {  // the graph of this backward is wanted: torch's own ops have one
-      const at::Tensor t = at::where(targets.ge(0), targets, at::full_like(targets, -100));
-      const at::Tensor loss = at::cross_entropy_loss(logits.to(at::kFloat), t);
-      return {torch::autograd::grad({loss}, {logits}, {grads[0]}, std::nullopt, true)[0], at::Tensor(), at::Tensor()};
-    }
+    if (at::GradMode::is_enabled())
+      return {crossEntropyBackwardGraph(logits, targets, grads[0], saved[3]), at::Tensor(), at::Tensor()};
     const at::Tensor grad = keep ? at::empty_like(logits) : logits.detach();
     crossEntropyBackward(grad, logits, targets, saved[2], grads[0].to(at::kFloat).reshape({1}), 1.0, saved[3]);
     return {grad, at::Tensor(), at::Tensor()};
@@ -651,7 +678,7 @@ struct CrossEntropyNode : torch::autograd::Function<CrossEntropyNode> {
 
 at::Tensor layerNorm(const at::Tensor& x, const at::Tensor& gamma, const at::Tensor& beta, double eps,
                      at::ScalarType out_dtype) {
-  return LayerNormNode::apply(x, gamma, beta, eps, out_dtype);
+  return LayerNormNode::apply(x.contiguous(), gamma, beta, eps, out_dtype);
 }
 std::tuple<at::Tensor, at::Tensor> addLayerNorm(const at::Tensor& x, const at::Tensor& branch, const at::Tensor& gamma,
                                                 const at::Tensor& beta, double eps, at::ScalarType out_dtype) {
@@ -678,6 +705,10 @@ void bindLocalOps(pybind11::module_& m) {
   m.def("add_layer_norm", &addLayerNorm, py::arg("x"), py::arg("branch"), py::arg("weight"), py::arg("bias"),
         py::arg("eps"), py::arg("out_dtype"));
   m.def("cross_entropy", &crossEntropy, py::arg("logits"), py::arg("targets"), py::arg("keep"));
+  m.def("layer_norm_bwd_graph", &layerNormBackwardGraph, py::arg("dy"), py::arg("x"), py::arg("weight"),
+        py::arg("mean"), py::arg("rstd"));
+  m.def("cross_entropy_bwd_graph", &crossEntropyBackwardGraph, py::arg("logits"), py::arg("targets"),
+        py::arg("upstream"), py::arg("count"));
   m.def("sumsq", &sumSq, py::arg("x"), py::arg("root") = false);
   m.def("cross_entropy_fwd", &crossEntropyForward, py::arg("logits"), py::arg("targets"),
         py::arg("bad_target") = 0.0);

@@ -31,6 +31,8 @@ class _FusedCrossEntropyFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         logits, targets, lse, count = ctx.saved_tensors
+        if torch.is_grad_enabled():  # the graph of this backward is wanted
+            return _C.cross_entropy_bwd_graph(logits, targets, g, count), None
         grad = logits.detach()
         _C.cross_entropy_bwd_(grad, targets, lse, g.float().reshape(1), 1.0, count)
         return grad, None
@@ -39,7 +41,8 @@ class _FusedCrossEntropyFn(torch.autograd.Function):
 def fused_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
     """Mean cross-entropy of ``logits`` [rows, vocab] (fp32 or bf16) against
     ``targets`` [rows] (negative entries are ignored).  Consumes the logits when the
-    vocabulary is a multiple of 8: after backward their storage holds the gradient.
+    vocabulary is a multiple of 8: after backward their storage holds the gradient (unless the
+    backward's own graph was asked for).
     Falls back to ``F.cross_entropy(logits.float(), targets)`` off the GPU and for
     what the kernels do not take."""
     ok = (logits.is_cuda and logits.dim() == 2 and logits.is_contiguous()

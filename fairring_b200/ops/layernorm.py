@@ -26,15 +26,16 @@ from ._plain import FUSE_FROM, native, plain_autograd, plain_module
 class _FusedLayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, eps, out_dtype):
-        xc = x.contiguous()
-        y, mean, rstd = _C.layer_norm_fwd(xc, weight, bias, eps, out_dtype)
-        ctx.save_for_backward(xc, weight, mean, rstd)
+        y, mean, rstd = _C.layer_norm_fwd(x, weight, bias, eps, out_dtype)
+        ctx.save_for_backward(x, weight, mean, rstd)
         ctx.out_dtype = out_dtype
         return y
 
     @staticmethod
     def backward(ctx, dy):
         x, weight, mean, rstd = ctx.saved_tensors
+        if torch.is_grad_enabled():  # the graph of this backward is wanted
+            return *_C.layer_norm_bwd_graph(dy, x, weight, mean, rstd), None, None
         if dy.dtype != ctx.out_dtype:
             dy = dy.to(ctx.out_dtype)
         dx, dgamma, dbeta = _C.layer_norm_bwd(dy.contiguous(), x, weight, mean, rstd)
@@ -47,7 +48,9 @@ def fused_layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, 
     dtype inside an autocast region and to ``x.dtype`` otherwise."""
     if out_dtype is None:
         out_dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
-    return (_C.layer_norm if plain_autograd() else _FusedLayerNormFn.apply)(x, weight, bias, eps, out_dtype)
+    if plain_autograd():
+        return _C.layer_norm(x, weight, bias, eps, out_dtype)
+    return _FusedLayerNormFn.apply(x.contiguous(), weight, bias, eps, out_dtype)
 
 
 class FusedLayerNorm(nn.LayerNorm):
@@ -87,6 +90,10 @@ class _AddLayerNormFn(torch.autograd.Function):
         if dy is None:  # the normalised output was not used: only the residual path carries gradient
             g = g_xnew if g_xnew is not None else torch.zeros_like(xnew)
             return g, g.to(ctx.branch_dtype), torch.zeros_like(weight), torch.zeros_like(weight), None, None
+        if torch.is_grad_enabled():  # the graph of this backward is wanted
+            dx, dgamma, dbeta = _C.layer_norm_bwd_graph(dy, xnew, weight, mean, rstd)
+            dx = dx if g_xnew is None else dx + g_xnew
+            return dx, dx.to(ctx.branch_dtype), dgamma, dbeta, None, None
         if dy.dtype != ctx.out_dtype:
             dy = dy.to(ctx.out_dtype)
         gres = None if g_xnew is None else g_xnew.float().contiguous()

@@ -105,3 +105,31 @@ def test_no_counted_row_and_second_derivative():
         (g,) = torch.autograd.grad(f(x, t), x, create_graph=True)
         got.append(torch.autograd.grad((g ** 2).sum(), x)[0])
     torch.testing.assert_close(got[0], got[1], rtol=1e-4, atol=1e-6)
+
+
+# the vocabulary of the gradient over the logits, and one that keeps them
+@pytest.mark.parametrize("vocab", [16, 17])
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_second_derivative_and_the_logits_behind_it(vocab, native, dtype, monkeypatch):
+    _need_gpu()
+    import sys
+
+    from fairring_b200.ops import fused_cross_entropy
+
+    if not native:
+        monkeypatch.setattr(sys.modules[fused_cross_entropy.__module__], "plain_autograd", lambda: False)
+    leaf = torch.randn(5, vocab, device="cuda", generator=torch.Generator(device="cuda").manual_seed(vocab)).to(dtype)
+    t = torch.tensor([1, -100, 0, vocab - 1, 2], device="cuda")
+    got = []
+    for f in (fused_cross_entropy, lambda a, b: F.cross_entropy(a.float(), b)):
+        x = leaf.clone().requires_grad_(True)
+        logits = x * 1.0
+        before = logits.detach().clone()
+        loss = f(logits, t)
+        (g,) = torch.autograd.grad(loss * loss, x, create_graph=True)
+        assert g.requires_grad and torch.equal(logits, before)
+        got.append([g, torch.autograd.grad((g.float() ** 2).sum(), x)[0]])
+    rtol = 2.0 ** -6 if dtype == torch.bfloat16 else 1e-4  # two to three roundings on the way
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, rtol=rtol, atol=rtol * float(b.detach().abs().max()))

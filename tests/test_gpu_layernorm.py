@@ -45,3 +45,39 @@ def test_rows_off_a_16_byte_boundary():
     x = torch.randn(5 * 64 + 1, device="cuda")[1:].view(5, 64)
     w, b = torch.ones(65, device="cuda")[1:], torch.zeros(65, device="cuda")[1:]
     torch.testing.assert_close(fused_layer_norm(x, w, b), F.layer_norm(x, (64,)), rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("kind", ["norm", "transposed", "bf16", "residual", "residual bf16"])
+def test_second_derivative(kind, native, monkeypatch):
+    _need_gpu()
+    import sys
+
+    from fairring_b200.ops import FusedLayerNorm, add_layer_norm
+
+    if not native:
+        monkeypatch.setattr(sys.modules[FusedLayerNorm.__module__], "plain_autograd", lambda: False)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    x0, br0 = torch.randn(24, 24, device="cuda", generator=gen), torch.randn(24, 24, device="cuda", generator=gen)
+    low = kind.endswith("bf16")
+    if low:
+        br0 = br0.bfloat16()
+        x0 = x0.bfloat16() if kind == "bf16" else x0
+    got = []
+    for fused in (True, False):
+        norm = (FusedLayerNorm if fused else torch.nn.LayerNorm)(24, device="cuda")
+        x, br = x0.clone().requires_grad_(True), br0.clone().requires_grad_(True)
+        if kind.startswith("residual"):
+            stream = x + br
+            stream, y = add_layer_norm(norm, x, br) if fused else (stream, norm(stream))
+            out, leaves = (y ** 3).sum() + (stream ** 3).sum(), [x, br, norm.weight, norm.bias]
+        else:
+            a = x.t() if kind == "transposed" else x
+            y = norm(a) if fused else F.layer_norm(a.float(), (24,), norm.weight, norm.bias).to(a.dtype)
+            out, leaves = (y.float() ** 3).sum(), [x, norm.weight, norm.bias]
+        first = torch.autograd.grad(out, leaves, create_graph=True)
+        assert all(g.requires_grad for g in first)
+        got.append([*first, *torch.autograd.grad(sum((g.float() ** 2).sum() for g in first), leaves)])
+    rtol = 2.0 ** -5 if low else 1e-3  # up to four roundings of the type on the way
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, rtol=rtol, atol=rtol * float(b.detach().abs().max()))
