@@ -14,7 +14,6 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
-from torch.autograd.function import once_differentiable
 
 from .. import _C
 from ._plain import FUSE_FROM, native, plain_autograd, plain_module
@@ -123,7 +122,8 @@ def add_layer_norm(norm: nn.LayerNorm, x: torch.Tensor, branch: torch.Tensor | N
 class _AddLayerNormPairFn(torch.autograd.Function):
     """LayerNorm(x + branch) in fp32 and in ``low``.  The forward is torch's LayerNorm: one that sums a
     row in another order is as exact, but through 24 post-LayerNorm layers in bf16 it moves the gradients
-    by 1.6 % at random weights.  The backward takes both gradients in one kernel."""
+    by 1.6 % at random weights.  The backward takes both gradients in one kernel.  The sum is an output
+    too, for the graph of the backward alone: through it that graph reaches both addends."""
 
     @staticmethod
     def forward(ctx, x, branch, weight, bias, eps, low):
@@ -133,18 +133,23 @@ class _AddLayerNormPairFn(torch.autograd.Function):
         ctx.save_for_backward(xnew, weight, mean.view(-1), rstd.view(-1))
         ctx.set_materialize_grads(False)  # an unused output arrives as None, not as zeros
         ctx.low, ctx.branch_dtype = low, branch.dtype
-        return y, y.to(low)
+        return y, y.to(low), xnew
 
     @staticmethod
-    @once_differentiable
-    def backward(ctx, dy, dy_low):
+    def backward(ctx, dy, dy_low, g_xnew):
         xnew, weight, mean, rstd = ctx.saved_tensors
         if dy is None and dy_low is None:
-            return None, None, None, None, None, None
+            return g_xnew, None if g_xnew is None else g_xnew.to(ctx.branch_dtype), None, None, None, None
+        if torch.is_grad_enabled():  # the graph of this backward is wanted
+            g = dy_low.float() if dy is None else dy if dy_low is None else dy + dy_low.float()
+            dx, dgamma, dbeta = _C.layer_norm_bwd_graph(g, xnew, weight, mean, rstd)
+            dx = dx if g_xnew is None else dx + g_xnew
+            return dx, dx.to(ctx.branch_dtype), dgamma, dbeta, None, None
+        g_xnew = None if g_xnew is None else g_xnew.float().contiguous()
         dy = None if dy is None else dy.float().contiguous()
         dy_low = None if dy_low is None else dy_low.to(ctx.low).contiguous()
         want_bf16 = ctx.branch_dtype == torch.bfloat16
-        dx, dbr, dgamma, dbeta = _C.add_layer_norm_bwd(dy_low, xnew, weight, mean, rstd, None, want_bf16, dy)
+        dx, dbr, dgamma, dbeta = _C.add_layer_norm_bwd(dy_low, xnew, weight, mean, rstd, g_xnew, want_bf16, dy)
         return dx, (dbr if want_bf16 else dx), dgamma, dbeta, None, None
 
 
@@ -165,6 +170,6 @@ def add_layer_norm_pair(norm: nn.LayerNorm, x: torch.Tensor, branch: torch.Tenso
             and branch.device == x.device and norm.normalized_shape == (d,) and d % 8 == 0
             and d <= 8192 and norm.weight is not None and norm.bias is not None
             and norm.weight.dtype == norm.bias.dtype == torch.float32 and norm.weight.device == x.device):
-        return _AddLayerNormPairFn.apply(x, branch, norm.weight, norm.bias, norm.eps, torch.bfloat16)
+        return _AddLayerNormPairFn.apply(x, branch, norm.weight, norm.bias, norm.eps, torch.bfloat16)[:2]
     y = norm(x + branch)
     return y, y

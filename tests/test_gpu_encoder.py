@@ -68,6 +68,35 @@ def test_a_mean_far_from_zero_keeps_the_variance(cols):
     assert float((y.double() - F.layer_norm(x.double(), (cols,))).abs().max()) < 2e-4
 
 
+@pytest.mark.parametrize("branch_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("use", ["both", "fp32", "low"])
+def test_pair_second_derivative(use, branch_dtype):
+    _need_gpu()
+    from fairring_b200.ops import add_layer_norm_pair
+
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    x0, br0 = torch.randn(12, 24, device="cuda", generator=gen), torch.randn(12, 24, device="cuda", generator=gen)
+    got = []
+    for fused in (True, False):
+        norm = nn.LayerNorm(24, device="cuda")
+        x, br = x0.clone().requires_grad_(True), br0.to(branch_dtype).requires_grad_(True)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            if fused:
+                y, low = add_layer_norm_pair(norm, x, br)
+                assert type(y.grad_fn).__name__ == "_AddLayerNormPairFnBackward"
+            else:
+                y = norm(x + br)
+                low = y.bfloat16()
+        out = (0.0 if use == "low" else (y ** 3).sum()) + (0.0 if use == "fp32" else (low.float() ** 3).sum())
+        leaves = [x, br, norm.weight, norm.bias]
+        first = torch.autograd.grad(out, leaves, create_graph=True)
+        assert all(g.requires_grad for g in first)
+        got.append([*first, *torch.autograd.grad(sum((g.float() ** 2).sum() for g in first), leaves)])
+    rtol = 2.0 ** -5 if branch_dtype == torch.bfloat16 or use != "fp32" else 1e-3  # up to four roundings to bf16
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, rtol=rtol, atol=rtol * float(b.detach().abs().max()))
+
+
 @pytest.mark.parametrize("vocab", [1000, 1001, 1007])
 @pytest.mark.parametrize("rows", [37, 0])
 def test_padded_head_matches_torch(vocab, rows):
