@@ -25,6 +25,11 @@ at::Tensor aligned16(const at::Tensor& t) {
   return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone();
 }
 
+// A sum over rows that a kernel will write, or zeros where there is no row and no launch.
+at::Tensor sumOfRows(int64_t rows, at::IntArrayRef sizes, const at::TensorOptions& options) {
+  return rows > 0 ? at::empty(sizes, options) : at::zeros(sizes, options);
+}
+
 // One AdamW step over flat buffers, in place.  `step` counts from 1.
 void adamwFlat(at::Tensor p, at::Tensor g, at::Tensor m, at::Tensor v, double lr, double beta1,
                double beta2, double eps, double weight_decay, int64_t step, double grad_scale,
@@ -133,8 +138,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> layerNormBackward(at::Tensor dy, 
   x = aligned16(x);
   gamma = aligned16(gamma);
   at::Tensor dx = at::empty_like(x);
-  at::Tensor dgamma = at::empty({cols}, gamma.options());
-  at::Tensor dbeta = at::empty({cols}, gamma.options());
+  at::Tensor dgamma = sumOfRows(rows, {cols}, gamma.options());
+  at::Tensor dbeta = sumOfRows(rows, {cols}, gamma.options());
   at::Tensor partial = at::empty({(int64_t)layerNormBackwardBlocks(rows, sms), 2, cols}, gamma.options());
   cudaError_t e = launchLayerNormBackward(
       dy.data_ptr(), dy.scalar_type() == at::kBFloat16, x.data_ptr(), x.scalar_type() == at::kBFloat16,
@@ -223,8 +228,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> addLayerNormBackward(
   at::Tensor dx = at::empty_like(xnew);
   at::Tensor dbr;
   if (want_bf16) dbr = at::empty(xnew.sizes(), xnew.options().dtype(at::kBFloat16));
-  at::Tensor dgamma = at::empty({cols}, gamma.options());
-  at::Tensor dbeta = at::empty({cols}, gamma.options());
+  at::Tensor dgamma = sumOfRows(rows, {cols}, gamma.options());
+  at::Tensor dbeta = sumOfRows(rows, {cols}, gamma.options());
   at::Tensor partial = at::empty({(int64_t)layerNormBackwardBlocks(rows, sms), 2, cols}, gamma.options());
   cudaError_t e = launchAddLayerNormBackward(
       d.defined() ? d.data_ptr() : nullptr, d.defined() && d.scalar_type() == at::kBFloat16,
@@ -545,7 +550,7 @@ std::tuple<at::Tensor, at::Tensor> embedBackward(std::optional<at::Tensor> dx, s
                   dx->is_contiguous() && dx->numel() == tokens.numel() * d && d % 8 == 0,
               "dx must be contiguous fp32 with one row per token");
   const at::Tensor g = aligned16(*dx);
-  at::Tensor dpos = tokens.size(1) < positions ? at::zeros({positions, d}, fopt) : at::empty({positions, d}, fopt);
+  at::Tensor dpos = sumOfRows(tokens.size(1) < positions ? 0 : tokens.numel(), {positions, d}, fopt);
   cudaError_t e = launchEmbedBackward(g.data_ptr<float>(), tokens.data_ptr<int64_t>(), dtable.data_ptr<float>(),
                                       dpos.data_ptr<float>(), (int)tokens.size(0), (int)tokens.size(1), vocab, (int)d, sms,
                                       stream);

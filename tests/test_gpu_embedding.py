@@ -79,6 +79,17 @@ def test_the_gradient_repeats_itself(d, batch, seq, mix):
         assert torch.equal(again[0], dtable) and torch.equal(again[1], dpos)
 
 
+def test_no_tokens():
+    _need_gpu()
+    from fairring_b200 import _C
+
+    junk = [torch.full((4, 8), 7.0, device="cuda") for _ in range(8)]  # what the allocator hands out next
+    del junk
+    dtable, dpos = _C.embed_bwd(torch.empty(0, 4, 8, device="cuda"), None, torch.empty(0, 4, dtype=torch.long, device="cuda"),
+                                5, 4, 8)
+    assert not dtable.any() and not dpos.any()
+
+
 def test_calls_the_modules_where_they_cannot_be_skipped():
     _need_gpu()
     from fairring_b200.ops import tied_embedding

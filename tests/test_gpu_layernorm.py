@@ -81,3 +81,26 @@ def test_second_derivative(kind, native, monkeypatch):
     rtol = 2.0 ** -5 if low else 1e-3  # up to four roundings of the type on the way
     for a, b in zip(*got):
         torch.testing.assert_close(a, b, rtol=rtol, atol=rtol * float(b.detach().abs().max()))
+
+
+@pytest.mark.parametrize("kind", ["norm", "residual", "pair"])
+def test_no_rows(kind):
+    """An empty batch gives parameter gradients of zero."""
+    _need_gpu()
+    from fairring_b200.ops import FusedLayerNorm, add_layer_norm
+
+    norm = FusedLayerNorm(2048, device="cuda")
+    x, br = (torch.empty(0, 2048, device="cuda", requires_grad=True) for _ in range(2))
+    junk = [torch.full((2048,), 7.0, device="cuda") for _ in range(8)]  # what the allocator hands out next
+    del junk
+    if kind == "pair":
+        from fairring_b200 import _C
+
+        d = torch.empty(0, 2048, device="cuda")
+        stat = torch.empty(0, device="cuda")
+        _, _, dw, db = _C.add_layer_norm_bwd(None, d, norm.weight.detach(), stat, stat, None, False, d)
+    else:
+        y = norm(x) if kind == "norm" else add_layer_norm(norm, x, br)[1]
+        dx, dw, db = torch.autograd.grad(y.sum(), [x, norm.weight, norm.bias])
+        assert dx.shape == x.shape
+    assert not dw.any() and not db.any()
