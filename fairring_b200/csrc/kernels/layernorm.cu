@@ -64,32 +64,85 @@ __device__ __forceinline__ float2 blockSum2(float a, float b, float2 (&halves)[2
   return s;
 }
 
+// Mean and variance of a row that the block holds in registers; every thread gets both.
+// Differences throughout, since E[x^2] - mean^2 cancels in a row whose mean is far from
+// zero: a warp sums its part relative to its first element, then squares relative to its
+// own mean, and the warps' results are merged relative to the first one's, behind one barrier.
+template <int ITER> struct RowMoments {
+  static constexpr int kWarps = kLnThreads / 32;
+  float2 part[2][kWarps];  // (mean, sum of squares) per warp, in two halves as above
+  float share[kWarps];     // its part of the row
+
+  // Columns of warp w.
+  static __device__ __forceinline__ int columns(int w, int cols) {
+    int n = 0;
+#pragma unroll
+    for (int it = 0; it < ITER; ++it) n += min(max(cols - (it * kLnThreads + w * 32) * 8, 0), 256);
+    return n;
+  }
+  // Before the first row, whose barrier makes it visible.
+  __device__ __forceinline__ void init(int cols) {
+    if (threadIdx.x < kWarps) share[threadIdx.x] = (float)columns(threadIdx.x, cols) / cols;
+  }
+  // `inv`: 1 / columns of this warp, 0 if it has none.
+  __device__ __forceinline__ float2 of(const float (&v)[ITER][8], int cols, float inv, int half) {
+    const float first = __shfl_sync(0xffffffffu, v[0][0], 0);
+    float s = 0.f, q = 0.f;
+#pragma unroll
+    for (int it = 0; it < ITER; ++it) {
+      if ((it * kLnThreads + (int)threadIdx.x) * 8 < cols) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s += v[it][i] - first;
+      }
+    }
+    const float own = fmaf(warpSum(s), inv, first);
+#pragma unroll
+    for (int it = 0; it < ITER; ++it) {
+      if ((it * kLnThreads + (int)threadIdx.x) * 8 < cols) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float d = v[it][i] - own;
+          q = fmaf(d, d, q);
+        }
+      }
+    }
+    q = warpSum(q);
+    if ((threadIdx.x & 31) == 0) part[half][threadIdx.x >> 5] = make_float2(own, q);
+    __syncthreads();
+    const float about = part[half][0].x;
+    float d = 0.f, between = 0.f, within = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float2 p = part[half][w];
+      const float e = p.x - about, f = share[w];
+      d = fmaf(f, e, d);
+      between = fmaf(f * e, e, between);
+      within += p.y;
+    }
+    const float var = within / cols + (between - d * d);
+    return make_float2(about + d, var < 0.f ? 0.f : var);  // NaN stays
+  }
+};
+
 template <typename TX, typename TY, int ITER>
 __global__ void __launch_bounds__(kLnThreads, ITER == 1 ? 8 : 1)
 layer_norm_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ gamma,
                       const float* __restrict__ beta, TY* __restrict__ y, float* __restrict__ mean_out,
                       float* __restrict__ rstd_out, int64_t rows, int cols, float eps) {
-  __shared__ float2 scratch[2][kLnThreads / 32];
+  __shared__ RowMoments<ITER> moments;
+  moments.init(cols);
+  const int own = moments.columns(threadIdx.x >> 5, cols);
+  const float inv = own > 0 ? 1.f / own : 0.f;
   int half = 0;
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, half ^= 1) {
-    float v[ITER][8];
-    float s = 0.f, ss = 0.f;
+    float v[ITER][8] = {};
 #pragma unroll
     for (int it = 0; it < ITER; ++it) {
       const int c = (it * kLnThreads + threadIdx.x) * 8;
-      if (c < cols) {
-        load8<TX>(x + r * cols + c, v[it]);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          s += v[it][i];
-          ss += v[it][i] * v[it][i];
-        }
-      }
+      if (c < cols) load8<TX>(x + r * cols + c, v[it]);
     }
-    const float2 t = blockSum2(s, ss, scratch, half);
-    const float mean = t.x / cols;
-    const float var = fmaxf(t.y / cols - mean * mean, 0.f);
-    const float rstd = rsqrtf(var + eps);
+    const float2 t = moments.of(v, cols, inv, half);
+    const float mean = t.x, rstd = rsqrtf(t.y + eps);
     if (threadIdx.x == 0) {
       mean_out[r] = mean;
       rstd_out[r] = rstd;
@@ -218,11 +271,13 @@ add_layer_norm_fwd_kernel(const float* __restrict__ x, const TB* __restrict__ br
                           const float* __restrict__ gamma, const float* __restrict__ beta,
                           float* __restrict__ xnew, TY* __restrict__ y, float* __restrict__ mean_out,
                           float* __restrict__ rstd_out, int64_t rows, int cols, float eps) {
-  __shared__ float2 scratch[2][kLnThreads / 32];
+  __shared__ RowMoments<ITER> moments;
+  moments.init(cols);
+  const int own = moments.columns(threadIdx.x >> 5, cols);
+  const float inv = own > 0 ? 1.f / own : 0.f;
   int half = 0;
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, half ^= 1) {
-    float v[ITER][8];
-    float s = 0.f, ss = 0.f;
+    float v[ITER][8] = {};
 #pragma unroll
     for (int it = 0; it < ITER; ++it) {
       const int c = (it * kLnThreads + threadIdx.x) * 8;
@@ -231,18 +286,12 @@ add_layer_norm_fwd_kernel(const float* __restrict__ x, const TB* __restrict__ br
         load8<float>(x + r * cols + c, v[it]);
         load8<TB>(branch + r * cols + c, b);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          v[it][i] += b[i];
-          s += v[it][i];
-          ss += v[it][i] * v[it][i];
-        }
+        for (int i = 0; i < 8; ++i) v[it][i] += b[i];
         store8<float>(xnew + r * cols + c, v[it]);
       }
     }
-    const float2 t = blockSum2(s, ss, scratch, half);
-    const float mean = t.x / cols;
-    const float var = fmaxf(t.y / cols - mean * mean, 0.f);
-    const float rstd = rsqrtf(var + eps);
+    const float2 t = moments.of(v, cols, inv, half);
+    const float mean = t.x, rstd = rsqrtf(t.y + eps);
     if (threadIdx.x == 0) {
       mean_out[r] = mean;
       rstd_out[r] = rstd;

@@ -104,3 +104,35 @@ def test_no_rows(kind):
         dx, dw, db = torch.autograd.grad(y.sum(), [x, norm.weight, norm.bias])
         assert dx.shape == x.shape
     assert not dw.any() and not db.any()
+
+
+# a warp's columns and part of another's, all warps', ragged second and third rounds
+@pytest.mark.parametrize("cols", [8, 264, 2048, 4104, 8192])
+@pytest.mark.parametrize("kind", ["norm", "residual"])
+@pytest.mark.parametrize("row", ["far", "outlier", "far and outlier", "constant"])
+def test_a_mean_far_from_zero_keeps_the_variance(cols, kind, row):
+    _need_gpu()
+    from fairring_b200.ops import FusedLayerNorm, add_layer_norm
+
+    gen = torch.Generator(device="cuda").manual_seed(cols)
+    x = torch.randn(64, cols, device="cuda", generator=gen)
+    if row == "constant":
+        x[:] = 1000.0
+    if row.startswith("far"):
+        x += 1000
+    if row.endswith("outlier"):
+        x[:, 0] += 500.0  # the element that the differences are taken from
+    norm = FusedLayerNorm(cols, device="cuda")
+    y = norm(x) if kind == "norm" else add_layer_norm(norm, x, torch.zeros_like(x))[1]
+    # the mean is known to a few of fp32's steps at 1000 (6e-5), everything else to a few of its own
+    assert float((y.double() - F.layer_norm(x.double(), (cols,))).abs().max()) < 2e-4
+
+
+def test_a_row_that_is_not_finite():
+    _need_gpu()
+    from fairring_b200.ops import FusedLayerNorm
+
+    norm = FusedLayerNorm(512, device="cuda")
+    x = torch.randn(6, 512, device="cuda")
+    x[0, 0], x[1, 300], x[2, 511], x[3, 0] = float("inf"), float("-inf"), float("nan"), float("nan")
+    assert torch.equal(norm(x).isnan().all(1), torch.tensor([1, 1, 1, 1, 0, 0], device="cuda", dtype=torch.bool))
