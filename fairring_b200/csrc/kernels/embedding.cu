@@ -12,6 +12,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cassert>
 #include <cstdint>
 
 #include "local_kernels.h"
@@ -25,16 +26,17 @@ __device__ __forceinline__ float4 operator+(const float4& a, const float4& b) {
   return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
 
-// One block per token and 4 x 256 columns.  A token outside the table gives a row of NaN.
+// One block per token and 4 x 256 columns.  A token outside the table ends the program, as it does
+// in torch's embedding; nothing is read for it.
 __global__ void __launch_bounds__(kEmbThreads)
 embed_fwd_kernel(const int64_t* __restrict__ tokens, const float4* __restrict__ table, const float4* __restrict__ pos,
                  float4* __restrict__ x, int seq, int64_t vocab, int d4) {
   const int c = blockIdx.y * kEmbThreads + threadIdx.x;
   if (c >= d4) return;
   const int64_t r = blockIdx.x, t = tokens[r];
-  const float nan = __int_as_float(0x7fffffff);
-  const float4 row = t >= 0 && t < vocab ? table[t * d4 + c] : make_float4(nan, nan, nan, nan);
-  x[r * d4 + c] = row + pos[(r % seq) * d4 + c];
+  const bool inside = t >= 0 && t < vocab;
+  assert(inside && "token outside the table");
+  if (inside) x[r * d4 + c] = table[t * d4 + c] + pos[(r % seq) * d4 + c];
 }
 
 // One block per position and 4 x 256 columns: the sum over the sequences.
