@@ -19,6 +19,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cassert>
 #include <cstdint>
 
 #include "local_kernels.h"
@@ -115,14 +116,15 @@ __device__ __forceinline__ float blockReduce(float v, bool is_max, float* scratc
 }
 
 // loss[r] = logsumexp(row r) - row r[target]; lse[r] kept for the backward.
-// A negative target marks a row that does not count: loss 0.  A target past the
-// vocabulary gives `bad_target`.  One block per row, one sweep over it: a thread
+// A negative target marks a row that does not count: loss 0, as for a target past the
+// vocabulary.  With `classes` > 0 a target that is neither below it nor -100 ends the program, as it
+// does in torch's loss.  One block per row, one sweep over it: a thread
 // rescales its sum once per batch of vectors when its maximum grew, and the next
 // batch is on its way while this one is used.
 template <typename T, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1280 / kThreads)
 cross_entropy_fwd_kernel(const T* __restrict__ logits, const int64_t* __restrict__ targets,
-                         float* __restrict__ loss, float* __restrict__ lse, int vocab, float bad_target) {
+                         float* __restrict__ loss, float* __restrict__ lse, int vocab, int classes) {
   constexpr int E = Vec16<T>::kElems, U = kCeBatch;
   __shared__ float scratch[kThreads / 32];
   const int64_t r = blockIdx.x;
@@ -169,7 +171,9 @@ cross_entropy_fwd_kernel(const T* __restrict__ logits, const int64_t* __restrict
     const float l = m + logf(s);
     lse[r] = l;
     const int64_t t = targets[r];
-    loss[r] = t < 0 ? 0.f : t < vocab ? l - toFloat(row[t]) : bad_target;
+    const bool counts = t >= 0 && t < vocab;
+    assert((classes == 0 || t == -100 || (t >= 0 && t < classes)) && "target outside the vocabulary");
+    loss[r] = counts ? l - toFloat(row[t]) : 0.f;
   }
 }
 
@@ -246,17 +250,17 @@ constexpr int kCeFwdWide = 256, kCeFwdNarrow = 128, kCeBwdThreads = 256;
 
 template <typename T>
 void forwardOf(const void* logits, const int64_t* targets, float* loss, float* lse, int64_t rows, int vocab,
-               float bad_target, cudaStream_t stream) {
+               int classes, cudaStream_t stream) {
   // A row that one batch of 256 threads would not fill takes 128.
   for (int64_t done = 0; done < rows; done += 1 << 30) {
     const unsigned n = (unsigned)(rows - done < (1 << 30) ? rows - done : (1 << 30));
     const T* at = static_cast<const T*>(logits) + done * vocab;
     if (vocab >= kCeFwdWide * kCeBatch * Vec16<T>::kElems)
       cross_entropy_fwd_kernel<T, kCeFwdWide><<<n, kCeFwdWide, 0, stream>>>(at, targets + done, loss + done, lse + done,
-                                                                           vocab, bad_target);
+                                                                           vocab, classes);
     else
       cross_entropy_fwd_kernel<T, kCeFwdNarrow><<<n, kCeFwdNarrow, 0, stream>>>(at, targets + done, loss + done,
-                                                                               lse + done, vocab, bad_target);
+                                                                               lse + done, vocab, classes);
     noteLocalLaunch();
   }
 }
@@ -276,13 +280,13 @@ void backwardOf(const void* logits, void* grad, const int64_t* targets, const fl
 }  // namespace
 
 cudaError_t launchCrossEntropyForward(const void* logits, bool bf16, const int64_t* targets, float* loss,
-                                      float* lse, int64_t rows, int vocab, float bad_target, cudaStream_t stream) {
+                                      float* lse, int64_t rows, int vocab, int classes, cudaStream_t stream) {
   if (rows <= 0) return cudaSuccess;
   if (vocab <= 0) return cudaErrorInvalidValue;
   if (bf16)
-    forwardOf<__nv_bfloat16>(logits, targets, loss, lse, rows, vocab, bad_target, stream);
+    forwardOf<__nv_bfloat16>(logits, targets, loss, lse, rows, vocab, classes, stream);
   else
-    forwardOf<float>(logits, targets, loss, lse, rows, vocab, bad_target, stream);
+    forwardOf<float>(logits, targets, loss, lse, rows, vocab, classes, stream);
   return cudaGetLastError();
 }
 

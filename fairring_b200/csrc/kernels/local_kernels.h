@@ -68,10 +68,10 @@ cudaError_t launchAddLayerNormBackward(const void* dy, bool y_bf16, const float*
 cudaError_t launchAddBranch(const float* x, const void* branch_bf16, float* out, int64_t n, cudaStream_t stream);
 
 // Softmax cross-entropy over [rows, vocab] logits (fp32 or bf16): per-row loss
-// and log-sum-exp; a negative target's row has loss 0, one past the vocabulary
-// has loss `bad_target`.
+// and log-sum-exp; the row of a target that is negative or past the vocabulary has
+// loss 0; with `classes` > 0 a target is an error unless it is below that or -100.
 cudaError_t launchCrossEntropyForward(const void* logits, bool bf16, const int64_t* targets, float* loss,
-                                      float* lse, int64_t rows, int vocab, float bad_target, cudaStream_t stream);
+                                      float* lse, int64_t rows, int vocab, int classes, cudaStream_t stream);
 // *mean = sum of `loss` / *count, *count = max(number of targets >= 0, least).
 cudaError_t launchCrossEntropyMean(const float* loss, const int64_t* targets, int64_t rows, float least,
                                    float* mean, float* count, cudaStream_t stream);

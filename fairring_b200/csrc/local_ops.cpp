@@ -6,7 +6,6 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
-#include <cmath>
 #include <optional>
 #include <tuple>
 
@@ -303,16 +302,17 @@ void checkLogits(const at::Tensor& logits, const at::Tensor& targets) {
 }
 
 // (per-row loss, per-row log-sum-exp) of logits [rows, vocab] against targets [rows];
-// a target past the vocabulary gives `bad_target`.
-std::tuple<at::Tensor, at::Tensor> crossEntropyForward(at::Tensor logits, at::Tensor targets, double bad_target) {
+// `classes`, if not 0: a target that is neither one of them nor -100 is an error.
+std::tuple<at::Tensor, at::Tensor> crossEntropyForward(at::Tensor logits, at::Tensor targets, int64_t classes) {
   checkLogits(logits, targets);
+  TORCH_CHECK(classes >= 0 && classes <= logits.size(1), "no more classes than logits");
   c10::cuda::CUDAGuard guard(logits.device());
   auto fopt = logits.options().dtype(at::kFloat);
   at::Tensor loss = at::empty({logits.size(0)}, fopt), lse = at::empty({logits.size(0)}, fopt);
   cudaError_t e = launchCrossEntropyForward(logits.data_ptr(), logits.scalar_type() == at::kBFloat16,
                                             targets.data_ptr<int64_t>(), loss.data_ptr<float>(),
                                             lse.data_ptr<float>(), logits.size(0), (int)logits.size(1),
-                                            (float)bad_target, c10::cuda::getCurrentCUDAStream());
+                                            (int)classes, c10::cuda::getCurrentCUDAStream());
   TORCH_CHECK(e == cudaSuccess, "cross_entropy forward launch failed: ", cudaGetErrorString(e));
   return std::make_tuple(loss, lse);
 }
@@ -659,11 +659,12 @@ struct AddLayerNormNode : torch::autograd::Function<AddLayerNormNode> {
   }
 };
 
-// Mean cross-entropy.  `keep`: as torch's own loss -- the logits stay as they are, no counted row gives
-// NaN, and so does a target past the vocabulary; otherwise the gradient is written over the logits.
+// Mean cross-entropy.  `classes` > 0: as torch's own loss -- the logits stay as they are (they may be more
+// than the classes), no counted row gives NaN, a target that is no class is an error unless it is -100; otherwise the gradient is written over the logits.
 struct CrossEntropyNode : torch::autograd::Function<CrossEntropyNode> {
-  static at::Tensor forward(AutogradContext* ctx, const at::Tensor& logits, const at::Tensor& targets, bool keep) {
-    auto [losses, lse] = crossEntropyForward(logits, targets, keep ? std::nan("") : 0.0);
+  static at::Tensor forward(AutogradContext* ctx, const at::Tensor& logits, const at::Tensor& targets, int64_t classes) {
+    const bool keep = classes > 0;
+    auto [losses, lse] = crossEntropyForward(logits, targets, classes);
     auto [mean, count] = crossEntropyMean(losses, targets, keep ? 0.0 : 1.0);
     ctx->save_for_backward({logits, targets, lse, count});
     ctx->saved_data["keep"] = keep;
@@ -690,8 +691,8 @@ std::tuple<at::Tensor, at::Tensor> addLayerNorm(const at::Tensor& x, const at::T
   auto out = AddLayerNormNode::apply(x, branch, gamma, beta, eps, out_dtype);
   return std::make_tuple(out[0], out[1]);
 }
-at::Tensor crossEntropy(const at::Tensor& logits, const at::Tensor& targets, bool keep) {
-  return CrossEntropyNode::apply(logits, targets, keep);
+at::Tensor crossEntropy(const at::Tensor& logits, const at::Tensor& targets, int64_t classes) {
+  return CrossEntropyNode::apply(logits, targets, classes);
 }
 }  // namespace
 
@@ -709,14 +710,14 @@ void bindLocalOps(pybind11::module_& m) {
         py::arg("out_dtype"));
   m.def("add_layer_norm", &addLayerNorm, py::arg("x"), py::arg("branch"), py::arg("weight"), py::arg("bias"),
         py::arg("eps"), py::arg("out_dtype"));
-  m.def("cross_entropy", &crossEntropy, py::arg("logits"), py::arg("targets"), py::arg("keep"));
+  m.def("cross_entropy", &crossEntropy, py::arg("logits"), py::arg("targets"), py::arg("classes") = 0);
   m.def("layer_norm_bwd_graph", &layerNormBackwardGraph, py::arg("dy"), py::arg("x"), py::arg("weight"),
         py::arg("mean"), py::arg("rstd"));
   m.def("cross_entropy_bwd_graph", &crossEntropyBackwardGraph, py::arg("logits"), py::arg("targets"),
         py::arg("upstream"), py::arg("count"));
   m.def("sumsq", &sumSq, py::arg("x"), py::arg("root") = false);
   m.def("cross_entropy_fwd", &crossEntropyForward, py::arg("logits"), py::arg("targets"),
-        py::arg("bad_target") = 0.0);
+        py::arg("classes") = 0);
   m.def("cross_entropy_mean", &crossEntropyMean, py::arg("losses"), py::arg("targets"), py::arg("least"));
   m.def("cross_entropy_bwd", &crossEntropyBackward, py::arg("grad"), py::arg("logits"), py::arg("targets"),
         py::arg("lse"), py::arg("upstream"), py::arg("scale"), py::arg("count") = py::none());

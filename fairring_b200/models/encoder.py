@@ -121,7 +121,7 @@ class EncoderMLM(nn.Module):
         h = low.reshape(b * s, -1)[sel]
         h = self.head_ln(linear_gelu(self.head_dense, h))
         logits = vocab_logits(h, table, self.head_bias)
-        return cross_entropy_keeping_logits(logits, labels.reshape(-1)[sel])
+        return cross_entropy_keeping_logits(logits, labels.reshape(-1)[sel], self.head_bias.shape[0])
 
 
 def mask_tokens(tokens: torch.Tensor, cfg: EncoderConfig, generator: torch.Generator, mask_id: int = 0):

@@ -40,7 +40,8 @@ class _FusedCrossEntropyFn(torch.autograd.Function):
 
 def fused_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
     """Mean cross-entropy of ``logits`` [rows, vocab] (fp32 or bf16) against
-    ``targets`` [rows] (negative entries are ignored).  Consumes the logits when the
+    ``targets`` [rows] (-100 is ignored; so is every other negative entry when the vocabulary is a
+    multiple of 8, while with any other one it is an error as in ``F.cross_entropy``).  Consumes the logits when the
     vocabulary is a multiple of 8: after backward their storage holds the gradient (unless the
     backward's own graph was asked for).
     Falls back to ``F.cross_entropy(logits.float(), targets)`` off the GPU and for
@@ -49,16 +50,17 @@ def fused_cross_entropy(logits: torch.Tensor, targets: torch.Tensor) -> torch.Te
           and logits.dtype in (torch.float32, torch.bfloat16) and targets.dtype == torch.long)
     if ok and logits.shape[1] % 8 == 0:
         targets = targets.contiguous()
-        return _C.cross_entropy(logits, targets, False) if plain_autograd() else _FusedCrossEntropyFn.apply(logits, targets)
+        return _C.cross_entropy(logits, targets) if plain_autograd() else _FusedCrossEntropyFn.apply(logits, targets)
     return cross_entropy_keeping_logits(logits, targets)
 
 
-def cross_entropy_keeping_logits(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
-    """``F.cross_entropy(logits.float(), targets)`` (negative targets are ignored) by the same kernels;
-    the logits stay as they are whatever the vocabulary."""
+def cross_entropy_keeping_logits(logits: torch.Tensor, targets: torch.Tensor, classes: int | None = None) -> torch.Tensor:
+    """``F.cross_entropy(logits.float(), targets)`` by the same kernels; the logits stay as they are whatever
+    the vocabulary.  With ``classes`` the logits from there on are padding."""
     if (native(logits) and logits.dim() == 2 and logits.is_contiguous() and logits.shape[1] > 0
             and logits.dtype in (torch.float32, torch.bfloat16) and logits.data_ptr() % 16 == 0
             and targets.dtype == torch.long and targets.shape == logits.shape[:1]
             and targets.device == logits.device):
-        return _C.cross_entropy(logits, targets.contiguous(), True)
+        return _C.cross_entropy(logits, targets.contiguous(), logits.shape[1] if classes is None else classes)
+    logits = logits if classes is None else logits[:, :classes]
     return F.cross_entropy(logits.float(), targets, ignore_index=-100)

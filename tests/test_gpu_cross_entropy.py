@@ -133,3 +133,24 @@ def test_second_derivative_and_the_logits_behind_it(vocab, native, dtype, monkey
     rtol = 2.0 ** -6 if dtype == torch.bfloat16 else 1e-4  # two to three roundings on the way
     for a, b in zip(*got):
         torch.testing.assert_close(a, b, rtol=rtol, atol=rtol * float(b.detach().abs().max()))
+
+
+def test_padding_behind_the_classes():
+    """Targets at the edges of what is allowed; one outside would fail an assertion on the GPU."""
+    _need_gpu()
+    from fairring_b200 import _C
+    from fairring_b200.ops import cross_entropy_keeping_logits
+
+    base = torch.randn(4, 24, device="cuda")
+    base[:, 19:] = float("-inf")
+    targets = torch.tensor([0, 18, -100, 7], device="cuda")
+    x = base.clone().requires_grad_(True)
+    loss = cross_entropy_keeping_logits(x, targets, 19)
+    ref = base[:, :19].double().requires_grad_(True)
+    want = F.cross_entropy(ref, targets)
+    assert abs(float(loss) - float(want)) < 1e-5
+    (g,) = torch.autograd.grad(loss, x)
+    assert not g[:, 19:].any()
+    torch.testing.assert_close(g[:, :19].double(), torch.autograd.grad(want, ref)[0], rtol=1e-5, atol=1e-6)
+    with pytest.raises(RuntimeError):
+        _C.cross_entropy(base, targets, 25)
