@@ -34,6 +34,12 @@ __device__ __forceinline__ float toFloat(__nv_bfloat16 v) { return __bfloat162fl
 __device__ __forceinline__ void fromFloat(float* p, float v) { *p = v; }
 __device__ __forceinline__ void fromFloat(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
+// exp() of a difference of logits.  The fast form's relative error grows with the argument (2 + 1.17 |x|
+// units in the last place of fp32): far below bf16's rounding, but not below that of fp32 results.
+template <typename T> __device__ __forceinline__ float expOf(float v);
+template <> __device__ __forceinline__ float expOf<float>(float v) { return expf(v); }
+template <> __device__ __forceinline__ float expOf<__nv_bfloat16>(float v) { return __expf(v); }
+
 template <typename T> struct Vec16;
 template <> struct Vec16<float> {
   static constexpr int kElems = 4;
@@ -89,13 +95,13 @@ template <typename T> struct RowParts {
 };
 
 // A running maximum and the sum of exp(value - maximum) below it.
-struct SoftSum {
+template <typename T> struct SoftSum {
   float m = -INFINITY, s = 0.f;
   // What exp() is taken relative to: never -inf, whose difference from itself is NaN.
   static __device__ __forceinline__ float reference(float m) { return m == -INFINITY ? 0.f : m; }
   __device__ __forceinline__ void add(float v) {
     const float m_new = fmaxf(m, v), ref = reference(m_new);
-    s = s * __expf(m - ref) + __expf(v - ref);
+    s = s * expOf<T>(m - ref) + expOf<T>(v - ref);
     m = m_new;
   }
 };
@@ -131,7 +137,7 @@ cross_entropy_fwd_kernel(const T* __restrict__ logits, const int64_t* __restrict
   const T* row = logits + r * vocab;
   const RowParts<T> parts(row, vocab);
   const uint4* vecs = reinterpret_cast<const uint4*>(row + parts.head);
-  SoftSum a;
+  SoftSum<T> a;
   uint4 raw[U];
   auto fetch = [&](int i) {
 #pragma unroll
@@ -151,22 +157,22 @@ cross_entropy_fwd_kernel(const T* __restrict__ logits, const int64_t* __restrict
     float top = a.m;
 #pragma unroll
     for (int u = 0; u < U; ++u) top = fmaxf(top, Vec16<T>::max(now[u]));
-    const float ref = SoftSum::reference(top);
+    const float ref = SoftSum<T>::reference(top);
     float s[2] = {};
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       float v[E];
       Vec16<T>::get(now[u], v);
 #pragma unroll
-      for (int k = 0; k < E; ++k) s[k & 1] += __expf(v[k] - ref);
+      for (int k = 0; k < E; ++k) s[k & 1] += expOf<T>(v[k] - ref);
     }
-    a.s = a.s * __expf(a.m - ref) + (s[0] + s[1]);
+    a.s = a.s * expOf<T>(a.m - ref) + (s[0] + s[1]);
     a.m = top;
   }
   if ((int)threadIdx.x < parts.head) a.add(toFloat(row[threadIdx.x]));
   if ((int)threadIdx.x < parts.tail) a.add(toFloat(row[vocab - parts.tail + threadIdx.x]));
   const float m = blockReduce<kThreads>(a.m, true, scratch);
-  const float s = blockReduce<kThreads>(a.s * __expf(a.m - SoftSum::reference(m)), false, scratch);
+  const float s = blockReduce<kThreads>(a.s * expOf<T>(a.m - SoftSum<T>::reference(m)), false, scratch);
   if (threadIdx.x == 0) {
     const float l = m + logf(s);
     lse[r] = l;
@@ -225,7 +231,7 @@ cross_entropy_bwd_kernel(const T* logits, T* grad, const int64_t* __restrict__ t
     const bool counts = t64 >= 0 && t64 < vocab;
     const int t = counts ? (int)t64 : -1;
     const float l = lse[r];
-    auto one = [&](float v, int j) { return counts ? (__expf(v - l) - (j == t ? 1.f : 0.f)) * g : 0.f; };
+    auto one = [&](float v, int j) { return counts ? (expOf<T>(v - l) - (j == t ? 1.f : 0.f)) * g : 0.f; };
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = first + u * kThreads;

@@ -135,6 +135,28 @@ def test_second_derivative_and_the_logits_behind_it(vocab, native, dtype, monkey
         torch.testing.assert_close(a, b, rtol=rtol, atol=rtol * float(b.detach().abs().max()))
 
 
+@pytest.mark.parametrize("vocab", [1000, 1001, 50257])
+def test_fp32_gradients_are_as_exact_as_torch(vocab):
+    """Logits as a trained head has them, far apart: exp() of differences down to -40."""
+    _need_gpu()
+    from fairring_b200.ops import fused_cross_entropy
+
+    gen = torch.Generator(device="cuda").manual_seed(vocab)
+    x = torch.randn(512, vocab, device="cuda", generator=gen) * 5
+    t = torch.randint(0, vocab, (512,), device="cuda", generator=gen)
+    ref = x.double().requires_grad_(True)
+    want = F.cross_entropy(ref, t)
+    (wg,) = torch.autograd.grad(want, ref)
+    wg.scatter_(1, t[:, None], 0.0)  # the probabilities alone: the target's entry is 1 minus one
+    error = []
+    for f in (fused_cross_entropy, F.cross_entropy):
+        leaf = x.clone().requires_grad_(True)
+        (g,) = torch.autograd.grad(f(leaf * 1.0, t), leaf)
+        error.append(float((g.double().scatter_(1, t[:, None], 0.0) - wg).norm() / wg.norm()))
+    # both round the argument of exp() and its result; torch's own sum and logarithm may fall on either side
+    assert error[0] <= 1.2 * error[1] + 2.0 ** -24, error
+
+
 def test_padding_behind_the_classes():
     """Targets at the edges of what is allowed; one outside would fail an assertion on the GPU."""
     _need_gpu()
