@@ -24,7 +24,7 @@ class _BatchNormActFn(torch.autograd.Function):
                                           eps, relu)
         torch.autograd.graph.increment_version(tracked)  # as torch's own layer does, which adds 1 in place
         ctx.relu, ctx.eps, ctx.has_residual = relu, eps, residual is not None
-        ctx.save_for_backward(x, weight, bias, mean, rstd, residual, y if relu and residual is not None else None)
+        ctx.save_for_backward(x, weight, bias, mean, rstd, y if relu and residual is not None else None)
         if not twice:
             return y
         ctx.set_materialize_grads(False)  # an unused output arrives as None, not as zeros
@@ -36,18 +36,17 @@ class _BatchNormActFn(torch.autograd.Function):
             dy, dy2 = dy2, None
         if dy is None:
             return (None,) * 11
-        x, weight, bias, mean, rstd, residual, y = ctx.saved_tensors
+        x, weight, bias, mean, rstd, y = ctx.saved_tensors
         if torch.is_grad_enabled():  # the graph of this backward is wanted: torch's own ops have one
-            inputs = (x, weight, bias) if residual is None else (x, weight, bias, residual)
-            wanted = [t for t in inputs if t.requires_grad]
-            with torch.enable_grad():
-                dy = dy if dy2 is None else dy + dy2
-                out = F.batch_norm(x, None, None, weight, bias, True, 0.0, ctx.eps)
-                out = out if residual is None else out + residual
-                out = F.relu(out) if ctx.relu else out
-                grads = iter(torch.autograd.grad(out, wanted, dy, create_graph=True))
-            got = [next(grads) if t.requires_grad else None for t in inputs] + [None]
-            return got[0], got[3], got[1], got[2], None, None, None, None, None, None, None
+            dy = dy if dy2 is None else dy + dy2
+            out = F.batch_norm(x, None, None, weight, bias, True, 0.0, ctx.eps)
+            if ctx.relu:
+                dy = torch.where((out if y is None else y).detach() <= 0, torch.zeros_like(dy), dy)
+            inputs = (x, weight, bias)
+            grads = iter(torch.autograd.grad(out, [t for t in inputs if t.requires_grad], dy, create_graph=True)
+                         if any(t.requires_grad for t in inputs) else ())
+            dx, dgamma, dbeta = (next(grads) if t.requires_grad else None for t in inputs)
+            return dx, dy if ctx.has_residual else None, dgamma, dbeta, None, None, None, None, None, None, None
         dy = dy.contiguous(memory_format=torch.channels_last)
         if dy2 is not None:
             dy2 = dy2.contiguous(memory_format=torch.channels_last)

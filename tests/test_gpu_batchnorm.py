@@ -127,6 +127,48 @@ def test_second_derivative():
     torch.testing.assert_close(got[0], got[1], rtol=1e-3, atol=1e-4 * float(got[1].abs().max()))
 
 
+@pytest.mark.parametrize("residual", ["none", "other", "same"])
+@pytest.mark.parametrize("relu", [True, False])
+@pytest.mark.parametrize("twice", [True, False])
+def test_second_derivative_with_all_that_follows(residual, relu, twice):
+    """`same`: the input itself as the residual, whose gradient must not be counted twice."""
+    _need_gpu()
+    from fairring_b200.ops import batch_norm_act
+
+    torch.manual_seed(1)
+    x0, r0 = (torch.randn(3, 8, 4, 4, device="cuda").contiguous(memory_format=torch.channels_last) for _ in range(2))
+    act, got = nn.ReLU() if relu else None, []
+    for fused in (True, False):
+        x, r = (t.clone(memory_format=torch.channels_last).requires_grad_(True) for t in (x0, r0))
+        bn = nn.BatchNorm2d(8, device="cuda")
+        a = x * 1.0
+        res = {"none": None, "other": r * 1.0, "same": a}[residual]
+        if fused:
+            y, y2 = batch_norm_act(bn, a, res, act, twice=True) if twice else (batch_norm_act(bn, a, res, act),) * 2
+        else:
+            z = bn(a) if res is None else bn(a) + res
+            y = y2 = act(z) if relu else z
+        leaves = [x, bn.weight, bn.bias] + ([r] if residual == "other" else [])
+        first = torch.autograd.grad((y ** 3).sum() + (y2 ** 2).sum(), leaves, create_graph=True)
+        got.append([*first, *torch.autograd.grad(sum((g ** 2).sum() for g in first), leaves)])
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, rtol=1e-3, atol=1e-4 * float(b.detach().abs().max()))
+
+
+def test_the_residual_is_not_kept():
+    _need_gpu()
+    import weakref
+
+    from fairring_b200.ops import batch_norm_act
+
+    x = torch.randn(4, 16, 6, 6, device="cuda").contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    res = x.detach().clone(memory_format=torch.channels_last)
+    y = batch_norm_act(nn.BatchNorm2d(16, device="cuda"), x, res, nn.ReLU())
+    gone = weakref.ref(res)
+    del res
+    assert gone() is None and y.requires_grad
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("residual,relu", [(True, True), (False, True), (True, False)])
 @pytest.mark.parametrize("use", ["both", "first", "second"])
