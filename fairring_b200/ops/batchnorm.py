@@ -47,7 +47,9 @@ class _BatchNormActFn(torch.autograd.Function):
                          if any(t.requires_grad for t in inputs) else ())
             dx, dgamma, dbeta = (next(grads) if t.requires_grad else None for t in inputs)
             return dx, dy if ctx.has_residual else None, dgamma, dbeta, None, None, None, None, None, None, None
-        dy = dy.contiguous(memory_format=torch.channels_last)
+        # Saved-tensor hooks may have brought x and y back in another layout (save_on_cpu with pinned memory).
+        x, dy = (t.contiguous(memory_format=torch.channels_last) for t in (x, dy))
+        y = None if y is None else y.contiguous(memory_format=torch.channels_last)
         if dy2 is not None:
             dy2 = dy2.contiguous(memory_format=torch.channels_last)
             if y is None:

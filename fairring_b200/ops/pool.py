@@ -25,7 +25,8 @@ class _MaxPoolFn(torch.autograd.Function):
         if torch.is_grad_enabled():  # the graph of this backward is wanted: torch's own op has one
             with torch.enable_grad():
                 return torch.autograd.grad(F.max_pool2d(x, *ctx.geometry), x, dy, create_graph=True)[0], None, None, None
-        dy = dy.contiguous(memory_format=torch.channels_last)
+        # Saved-tensor hooks may have brought x back in another layout (save_on_cpu with pinned memory).
+        x, dy = (t.contiguous(memory_format=torch.channels_last) for t in (x, dy))
         return _C.max_pool_bwd(dy, x, chosen, *ctx.geometry), None, None, None
 
 

@@ -155,6 +155,22 @@ def test_second_derivative_with_all_that_follows(residual, relu, twice):
         torch.testing.assert_close(a, b, rtol=1e-3, atol=1e-4 * float(b.detach().abs().max()))
 
 
+@pytest.mark.parametrize("pin", [False, True])
+def test_saved_tensors_that_come_back_in_another_layout(pin):
+    _need_gpu()
+    from fairring_b200.ops import batch_norm_act
+
+    x0, r0, dy = (torch.randn(3, 16, 5, 7, device="cuda").contiguous(memory_format=torch.channels_last) for _ in range(3))
+    bn, got = nn.BatchNorm2d(16, device="cuda"), []
+    for hooks in (torch.autograd.graph.save_on_cpu(pin_memory=pin), torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t)):
+        x, r = x0.clone(memory_format=torch.channels_last).requires_grad_(True), r0.clone(memory_format=torch.channels_last).requires_grad_(True)
+        with hooks:
+            y = batch_norm_act(bn, x, r, nn.ReLU())
+        got.append(torch.autograd.grad(y, [x, r, bn.weight, bn.bias], dy))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 def test_the_residual_is_not_kept():
     _need_gpu()
     import weakref

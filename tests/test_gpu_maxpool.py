@@ -49,6 +49,20 @@ def test_nan_and_infinities():
     assert torch.equal(torch.autograd.grad(y, x, dy)[0], torch.autograd.grad(want, x, dy)[0])
 
 
+@pytest.mark.parametrize("pin", [False, True])
+def test_saved_tensors_that_come_back_in_another_layout(pin):
+    _need_gpu()
+    from fairring_b200.ops import max_pool
+
+    x = torch.randn(2, 8, 13, 12, device="cuda").contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    pool = nn.MaxPool2d(3, 2, 1)
+    with torch.autograd.graph.save_on_cpu(pin_memory=pin):
+        y = max_pool(pool, x)
+    assert type(y.grad_fn).__name__ == "_MaxPoolFnBackward"
+    dy = torch.randint(-2, 3, y.shape, device="cuda").float()
+    assert torch.equal(torch.autograd.grad(y, x, dy)[0], torch.autograd.grad(pool(x), x, dy)[0])
+
+
 def test_calls_the_module_where_it_cannot_be_skipped():
     _need_gpu()
     from fairring_b200.ops import max_pool
