@@ -70,16 +70,18 @@ __global__ void __launch_bounds__(kNaThreads) sum_static_kernel(NaBufs b, int n)
   }
 }
 
+// The launch's own status: cudaGetLastError() would also return, and clear, an error that the
+// host program has pending from something else.
 template <int W>
-cudaError_t launchSum(const NaBufs& b, int n, bool aligned, cudaStream_t stream) {
-  if (aligned) {
-    const int blocks = n / 4 > 0 ? (n / 4 + kNaThreads - 1) / kNaThreads : 1;
-    sum_static_kernel<W, float4><<<blocks, kNaThreads, 0, stream>>>(b, n);
-  } else {
-    sum_static_kernel<W, float><<<(n + kNaThreads - 1) / kNaThreads, kNaThreads, 0, stream>>>(b, n);
-  }
-  fairring::noteLocalLaunch();
-  return cudaGetLastError();
+cudaError_t launchSum(NaBufs& b, int n, bool aligned, cudaStream_t stream) {
+  const int vectors = aligned ? n / 4 : n;
+  const int blocks = vectors > 0 ? (vectors + kNaThreads - 1) / kNaThreads : 1;
+  void* args[] = {&b, &n};
+  const void* kernel = aligned ? reinterpret_cast<const void*>(&sum_static_kernel<W, float4>)
+                               : reinterpret_cast<const void*>(&sum_static_kernel<W, float>);
+  const cudaError_t e = cudaLaunchKernel(kernel, dim3(blocks), dim3(kNaThreads), args, 0, stream);
+  if (e == cudaSuccess) fairring::noteLocalLaunch();
+  return e;
 }
 
 int fail(int code, char* err, unsigned long err_len, const char* msg) {

@@ -1,6 +1,8 @@
 """The allocation-free sum at its edges: remainders of the 4-element vectors, buffers that are only
 4-byte aligned, the smallest and largest size, every number of buffers."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -26,3 +28,18 @@ def test_sum_in_buffer_order(world, n, offset):
     for p, b in zip(pads, before):
         assert torch.equal(p[offset:offset + n], expect)
         assert torch.equal(p[:offset], b[:offset]) and torch.equal(p[offset + n:], b[offset + n:])
+
+
+def test_an_error_that_the_host_has_pending():
+    """It is neither reported by this call nor cleared."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    bufs = [torch.full((9,), float(r), device="cuda") for r in range(3)]
+    torch.cuda.synchronize()
+    runtime = ctypes.CDLL("libcudart.so.12")  # the one that torch and the library use
+    refused = runtime.cudaSetDevice(4096)  # no such device: an error of the host call alone
+    assert refused != 0
+    rc, msg = _call(_lib(), bufs)
+    assert runtime.cudaGetLastError() == refused
+    assert rc == 0, msg
+    assert all(bool((b == 3.0).all()) for b in bufs)
