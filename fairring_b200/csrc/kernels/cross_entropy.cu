@@ -2,9 +2,9 @@
 // language-model workloads.  torch's path under bf16 autocast widens the bf16
 // logits to fp32 (a pass), runs log_softmax (a pass each way), nll_loss, and
 // narrows the fp32 gradient back to bf16 (another pass): more than ten bytes of
-// HBM traffic per logit.  Here the forward reads every logit once and keeps one
-// float per row; the backward recomputes the softmax from the logits and that
-// float and writes the gradient in the logits' own dtype: six bytes per bf16
+// HBM traffic per logit.  Here the forward reads every logit once and keeps the
+// logarithm of a row's sum as two floats; the backward recomputes the softmax from the
+// logits and those and writes the gradient in the logits' own dtype: six bytes per bf16
 // logit in all, which is what bounds both kernels.
 //
 // Rows of any length: a row is the elements up to its first 16-byte boundary, 16-byte
@@ -121,7 +121,9 @@ __device__ __forceinline__ float blockReduce(float v, bool is_max, float* scratc
   return r;
 }
 
-// loss[r] = logsumexp(row r) - row r[target]; lse[r] kept for the backward.
+// loss[r] = logsumexp(row r) - row r[target]; kept for the backward: logsumexp in lse[r] and what
+// its rounding cut off in lse[kept + r].  At a maximum of 20 that is up to 1e-6 of every probability
+// of the row, several times fp32's own error.
 // A negative target marks a row that does not count: loss 0, as for a target past the
 // vocabulary.  With `classes` > 0 a target that is neither below it nor -100 ends the program, as it
 // does in torch's loss.  One block per row, one sweep over it: a thread
@@ -130,7 +132,7 @@ __device__ __forceinline__ float blockReduce(float v, bool is_max, float* scratc
 template <typename T, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1280 / kThreads)
 cross_entropy_fwd_kernel(const T* __restrict__ logits, const int64_t* __restrict__ targets,
-                         float* __restrict__ loss, float* __restrict__ lse, int vocab, int classes) {
+                         float* __restrict__ loss, float* __restrict__ lse, int64_t kept, int vocab, int classes) {
   constexpr int E = Vec16<T>::kElems, U = kCeBatch;
   __shared__ float scratch[kThreads / 32];
   const int64_t r = blockIdx.x;
@@ -174,12 +176,13 @@ cross_entropy_fwd_kernel(const T* __restrict__ logits, const int64_t* __restrict
   const float m = blockReduce<kThreads>(a.m, true, scratch);
   const float s = blockReduce<kThreads>(a.s * expOf<T>(a.m - SoftSum<T>::reference(m)), false, scratch);
   if (threadIdx.x == 0) {
-    const float l = m + logf(s);
+    const float ls = logf(s), l = m + ls, part = l - m;
     lse[r] = l;
+    lse[kept + r] = (m - (l - part)) + (ls - part);  // m + ls - l, exactly
     const int64_t t = targets[r];
     const bool counts = t >= 0 && t < vocab;
     assert((classes == 0 || t == -100 || (t >= 0 && t < classes)) && "target outside the vocabulary");
-    loss[r] = counts ? l - toFloat(row[t]) : 0.f;
+    loss[r] = counts ? (m - toFloat(row[t])) + ls : 0.f;
   }
 }
 
@@ -190,7 +193,7 @@ __global__ void __launch_bounds__(1024)
 cross_entropy_mean_kernel(const float* __restrict__ loss, const int64_t* __restrict__ targets, int64_t rows,
                           float least, float* __restrict__ mean, float* __restrict__ count) {
   __shared__ float scratch[32];
-  float s = 0.f, n = 0.f;  // counts stay exact: a thread's below 2^24
+  float s = 0.f, n = 0.f;  // the count is exact up to 2^24 rows, beyond that as good as the sum of the losses
   for (int64_t r = threadIdx.x; r < rows; r += 1024) {
     s += loss[r];
     n += targets[r] >= 0 ? 1.f : 0.f;
@@ -211,7 +214,7 @@ template <typename T, int kThreads>
 __global__ void __launch_bounds__(kThreads)
 cross_entropy_bwd_kernel(const T* logits, T* grad, const int64_t* __restrict__ targets,
                          const float* __restrict__ lse, const float* __restrict__ upstream,
-                         const float* __restrict__ count, float scale, int64_t pieces_total, int pieces, int vocab) {
+                         const float* __restrict__ count, float scale, int64_t kept, int64_t pieces_total, int pieces, int vocab) {
   constexpr int E = Vec16<T>::kElems, U = kCeBatch;
   const float g = (count != nullptr ? *upstream / *count : *upstream) * scale;
   for (int64_t w = blockIdx.x; w < pieces_total; w += gridDim.x) {
@@ -230,8 +233,8 @@ cross_entropy_bwd_kernel(const T* logits, T* grad, const int64_t* __restrict__ t
     const int64_t t64 = targets[r];
     const bool counts = t64 >= 0 && t64 < vocab;
     const int t = counts ? (int)t64 : -1;
-    const float l = lse[r];
-    auto one = [&](float v, int j) { return counts ? (expOf<T>(v - l) - (j == t ? 1.f : 0.f)) * g : 0.f; };
+    const float l = lse[r], cut = sizeof(T) == 4 ? lse[kept + r] : 0.f;  // far below bf16's rounding
+    auto one = [&](float v, int j) { return counts ? (expOf<T>(sizeof(T) == 4 ? (v - l) - cut : v - l) - (j == t ? 1.f : 0.f)) * g : 0.f; };
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = first + u * kThreads;
@@ -263,10 +266,10 @@ void forwardOf(const void* logits, const int64_t* targets, float* loss, float* l
     const T* at = static_cast<const T*>(logits) + done * vocab;
     if (vocab >= kCeFwdWide * kCeBatch * Vec16<T>::kElems)
       cross_entropy_fwd_kernel<T, kCeFwdWide><<<n, kCeFwdWide, 0, stream>>>(at, targets + done, loss + done, lse + done,
-                                                                           vocab, classes);
+                                                                           rows, vocab, classes);
     else
       cross_entropy_fwd_kernel<T, kCeFwdNarrow><<<n, kCeFwdNarrow, 0, stream>>>(at, targets + done, loss + done,
-                                                                               lse + done, vocab, classes);
+                                                                               lse + done, rows, vocab, classes);
     noteLocalLaunch();
   }
 }
@@ -279,7 +282,7 @@ void backwardOf(const void* logits, void* grad, const int64_t* targets, const fl
   const int64_t total = rows * pieces;
   const unsigned blocks = (unsigned)(total < (1 << 30) ? total : (1 << 30));
   cross_entropy_bwd_kernel<T, kCeBwdThreads><<<blocks, kCeBwdThreads, 0, stream>>>(
-      static_cast<const T*>(logits), static_cast<T*>(grad), targets, lse, upstream, count, scale, total, pieces, vocab);
+      static_cast<const T*>(logits), static_cast<T*>(grad), targets, lse, upstream, count, scale, rows, total, pieces, vocab);
   noteLocalLaunch();
 }
 

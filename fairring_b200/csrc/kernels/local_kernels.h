@@ -68,7 +68,7 @@ cudaError_t launchAddLayerNormBackward(const void* dy, bool y_bf16, const float*
 cudaError_t launchAddBranch(const float* x, const void* branch_bf16, float* out, int64_t n, cudaStream_t stream);
 
 // Softmax cross-entropy over [rows, vocab] logits (fp32 or bf16): per-row loss
-// and log-sum-exp; the row of a target that is negative or past the vocabulary has
+// and log-sum-exp (2 x rows: rounded, and what the rounding cut off); the row of a target that is negative or past the vocabulary has
 // loss 0; with `classes` > 0 a target is an error unless it is below that or -100.
 cudaError_t launchCrossEntropyForward(const void* logits, bool bf16, const int64_t* targets, float* loss,
                                       float* lse, int64_t rows, int vocab, int classes, cudaStream_t stream);

@@ -301,14 +301,14 @@ void checkLogits(const at::Tensor& logits, const at::Tensor& targets) {
   TORCH_CHECK(logits.size(1) > 0 && logits.size(1) <= INT32_MAX, "the vocabulary must not be empty");
 }
 
-// (per-row loss, per-row log-sum-exp) of logits [rows, vocab] against targets [rows];
+// (per-row loss, [2, rows] log-sum-exp and what its rounding cut off) of logits [rows, vocab] against targets [rows];
 // `classes`, if not 0: a target that is neither one of them nor -100 is an error.
 std::tuple<at::Tensor, at::Tensor> crossEntropyForward(at::Tensor logits, at::Tensor targets, int64_t classes) {
   checkLogits(logits, targets);
   TORCH_CHECK(classes >= 0 && classes <= logits.size(1), "no more classes than logits");
   c10::cuda::CUDAGuard guard(logits.device());
   auto fopt = logits.options().dtype(at::kFloat);
-  at::Tensor loss = at::empty({logits.size(0)}, fopt), lse = at::empty({logits.size(0)}, fopt);
+  at::Tensor loss = at::empty({logits.size(0)}, fopt), lse = at::empty({2, logits.size(0)}, fopt);
   cudaError_t e = launchCrossEntropyForward(logits.data_ptr(), logits.scalar_type() == at::kBFloat16,
                                             targets.data_ptr<int64_t>(), loss.data_ptr<float>(),
                                             lse.data_ptr<float>(), logits.size(0), (int)logits.size(1),
@@ -339,8 +339,9 @@ void crossEntropyBackward(at::Tensor grad, at::Tensor logits, at::Tensor targets
   TORCH_CHECK(grad.is_cuda() && grad.device() == logits.device() && grad.is_contiguous() &&
                   grad.sizes() == logits.sizes() && grad.scalar_type() == logits.scalar_type(),
               "grad must be like the logits");
-  TORCH_CHECK(lse.is_cuda() && lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.numel() == logits.size(0),
-              "lse must be a contiguous fp32 CUDA vector with one entry per row");
+  TORCH_CHECK(lse.is_cuda() && lse.scalar_type() == at::kFloat && lse.is_contiguous() &&
+                  lse.numel() == 2 * logits.size(0),
+              "lse must be the contiguous fp32 [2, rows] CUDA tensor that the forward made");
   TORCH_CHECK(upstream.is_cuda() && upstream.scalar_type() == at::kFloat && upstream.numel() == 1,
               "upstream must be a one-element fp32 CUDA tensor");
   const float* count_ptr = nullptr;
