@@ -54,8 +54,8 @@ __device__ __forceinline__ void loadChannels(const float* p, int group, float (&
 // Vectors in flight per thread and stream: 64 bytes.
 template <typename T> constexpr int kBnUnroll = sizeof(T) == 2 ? 4 : 2;
 
-// part[block][0][c] = mean and part[block][1][c] = M2 of this block's rows, of which
-// there are as many as rowsOfBlock() says.
+// part[block][0][c] = mean and part[block][1][c] = M2 of this block's rows; how
+// many those are, the merge works out.
 template <typename T>
 __global__ void __launch_bounds__(kBnThreads, 4)
 bn_stats_kernel(const T* __restrict__ x, int64_t nvec, int groups, float* __restrict__ part) {

@@ -13,7 +13,8 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops import add_layer_norm_pair, cross_entropy_keeping_logits, linear, linear_gelu, tied_embedding, vocab_logits
-from ..ops._plain import FUSE_FROM, native, plain_module
+from ..ops import _plain
+from ..ops._plain import native, plain_module
 
 
 @dataclass
@@ -108,7 +109,8 @@ class EncoderMLM(nn.Module):
         x, table = tied_embedding(self.tok, self.pos, tokens, pad_rows=labels is not None)
         x = self.ln_emb(x)
         low = x
-        large = x.is_cuda and b * s * self.cfg.d_ff >= FUSE_FROM
+        # By the widest activation: below it forward_pair() would fuse little or nothing and cost the host more.
+        large = x.is_cuda and b * s * max(self.cfg.d_ff, 3 * self.cfg.d_model) >= _plain.FUSE_FROM
         for layer in self.layers:
             if large and plain_module(layer, EncoderLayer):
                 x, low = layer.forward_pair(x, low)

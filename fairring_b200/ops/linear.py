@@ -81,9 +81,9 @@ _FUSE_FROM = FUSE_FROM
 
 def _fusable(fc: nn.Linear, x: torch.Tensor) -> bool:
     """Whether the layer's output will be bf16 on the GPU and large, and its bias wants a gradient."""
-    if not native(x) or x.dim() < 2 or x.numel() // max(1, x.shape[-1]) * fc.out_features < _FUSE_FROM:
+    if not ordinary(x) or x.dim() < 2 or x.numel() // max(1, x.shape[-1]) * fc.out_features < _FUSE_FROM:
         return False
-    if not (plain_module(fc, nn.Linear) and ordinary(fc.weight) and fc.bias is not None
+    if not (native(x) and plain_module(fc, nn.Linear) and ordinary(fc.weight) and fc.bias is not None
             and fc.bias.requires_grad and torch.is_grad_enabled() and fc.out_features % 8 == 0
             and fc.bias.dtype in (torch.float32, torch.bfloat16) and fc.bias.device == x.device):
         return False

@@ -90,6 +90,24 @@ def test_a_channel_far_from_zero_keeps_its_variance():
     assert ((bn.running_var.double() - want).abs() <= 1e-5 * want).all()
 
 
+def test_nan_passes_the_relu():
+    """As in torch: NaN stays NaN forward, and a gradient passes where the output is NaN."""
+    _need_gpu()
+    from fairring_b200 import _C
+
+    x = torch.randn(2, 8, 4, 4, device="cuda").contiguous(memory_format=torch.channels_last)
+    x[0, 3, 1, 1] = float("nan")  # its channel's statistics are NaN
+    res = torch.randn_like(x)
+    bn, relu = nn.BatchNorm2d(8, device="cuda"), nn.ReLU()
+    from fairring_b200.ops import batch_norm_act
+
+    y, want = batch_norm_act(bn, x, res, relu), relu(nn.BatchNorm2d(8, device="cuda")(x) + res)
+    assert torch.equal(y.isnan(), want.isnan()) and bool(y[:, 3].isnan().all()) and int(y.isnan().sum()) == 32
+    ones, stat = torch.ones_like(x), torch.ones(8, device="cuda")
+    dz = _C.batch_norm_bwd(ones, torch.zeros_like(x), y.detach(), bn.weight.detach(), bn.bias.detach(), stat, stat, True)[1]
+    assert torch.equal(dz, (~(y <= 0)).float())
+
+
 def test_calls_the_modules_where_they_cannot_be_skipped():
     _need_gpu()
     from fairring_b200.ops import batch_norm_act
@@ -101,7 +119,9 @@ def test_calls_the_modules_where_they_cannot_be_skipped():
     assert not _fusable(bn, x.contiguous(), None)  # NCHW
     assert not _fusable(bn, x.half(), None)
     assert not _fusable(bn, x, x.bfloat16())
-    assert not _fusable(nn.BatchNorm2d(24, device="cuda"), x.new_zeros(4, 24, 6, 6), None)
+    for channels in (24, 4096):  # no power of two, too many
+        wide = torch.zeros(2, channels, 4, 4, device="cuda").contiguous(memory_format=torch.channels_last)
+        assert not _fusable(nn.BatchNorm2d(channels, device="cuda"), wide, None)
     seen = []
     handle = relu.register_forward_hook(lambda *a: seen.append(1))
     batch_norm_act(bn, x, relu=relu)

@@ -18,6 +18,7 @@ def _small_sizes_too(monkeypatch):
     monkeypatch.setattr(sys.modules["fairring_b200.ops.layernorm"], "_PAIR_FROM", 0)
     monkeypatch.setattr(sys.modules["fairring_b200.ops.embedding"], "_PAD_FROM", 0)
     monkeypatch.setattr(sys.modules["fairring_b200.ops._plain"], "FUSE_FROM", 0)
+    monkeypatch.setattr(sys.modules["fairring_b200.ops.linear"], "_FUSE_FROM", 0)
 
 
 def _need_gpu():
@@ -124,6 +125,22 @@ def test_padded_head_matches_torch(vocab, rows):
         torch.testing.assert_close(a, r, rtol=2.0 ** -6, atol=2.0 ** -7 * scale, equal_nan=True)
 
 
+FUSED = {"_TiedEmbeddingFnBackward", "_AddLayerNormPairFnBackward", "_BiasGradFnBackward", "_GeluFnBackward",
+         "_PaddedHeadFnBackward"}
+
+
+def _nodes(loss):
+    """The names of all autograd nodes behind `loss`."""
+    seen, todo, names = set(), [loss.grad_fn], set()
+    while todo:
+        fn = todo.pop()
+        if fn is not None and fn not in seen:
+            seen.add(fn)
+            names.add(type(fn).__name__)
+            todo += [f for f, _ in fn.next_functions]
+    return names
+
+
 def test_encoder_matches_its_plain_layers():
     _need_gpu()
     from fairring_b200.models import EncoderConfig, EncoderMLM, mask_tokens
@@ -141,6 +158,7 @@ def test_encoder_matches_its_plain_layers():
                 m.register_forward_hook(lambda *a: None)
         with torch.autocast("cuda", dtype=torch.bfloat16):
             loss = model(tokens, labels)
+        assert _nodes(loss) >= FUSED if not hooked else not _nodes(loss) & FUSED
         got.append([loss, *torch.autograd.grad(loss, list(model.parameters()))])
     assert abs(float(got[0][0]) - float(got[1][0])) < 2e-3 * float(got[1][0])
     for a, r in zip(got[0][1:], got[1][1:]):

@@ -1,4 +1,4 @@
-"""The LayerNorm kernels where their groups of warps begin and end, against fp64."""
+"""The LayerNorm kernels at the edges of their warps and rounds, against fp64."""
 
 import pytest
 import torch
@@ -12,8 +12,9 @@ def _need_gpu():
         pytest.skip("needs a CUDA device")
 
 
-# one thread, one warp full and one column group past it, 2 and 3 warps, one group per block, 8 and 9 warps
-# (two ways to merge them), all 32; one row, fewer rows than groups, more rows than blocks
+# A block of 256 threads does a row, 8 columns to a thread, in up to four rounds of 2048: one thread, a warp
+# less one thread, a full warp and one thread more, several warps, a full round and one thread of the next, four
+# rounds less one thread and all four; one row, fewer rows than blocks, more rows than blocks
 @pytest.mark.parametrize("cols", [8, 248, 256, 264, 768, 1032, 2048, 2056, 8184, 8192])
 @pytest.mark.parametrize("rows", [1, 5, 3001])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

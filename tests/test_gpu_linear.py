@@ -41,6 +41,22 @@ def test_gelu_and_column_sums(rows, cols, form):
     assert torch.equal(low, plain.bfloat16())
 
 
+@pytest.mark.parametrize("form", ["none", "tanh"])
+def test_gelu_of_the_largest_values(form):
+    """Infinities, NaN and the largest finite values give what torch gives, NaN included."""
+    _need_gpu()
+    from fairring_b200 import _C
+
+    big = torch.finfo(torch.bfloat16).max
+    x = torch.tensor([float("inf"), float("-inf"), float("nan"), big, -big, 1e4, -1e4, 0.0], device="cuda").bfloat16().view(1, 8)
+    ref = x.detach().requires_grad_(True)
+    want = F.gelu(ref, approximate=form)
+    (want_dx,) = torch.autograd.grad(want, ref, torch.ones_like(x))
+    torch.testing.assert_close(_C.gelu_fwd(x, form == "tanh"), want, rtol=0, atol=0, equal_nan=True)
+    got = _C.gelu_bwd(torch.ones_like(x), x, form == "tanh", torch.float32)[0]
+    torch.testing.assert_close(got, want_dx, rtol=0, atol=0, equal_nan=True)
+
+
 @pytest.mark.parametrize("weights", [torch.float32, torch.bfloat16])
 def test_layers_match_torch(weights, monkeypatch):
     _need_gpu()

@@ -78,7 +78,7 @@ def _every_size(monkeypatch):
     import fairring_b200.models  # noqa: F401
 
     for module, name in (("ops.layernorm", "_PAIR_FROM"), ("ops.embedding", "_PAD_FROM"), ("ops.linear", "_FUSE_FROM"),
-                         ("ops.stem", "_FOLD_FROM"), ("models.encoder", "FUSE_FROM")):
+                         ("ops.stem", "_FOLD_FROM"), ("ops._plain", "FUSE_FROM")):
         monkeypatch.setattr(sys.modules["fairring_b200." + module], name, 0)
 
 

@@ -3,7 +3,7 @@
 Some hosts of this library cannot allocate device memory when they need a
 reduction (another part of the process is capturing a CUDA graph, or they live
 inside somebody else's memory budget).  For them the library exports one C
-function whose scratch memory is a static array inside the library.  This test
+function that needs no scratch memory at all.  This test
 calls it with ctypes, twice in a row, and compares with the regular (allocating)
 one-shot all-reduce.  The file sorts last so that a failure here cannot hide
 results of the other tests.
@@ -43,7 +43,7 @@ def test_matches_the_allocating_entry_point_twice(C, world, n):
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA device")
     fn = _lib()
-    for attempt in range(2):  # two calls in a row share the static scratch
+    for attempt in range(2):  # nothing is kept from one call for the next
         g = torch.Generator().manual_seed(10 * attempt + world)
         ins = [torch.randn(n, generator=g).cuda() for _ in range(world)]
         ref, status = C.emulated_collective("allreduce", [t.clone() for t in ins], world,
