@@ -8,7 +8,7 @@
 // rows of the lookup are added into it where they belong, those of one token by one
 // block in a fixed order; other blocks of the same launch sum the positions' gradient.
 // Bound by HBM, by the widening above all: of a 51200 x 2048 table 1.1 ms -> 0.2 ms, for
-// 8192 tokens 30 us forward besides.
+// 8192 tokens 30 us forward and 50 us backward besides.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -50,67 +50,105 @@ __device__ __forceinline__ void sumPositions(const float4* __restrict__ dx, floa
   dpos[s * d4 + c] = sum;
 }
 
-// The rows of the tokens that are `bucket` modulo `buckets`, 4 x 32 columns, added to the table's
+// The rows of the tokens that are `bucket` modulo `buckets`, 4 x 64 columns, added to the table's
 // gradient.  All of a token's rows meet in one block, so they are added without atomics and in an order that
 // depends on the tokens alone.  The block looks through all tokens, kTile at a time, and lists
-// its own in their order; then a warp takes a token and walks through its rows, except that
-// the rows of a frequent one are shared out among all warps.
+// its own in their order.  From a long list it takes out the frequent tokens, whose rows all warps share; of
+// the rest, where looking for equal tokens pair by pair is cheap, a warp takes a token at a time.
+//
+// With the positions' sums, rows of 2048: 8192 tokens of 51200 50 us (by atomics, in no fixed order, 33 us), with 15 %
+// of them one and the same 80 us (39), with all of them 272 us (83); a block's latency bounds the latter two.
 constexpr int kTile = 8 * kEmbThreads;  // tokens per round, 8 to a thread
 constexpr int kWarps = kEmbThreads / 32;
-constexpr int kFrequent = 32;  // occurrences within a round
+constexpr int kLong = 64;     // entries
+constexpr int kFrequent = 4;  // of 32 entries looked at
+constexpr int kWide = 2;      // float4 columns of a thread, 32 apart
 
 struct TokenLists {
-  uint32_t key[kTile];    // token / buckets
-  uint16_t at[kTile];     // place within the round
-  uint16_t rank[kTile];   // how many entries of the same token come before
-  uint16_t next[kTile];   // the one behind, or the list's length
-  uint16_t count[kTile];  // all of them, where rank is 0
-  uint16_t rows[kTile];   // of the frequent token at hand: its places by rank
-  float4 part[kWarps][32];
+  alignas(16) uint32_t key[kTile + 4];  // token / buckets; no token's behind the last entry
+  uint16_t at[kTile];                   // place within the round
+  uint16_t next[kTile];                 // the next entry of the same token, or the list's length
+  uint16_t count[kTile];                // entries of the token, 0 where this is not its first
+  uint16_t rows[kTile];                 // places of the frequent token at hand
+  float4 part[kWide][kWarps][32];
   int total[kWarps];
 };
+
+// Where a thread's `found` entries go, behind those of the threads before it, and the number of all.
+__device__ __forceinline__ int2 placeOf(int found, TokenLists& l) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int upto = found;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += up;
+  }
+  __syncthreads();  // `total` may still be read, and so may the lists that are about to be written
+  if (lane == 31) l.total[w] = upto;
+  __syncthreads();
+  int before = upto - found, all = 0;
+#pragma unroll
+  for (int v = 0; v < kWarps; ++v) {
+    if (v < w) before += l.total[v];
+    all += l.total[v];
+  }
+  return make_int2(before, all);
+}
+
+// The rows in l.rows, shared among the warps, added to a row of the table.
+__device__ __forceinline__ void sumFrequent(const float4* __restrict__ row, float4* out, int c, int d4, int count,
+                                            TokenLists& l) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  constexpr int U = 4;
+  float4 sum[kWide];
+#pragma unroll
+  for (int k = 0; k < kWide; ++k) sum[k] = zero;
+  for (int e = w; e < count; e += U * kWarps) {
+    float4 g[U][kWide];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int at = e + u * kWarps;
+#pragma unroll
+      for (int k = 0; k < kWide; ++k)
+        g[u][k] = at < count && c + k * 32 < d4 ? row[(int64_t)l.rows[at] * d4 + k * 32] : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int k = 0; k < kWide; ++k) sum[k] = sum[k] + g[u][k];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kWide; ++k) l.part[k][w][lane] = sum[k];
+  __syncthreads();
+  if (w < kWide && c + w * 32 < d4) {
+    float4 all = l.part[w][0][lane];
+#pragma unroll
+    for (int v = 1; v < kWarps; ++v) all = all + l.part[w][v][lane];
+    out[w * 32] = out[w * 32] + all;
+  }
+  __syncthreads();
+}
 
 __device__ __forceinline__ void sumTokens(const float4* __restrict__ dx, const int64_t* __restrict__ tokens,
                                           float4* dtable, uint32_t bucket, uint32_t buckets, int chunk, int64_t n,
                                           int64_t vocab, int d4, TokenLists& l) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int c = chunk * 32 + lane;
-  const bool mine = c < d4;
+  const int c = chunk * 32 * kWide + lane;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  int64_t t[8];
-  auto fetch = [&](int64_t base) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int64_t i = base + threadIdx.x * 8 + k;
-      t[k] = i < n ? tokens[i] : -1;
-    }
-  };
-  fetch(0);
+  auto tableRow = [&](uint32_t key) { return dtable + ((int64_t)key * buckets + bucket) * d4 + c; };
   for (int64_t base = 0; base < n; base += kTile) {
     uint32_t hits = 0;
     uint32_t key[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      key[k] = (uint32_t)t[k] / buckets;
-      if (t[k] >= 0 && t[k] < vocab && (uint32_t)t[k] - key[k] * buckets == bucket) hits |= 1u << k;
+      const int64_t i = base + threadIdx.x * 8 + k, t = i < n ? tokens[i] : -1;
+      key[k] = (uint32_t)t / buckets;
+      if (t >= 0 && t < vocab && (uint32_t)t - key[k] * buckets == bucket) hits |= 1u << k;
     }
-    if (base + kTile < n) fetch(base + kTile);
-    // where this thread's entries go: behind those of the threads before it
-    const int found = __popc(hits);
-    int before = found;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int up = __shfl_up_sync(0xffffffffu, before, o);
-      if (lane >= o) before += up;
-    }
-    if (lane == 31) l.total[w] = before;
-    __syncthreads();
-    int m = 0, slot = before - found;
-#pragma unroll
-    for (int v = 0; v < kWarps; ++v) {
-      if (v < w) slot += l.total[v];
-      m += l.total[v];
-    }
+    const int2 place = placeOf(__popc(hits), l);
+    int m = place.y, slot = place.x;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       if (hits >> k & 1u) {
@@ -119,76 +157,91 @@ __device__ __forceinline__ void sumTokens(const float4* __restrict__ dx, const i
       }
     }
     __syncthreads();
-    bool frequent = false;
-    for (int i = threadIdx.x; i < m; i += kEmbThreads) {
-      const uint32_t own = l.key[i];
-      int rank = 0, count = 0, next = m;
-      for (int j = 0; j < m; ++j) {
-        if (l.key[j] == own) {
-          ++count;
-          if (j < i) ++rank;
-          if (j > i && next == m) next = j;
+    const float4* row = dx + base * d4 + c;
+    while (m > kLong) {
+      const uint32_t sample = l.key[(2 * lane + 1) * m / 64];
+      const unsigned best = __reduce_max_sync(0xffffffffu, __popc(__match_any_sync(0xffffffffu, sample)) * 32u + lane);
+      if (best < kFrequent * 32u) break;
+      const uint32_t own = __shfl_sync(0xffffffffu, sample, best & 31u);  // the same in all warps
+      uint32_t mine = 0, other = 0, keys[8];
+      uint16_t ats[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int i = threadIdx.x * 8 + k;
+        if (i < m) {
+          keys[k] = l.key[i];
+          ats[k] = l.at[i];
+          (keys[k] == own ? mine : other) |= 1u << k;
         }
       }
-      l.rank[i] = (uint16_t)rank;
-      l.next[i] = (uint16_t)next;
-      l.count[i] = (uint16_t)(rank == 0 ? count : 0);
-      frequent |= count >= kFrequent;
+      const int2 to = placeOf(__popc(mine), l);
+      int in = to.x, out = threadIdx.x * 8 - to.x;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        if (mine >> k & 1u) l.rows[in++] = ats[k];
+        if (other >> k & 1u) {
+          l.key[out] = keys[k];
+          l.at[out++] = ats[k];
+        }
+      }
+      __syncthreads();
+      sumFrequent(row, tableRow(own), c, d4, to.y, l);
+      m -= to.y;
     }
-    frequent = __syncthreads_or(frequent);
-    const float4* row = dx + base * d4 + c;
-    for (int i = w; i < m; i += kWarps) {
-      if (l.count[i] == 0 || l.count[i] >= kFrequent) continue;
-      float4 sum = zero;
-      for (int e = i; e < m;) {
-        float4 g[4];
+    if (threadIdx.x < 4) l.key[m + threadIdx.x] = ~0u;
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += kEmbThreads) {
+      const uint32_t own = l.key[i];
+      int before = 0, count = 0, next = m;
+      for (int j = 0; j < m; j += 4) {
+        const uint4 k = *reinterpret_cast<const uint4*>(l.key + j);
+        const uint32_t there[4] = {k.x, k.y, k.z, k.w};
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          g[u] = e < m && mine ? row[(int64_t)l.at[e] * d4] : zero;
+          const bool hit = there[u] == own;
+          count += hit;
+          before += hit && j + u < i;
+          if (hit && j + u > i) next = min(next, j + u);
+        }
+      }
+      l.next[i] = (uint16_t)next;
+      l.count[i] = (uint16_t)(before == 0 ? count : 0);
+    }
+    __syncthreads();
+    for (int i = w; i < m; i += kWarps) {
+      if (l.count[i] == 0) continue;
+      float4* out = tableRow(l.key[i]);
+      float4 was[kWide], sum[kWide];
+#pragma unroll
+      for (int k = 0; k < kWide; ++k) {
+        was[k] = c + k * 32 < d4 ? out[k * 32] : zero;
+        sum[k] = zero;
+      }
+      for (int e = i; e < m;) {
+        float4 g[2][kWide];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+#pragma unroll
+          for (int k = 0; k < kWide; ++k)
+            g[u][k] = e < m && c + k * 32 < d4 ? row[(int64_t)l.at[e] * d4 + k * 32] : zero;
           if (e < m) e = l.next[e];
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) sum = sum + g[u];
-      }
-      if (mine) {
-        float4* out = dtable + ((int64_t)l.key[i] * buckets + bucket) * d4 + c;
-        *out = *out + sum;
-      }
-    }
-    for (int i = 0; frequent && i < m; ++i) {
-      const int count = l.count[i];
-      if (count < kFrequent) continue;
-      for (int j = threadIdx.x; j < m; j += kEmbThreads)
-        if (l.key[j] == l.key[i]) l.rows[l.rank[j]] = l.at[j];
-      __syncthreads();
-      float4 sum = zero;
-      for (int e = w; e < count; e += 8 * kWarps) {
-        float4 g[8];
+        for (int u = 0; u < 2; ++u) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int at = e + u * kWarps;
-          g[u] = at < count && mine ? row[(int64_t)l.rows[at] * d4] : zero;
+          for (int k = 0; k < kWide; ++k) sum[k] = sum[k] + g[u][k];
         }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) sum = sum + g[u];
       }
-      l.part[w][lane] = sum;
-      __syncthreads();
-      if (w == 0 && mine) {
-        sum = l.part[0][lane];
 #pragma unroll
-        for (int v = 1; v < kWarps; ++v) sum = sum + l.part[v][lane];
-        float4* out = dtable + ((int64_t)l.key[i] * buckets + bucket) * d4 + c;
-        *out = *out + sum;
-      }
-      // the next one writes `part` only behind its own first barrier
+      for (int k = 0; k < kWide; ++k)
+        if (c + k * 32 < d4) out[k * 32] = was[k] + sum[k];
     }
     __syncthreads();  // the lists are used up; and a table row may go to another warp in the next round
   }
 }
 
 // The first `buckets` x `chunks` blocks do the tokens, the others the positions.
-__global__ void __launch_bounds__(kEmbThreads)
+__global__ void __launch_bounds__(kEmbThreads, 4)
 embed_bwd_kernel(const float4* __restrict__ dx, const int64_t* __restrict__ tokens, float4* dtable,
                  float4* __restrict__ dpos, int batch, int seq, int64_t vocab, int d4, uint32_t buckets, uint32_t chunks) {
   __shared__ TokenLists lists;
@@ -226,9 +279,9 @@ cudaError_t launchEmbedBackward(const float* dx, const int64_t* tokens, float* d
   if (n <= 0) return cudaSuccess;
   if (d <= 0 || d % 4 != 0 || vocab > UINT32_MAX) return cudaErrorInvalidValue;
   const int d4 = d / 4;
-  const int64_t chunks = (d4 + 31) / 32, position_blocks = (int64_t)seq * ((d4 + kEmbThreads - 1) / kEmbThreads);
+  const int64_t chunks = (d4 + 32 * kWide - 1) / (32 * kWide), position_blocks = (int64_t)seq * ((d4 + kEmbThreads - 1) / kEmbThreads);
   // As many token blocks as are resident, each of which looks through all tokens, but at least 8 tokens for one.
-  int64_t buckets = (int64_t)sm_count * 5 / chunks;
+  int64_t buckets = (int64_t)sm_count * 4 / chunks;
   if (buckets > (n + 7) / 8) buckets = (n + 7) / 8;
   if (buckets < 1) buckets = 1;
   if (buckets * chunks + position_blocks > INT32_MAX) return cudaErrorInvalidValue;

@@ -47,8 +47,8 @@ def test_matches_torch(d, batch, seq, positions, use):
         assert float((a - b).abs().max()) <= 2e-6 * (batch * seq) ** 0.5 * max(1.0, float(b.abs().max()))
 
 
-# less than a round of the token lists, two rounds and a ragged third; tokens of one occurrence, of a warp's
-# share, of all warps' (32 and more within a round) and a batch of nothing else
+# less than one round of 2048 tokens, a ragged second and third; tokens of a few occurrences, lists long enough
+# to take a frequent token out, and a batch of nothing else
 @pytest.mark.parametrize("d", [8, 136, 2048])
 @pytest.mark.parametrize("batch,seq", [(1, 7), (3, 700), (5, 1001)])
 @pytest.mark.parametrize("mix", ["spread", "frequent", "one"])
