@@ -68,6 +68,7 @@ __device__ __forceinline__ float2 blockSum2(float a, float b, float2 (&halves)[2
 // Differences throughout, since E[x^2] - mean^2 cancels in a row whose mean is far from
 // zero: a warp sums its part relative to its first element, then squares relative to its
 // own mean, and the warps' results are merged relative to the first one's, behind one barrier.
+// With the residual add, 8192 x 2048: 35.1 us; 32.1 us with the difference that cancels.
 template <int ITER> struct RowMoments {
   static constexpr int kWarps = kLnThreads / 32;
   float2 part[2][kWarps];  // (mean, sum of squares) per warp, in two halves as above
@@ -228,7 +229,8 @@ layer_norm_bwd_kernel(const TY* __restrict__ dy, const TX* __restrict__ x,
 // dgamma[c] = sum over blocks of partial[b][0][c]; dbeta likewise.  A block owns 32
 // of the 2 x cols columns; warp w sums partial rows w, w+32, ... (one 128-byte line
 // per load, eight loads in flight), then the warps' sums are added through shared
-// memory.  Bound by the launch and two trips to L2: 592 rows of 2 x 2048 take 3.9 us;
+// memory.  Bound by the launch and two trips to L2: 592 rows of 2 x 2048 take 3.9 us right behind
+// the kernel that wrote them (4.5 us as the mean over a decoder step, 7.1 us from DRAM);
 // eight warps with four loads in flight took 9.8 us.
 __global__ void __launch_bounds__(1024, 1)
 layer_norm_param_grad_kernel(const float* __restrict__ partial, int nblocks, int cols,
