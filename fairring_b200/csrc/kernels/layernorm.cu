@@ -43,11 +43,10 @@ __device__ __forceinline__ float warpSum(float v) {
   return v;
 }
 
-// Sum of two values over the block; every thread gets the result.  `scratch` is in
-// two halves that rows alternate between: one barrier per row, which is what the
+// Sum of two values over the block; every thread gets the result.  Rows alternate between
+// two scratch arrays: one barrier per row, which is what the
 // kernels wait for when they do not wait for memory.
-__device__ __forceinline__ float2 blockSum2(float a, float b, float2 (&halves)[2][kLnThreads / 32], int half) {
-  float2* scratch = halves[half];
+__device__ __forceinline__ float2 blockSum2(float a, float b, float2 (&scratch)[kLnThreads / 32]) {
   for (int o = 16; o > 0; o >>= 1) {
     a += __shfl_xor_sync(0xffffffffu, a, o);
     b += __shfl_xor_sync(0xffffffffu, b, o);
@@ -64,85 +63,56 @@ __device__ __forceinline__ float2 blockSum2(float a, float b, float2 (&halves)[2
   return s;
 }
 
-// Mean and variance of a row that the block holds in registers; every thread gets both.
-// Differences throughout, since E[x^2] - mean^2 cancels in a row whose mean is far from
-// zero: a warp sums its part relative to its first element, then squares relative to its
-// own mean, and the warps' results are merged relative to the first one's, behind one barrier.
-// With the residual add, 8192 x 2048: 35.1 us; 32.1 us with the difference that cancels.
-template <int ITER> struct RowMoments {
-  static constexpr int kWarps = kLnThreads / 32;
-  float2 part[2][kWarps];  // (mean, sum of squares) per warp, in two halves as above
-  float share[kWarps];     // its part of the row
-
-  // Columns of warp w.
-  static __device__ __forceinline__ int columns(int w, int cols) {
-    int n = 0;
+// Mean and variance of a row that the block holds in registers, from its sum `t.x` and its sum
+// of squares `t.y`.  E[x^2] - mean^2 cancels where the mean is far from zero, off by several
+// percent for a mean of 1000 and a deviation of 1.  There, from a mean as large as the
+// deviation on, both are taken again from the differences to the mean, behind a second barrier,
+// which only such rows pay for.  Infinities and NaN take that way too and make the row NaN.
+template <int ITER>
+__device__ __forceinline__ float2 rowMoments(float2 t, const float (&v)[ITER][8], int cols,
+                                             float2 (&again)[kLnThreads / 32]) {
+  const float mean = t.x / cols, var = fmaf(-mean, mean, t.y / cols);
+  if (__fmul_rn(mean, mean) <= var) return make_float2(mean, var);  // the same for the whole block
+  float s = 0.f, q = 0.f;
 #pragma unroll
-    for (int it = 0; it < ITER; ++it) n += min(max(cols - (it * kLnThreads + w * 32) * 8, 0), 256);
-    return n;
-  }
-  // Before the first row, whose barrier makes it visible.
-  __device__ __forceinline__ void init(int cols) {
-    if (threadIdx.x < kWarps) share[threadIdx.x] = (float)columns(threadIdx.x, cols) / cols;
-  }
-  // `inv`: 1 / columns of this warp, 0 if it has none.
-  __device__ __forceinline__ float2 of(const float (&v)[ITER][8], int cols, float inv, int half) {
-    const float first = __shfl_sync(0xffffffffu, v[0][0], 0);
-    float s = 0.f, q = 0.f;
+  for (int it = 0; it < ITER; ++it) {
+    if ((it * kLnThreads + (int)threadIdx.x) * 8 < cols) {
 #pragma unroll
-    for (int it = 0; it < ITER; ++it) {
-      if ((it * kLnThreads + (int)threadIdx.x) * 8 < cols) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) s += v[it][i] - first;
+      for (int i = 0; i < 8; ++i) {
+        const float d = v[it][i] - mean;
+        s += d;
+        q = fmaf(d, d, q);
       }
     }
-    const float own = fmaf(warpSum(s), inv, first);
-#pragma unroll
-    for (int it = 0; it < ITER; ++it) {
-      if ((it * kLnThreads + (int)threadIdx.x) * 8 < cols) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float d = v[it][i] - own;
-          q = fmaf(d, d, q);
-        }
-      }
-    }
-    q = warpSum(q);
-    if ((threadIdx.x & 31) == 0) part[half][threadIdx.x >> 5] = make_float2(own, q);
-    __syncthreads();
-    const float about = part[half][0].x;
-    float d = 0.f, between = 0.f, within = 0.f;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const float2 p = part[half][w];
-      const float e = p.x - about, f = share[w];
-      d = fmaf(f, e, d);
-      between = fmaf(f * e, e, between);
-      within += p.y;
-    }
-    const float var = within / cols + (between - d * d);
-    return make_float2(about + d, var < 0.f ? 0.f : var);  // NaN stays
   }
-};
+  t = blockSum2(s, q, again);  // free again: the next row's first barrier lies behind its readers
+  const float off = t.x / cols, exact = t.y / cols - off * off;
+  return make_float2(mean + off, exact < 0.f ? 0.f : exact);
+}
 
 template <typename TX, typename TY, int ITER>
 __global__ void __launch_bounds__(kLnThreads, ITER == 1 ? 8 : 1)
 layer_norm_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ gamma,
                       const float* __restrict__ beta, TY* __restrict__ y, float* __restrict__ mean_out,
                       float* __restrict__ rstd_out, int64_t rows, int cols, float eps) {
-  __shared__ RowMoments<ITER> moments;
-  moments.init(cols);
-  const int own = moments.columns(threadIdx.x >> 5, cols);
-  const float inv = own > 0 ? 1.f / own : 0.f;
+  __shared__ float2 scratch[2][kLnThreads / 32], again[kLnThreads / 32];
   int half = 0;
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, half ^= 1) {
-    float v[ITER][8] = {};
+    float v[ITER][8];
+    float s = 0.f, ss = 0.f;
 #pragma unroll
     for (int it = 0; it < ITER; ++it) {
       const int c = (it * kLnThreads + threadIdx.x) * 8;
-      if (c < cols) load8<TX>(x + r * cols + c, v[it]);
+      if (c < cols) {
+        load8<TX>(x + r * cols + c, v[it]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          s += v[it][i];
+          ss += v[it][i] * v[it][i];
+        }
+      }
     }
-    const float2 t = moments.of(v, cols, inv, half);
+    const float2 t = rowMoments<ITER>(blockSum2(s, ss, scratch[half]), v, cols, again);
     const float mean = t.x, rstd = rsqrtf(t.y + eps);
     if (threadIdx.x == 0) {
       mean_out[r] = mean;
@@ -202,7 +172,7 @@ layer_norm_bwd_kernel(const TY* __restrict__ dy, const TX* __restrict__ x,
         }
       }
     }
-    const float2 t = blockSum2(s1, s2, scratch, half);
+    const float2 t = blockSum2(s1, s2, scratch[half]);
     const float m1 = t.x / cols, m2 = t.y / cols;
 #pragma unroll
     for (int it = 0; it < ITER; ++it) {
@@ -273,13 +243,11 @@ add_layer_norm_fwd_kernel(const float* __restrict__ x, const TB* __restrict__ br
                           const float* __restrict__ gamma, const float* __restrict__ beta,
                           float* __restrict__ xnew, TY* __restrict__ y, float* __restrict__ mean_out,
                           float* __restrict__ rstd_out, int64_t rows, int cols, float eps) {
-  __shared__ RowMoments<ITER> moments;
-  moments.init(cols);
-  const int own = moments.columns(threadIdx.x >> 5, cols);
-  const float inv = own > 0 ? 1.f / own : 0.f;
+  __shared__ float2 scratch[2][kLnThreads / 32], again[kLnThreads / 32];
   int half = 0;
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, half ^= 1) {
-    float v[ITER][8] = {};
+    float v[ITER][8];
+    float s = 0.f, ss = 0.f;
 #pragma unroll
     for (int it = 0; it < ITER; ++it) {
       const int c = (it * kLnThreads + threadIdx.x) * 8;
@@ -288,11 +256,15 @@ add_layer_norm_fwd_kernel(const float* __restrict__ x, const TB* __restrict__ br
         load8<float>(x + r * cols + c, v[it]);
         load8<TB>(branch + r * cols + c, b);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[it][i] += b[i];
+        for (int i = 0; i < 8; ++i) {
+          v[it][i] += b[i];
+          s += v[it][i];
+          ss += v[it][i] * v[it][i];
+        }
         store8<float>(xnew + r * cols + c, v[it]);
       }
     }
-    const float2 t = moments.of(v, cols, inv, half);
+    const float2 t = rowMoments<ITER>(blockSum2(s, ss, scratch[half]), v, cols, again);
     const float mean = t.x, rstd = rsqrtf(t.y + eps);
     if (threadIdx.x == 0) {
       mean_out[r] = mean;
@@ -366,7 +338,7 @@ add_layer_norm_bwd_kernel(const TY* __restrict__ dy, const float* __restrict__ d
         }
       }
     }
-    const float2 t = blockSum2(s1, s2, scratch, half);
+    const float2 t = blockSum2(s1, s2, scratch[half]);
     const float m1 = t.x / cols, m2 = t.y / cols;
 #pragma unroll
     for (int it = 0; it < ITER; ++it) {
